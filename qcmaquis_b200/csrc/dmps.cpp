@@ -452,7 +452,7 @@ void preconditioned_svd(Ctx& c, const DBlocks& both, BlockSVD& r, int* zero_coun
     batched_qr(qj, both.d.get(), both.total, Qb.get(), ql, Xb.get(), xl, Wq.get(), wq, c.qjobs, c.s, Pb.get(), pl);
     if (sweeps) QCM_CUDA(cudaEventRecord(ev[1], c.s));
     batched_jacobi_svd(sj, Xb.get(), xl, Uxb.get(), xl, r.S.get(), r.s_len, Vxb.get(), xl, Wjb.get(), wj, zero_count, c.sjobs,
-                       c.s, sweeps);
+                       c.side, c.s, sweeps);
     if (sweeps) QCM_CUDA(cudaEventRecord(ev[2], c.s));
     if (!gu.empty()) batched_gemm(gu, Qb.get(), ql, Vxb.get(), xl, r.U.get(), r.u_len, c.gjobs, c.gtiles, c.s);
     if (!gv.empty()) batched_gemm(gv, Qb.get(), ql, Vxb.get(), xl, r.V.get(), r.v_len, c.gjobs, c.gtiles, c.s);
@@ -524,18 +524,14 @@ BlockSVD svd_truncate_groups(Ctx& c, const DBlocks& both, const std::vector<std:
         QCM_CUDA(cudaStreamSynchronize(c.s));
         uint32_t mr = 0, mc = 0;
         std::size_t kbig = 0;
-        int modes[3] = {0, 0, 0};  // work matrix and rotations in shared memory / work matrix only / neither
         for (std::size_t k = 0; k < nb; ++k) {
             mr = std::max(mr, both.rows[k]);
             mc = std::max(mc, both.cols[k]);
-            // the Jacobi runs on the k x k factor R^T
-            const uint64_t cc = std::min(both.rows[k], both.cols[k]), cpd = (cc + (cc & 1)) * cc;
             if (uint64_t(both.rows[k]) * both.cols[k] > uint64_t(both.rows[kbig]) * both.cols[kbig]) kbig = k;
-            modes[2 * cpd <= jacobi_svd_smem_doubles() ? 0 : (cpd <= jacobi_svd_smem_doubles() ? 1 : 2)]++;
         }
-        std::fprintf(stderr, "[svd] %zu blocks (max %u x %u): %.3f ms, Jacobi sweeps max %d; largest %u x %u: %d sweeps; modes %d/%d/%d\n",
+        std::fprintf(stderr, "[svd] %zu blocks (max %u x %u): %.3f ms, Jacobi sweeps max %d; largest %u x %u: %d sweeps\n",
                      nb, mr, mc, ms, hsw.empty() ? 0 : *std::max_element(hsw.begin(), hsw.end()), both.rows[kbig],
-                     both.cols[kbig], nb ? hsw[kbig] : 0, modes[0], modes[1], modes[2]);
+                     both.cols[kbig], nb ? hsw[kbig] : 0);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }

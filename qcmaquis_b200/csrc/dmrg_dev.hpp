@@ -106,6 +106,7 @@ struct Ctx {
     DBuf<uint32_t> gtiles;
     DBuf<CopyJob> cjobs;
     DBuf<SvdJob> sjobs;
+    std::unique_ptr<SideStreams> side;
     DBuf<QrJob> qjobs;
     DBuf<PermJob> pjobs;
     DBuf<double> qrw;  // QR / LQ scratch

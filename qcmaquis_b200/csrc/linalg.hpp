@@ -1,7 +1,7 @@
 // Dense per-block factorizations on the device, used by the truncation and
 // canonisation steps of the sweep:
 //   thin SVD   (framework/alps/matrix/algorithms.hpp:243-257, gesvd 'S','S'): one-sided Jacobi,
-//              all blocks in one launch (cuSOLVER gesvdj completes a block whose kept singular
+//              all blocks at once (cuSOLVER gesvdj completes a block whose kept singular
 //              values include exact zeros)
 //   thin QR    (algorithms.hpp:260-291, geqrf + orgqr) and thin LQ (algorithms.hpp:293-325, gelqf
 //              + orglq, here QR of the transpose): Householder, all blocks in one launch
@@ -14,6 +14,7 @@
 #include <cusolverDn.h>
 
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "device.hpp"
@@ -54,7 +55,20 @@ struct Solver {
 // U (m x k, ld m), S (k, descending), V (n x k, ld n): A = U diag(S) V^T, by cuSOLVER's gesvdj on side
 // lane `l` (between fork and join), status to *info
 void svd_thin_lane(Solver& sv, int l, const double* A, int m, int n, double* U, double* S, double* V, int* info);
-// Thin SVDs of many small blocks in one launch (one-sided Jacobi, one CTA per block):
+// Streams beside a main one, for launches that run at the same time (fork from / join to the main stream).
+struct SideStreams {
+    static constexpr int N = 4;
+    cudaStream_t s[N] = {};
+    cudaEvent_t fork_ev = nullptr, done[N] = {};
+    SideStreams();
+    ~SideStreams();
+    SideStreams(const SideStreams&) = delete;
+    SideStreams& operator=(const SideStreams&) = delete;
+    void fork(cudaStream_t from);
+    void join(cudaStream_t to);
+};
+
+// Thin SVDs of many blocks (one-sided Jacobi, a cluster of 1 to 16 CTAs per block; jacobi_svd.cu):
 // A_j (m x n, ld m) = U_j diag(S_j) V_j^T with U_j (m x k, ld m), S_j descending (k), V_j
 // (n x k, ld n), k = min(m, n) -- the layout of gesvdj with econ = 1.  A singular value that
 // is exactly zero leaves a zero column in U_j (m >= n) or V_j (m < n); zero_count[id] counts them
@@ -66,16 +80,15 @@ struct SvdJob {
     uint32_t id, pad;  // zero_count[id] receives the block's number of zero singular values
 };
 uint64_t jacobi_svd_scratch(uint32_t m, uint32_t n);
-// doubles of the Jacobi kernel's shared-memory work space (blocks larger than it work in L2)
-uint64_t jacobi_svd_smem_doubles();
 // Symmetric eigendecomposition (divide and conquer, lower triangle) on lane `l`: A (n x n, ld n)
 // is overwritten by the eigenvectors, W receives the eigenvalues in ascending order.
 // Replaces heevd('V') of alps/matrix/algorithms.hpp:374-396 (which then reverses the order).
 void syevd_lane(Solver& sv, int l, double* A, int n, double* W, int* info);
-// A, U, S, V, W: base pointers of the offsets in jobs (host list, validated against the lengths)
+// A, U, S, V, W: base pointers of the offsets in jobs (host list, validated against the lengths); side: made on
+// the first call that launches more than one cluster size
 void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64_t a_len, double* U, uint64_t u_len, double* S,
                         uint64_t s_len, double* V, uint64_t v_len, double* W, uint64_t w_len, int* zero_count,
-                        DBuf<SvdJob>& jobbuf, cudaStream_t s, int* sweeps_used = nullptr);
+                        DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, int* sweeps_used = nullptr);
 // Thin QR / LQ of many blocks in one launch (Householder, one CTA per block; qr_batched.cu):
 //   lq = 0: A_j (m x n, ld m) = Q_j R_j, Q_j (m x k, ld m), R_j (k x n, ld k);
 //   lq = 1: A_j = L_j Q_j, L_j (m x k, ld m) at r_off, Q_j (k x n, ld k) at q_off;
