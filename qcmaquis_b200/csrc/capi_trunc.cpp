@@ -130,7 +130,7 @@ extern "C" int qcm_qr_blocks(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* ro
         wl += (qcm::qr_scratch(uint32_t(m), uint32_t(n), lq != 0) + 31) / 32 * 32;
     }
     qcm::DBuf<double> dq(std::max<uint64_t>(ql, 1)), dr(std::max<uint64_t>(rl, 1)), dw(std::max<uint64_t>(wl, 1));
-    qcm::batched_qr(jobs, M.d.get(), M.total, dq.get(), ql, dr.get(), rl, dw.get(), wl ? wl : 1, c.qjobs, c.s);
+    qcm::batched_qr(jobs, M.d.get(), M.total, dq.get(), ql, dr.get(), rl, dw.get(), wl ? wl : 1, c.qjobs, c.side, c.s);
     download(c, dq.get(), Q, ql);
     download(c, dr.get(), R, rl);
     QCM_CUDA(cudaStreamSynchronize(c.s));

@@ -4,7 +4,7 @@
 //              all blocks at once (cuSOLVER gesvdj completes a block whose kept singular
 //              values include exact zeros)
 //   thin QR    (algorithms.hpp:260-291, geqrf + orgqr) and thin LQ (algorithms.hpp:293-325, gelqf
-//              + orglq, here QR of the transpose): Householder, all blocks in one launch
+//              + orglq, here QR of the transpose): Householder, all blocks at once
 //   symmetric eigendecomposition of the density-matrix blocks (algorithms.hpp:374-396, heevd):
 //              cuSOLVER syevd on side lanes
 // plus the Rayleigh-Ritz eigenproblem of the Jacobi-Davidson solver (host, <= 64 x 64).
@@ -89,7 +89,7 @@ void syevd_lane(Solver& sv, int l, double* A, int n, double* W, int* info);
 void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64_t a_len, double* U, uint64_t u_len, double* S,
                         uint64_t s_len, double* V, uint64_t v_len, double* W, uint64_t w_len, int* zero_count,
                         DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, int* sweeps_used = nullptr);
-// Thin QR / LQ of many blocks in one launch (Householder, one CTA per block; qr_batched.cu):
+// Thin QR / LQ of many blocks (Householder, a cluster of 1 to 16 CTAs per block; qr_batched.cu):
 //   lq = 0: A_j (m x n, ld m) = Q_j R_j, Q_j (m x k, ld m), R_j (k x n, ld k);
 //   lq = 1: A_j = L_j Q_j, L_j (m x k, ld m) at r_off, Q_j (k x n, ld k) at q_off;
 // k = min(m, n); W: scratch of qr_scratch(m, n, lq) doubles per block at w_off.
@@ -113,8 +113,8 @@ struct QrJob {
 };
 uint64_t qr_scratch(uint32_t m, uint32_t n, bool lq);
 void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len, double* Q, uint64_t q_len, double* R,
-                uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, cudaStream_t s, uint32_t* P = nullptr,
-                uint64_t p_len = 0);
+                uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, std::unique_ptr<SideStreams>& side,
+                cudaStream_t s, uint32_t* P = nullptr, uint64_t p_len = 0);
 
 // Lowest eigenpair of the symmetric n x n matrix held in the upper triangle of
 // M (column-major, leading dimension ldm); cyclic Jacobi rotations, FP64.
