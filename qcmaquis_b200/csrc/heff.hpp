@@ -167,7 +167,7 @@ void add_unit_tiles(const UnitD& u, uint32_t item, const LKD* ents, std::size_t 
 //     alpha = op value * boundary conj scale(c, x) * (MPO scale * line_scale[line0 + l])
 // at W[w_off + l + slot * nl], where x is the entry's other MPO index, c the boundary cohort
 // of (unit, input state), and slot the unit's slot of slice id jbase(unit, input state) +
-// block position of x in cohort c.  Terms of one line are summed in entry, then operator-term
+// block position of x in cohort c.  Terms of one cell are summed in entry, then operator-term
 // order by one thread, with products and sums rounded separately.
 struct WGenUnitD {
     uint64_t w_off;
@@ -197,8 +197,25 @@ struct MPOTables {
     std::vector<uint32_t> row_ptr, row_other, row_op, col_ptr, col_other, col_op;
     std::vector<double> row_scale, col_scale;
     uint32_t rows = 0, cols = 0;
+    bool row_sorted = true, col_sorted = true;  // the other index does not decrease within any row / column
 };
 std::shared_ptr<const MPOTables> build_mpo_tables(const MPOTensor& W);
+
+// the coefficient-generation tables on the device (CoefGen::tables)
+struct WGenTab {
+    const WGenUnitD* units;
+    const WGenInD* gin;
+    const uint32_t* line_major;
+    const double* line_scale;
+    const uint32_t *smap_id, *smap_slot, *m_ptr, *m_other, *m_op;
+    const double* m_scale;
+    const uint32_t *o_ptr, *o_in;
+    const double* o_val;
+    const int32_t* b_pos;
+    const double* b_cs;
+    uint32_t nst, b_aux;
+    bool serial;
+};
 
 struct CoefGen {
     hvec<WGenUnitD> units;
@@ -212,6 +229,7 @@ struct CoefGen {
     std::vector<int32_t> b_pos;  // boundary cohort x aux: block position of the MPO index, or -1
     const std::vector<double>* b_cs = nullptr;  // boundary conj scales (cohort x aux)
     uint32_t b_aux = 0;
+    bool serial = false;  // two MPO indices of one boundary cohort share a block
     uint64_t w_len = 0;
 
     DBuf<WGenUnitD> d_units;
@@ -233,6 +251,7 @@ struct CoefGen {
     void append_units(const CoefGen& part, uint32_t line_base, uint32_t map_base, uint64_t w_base);
     void validate() const;  // throws unless every index k_wgen derives stays in its buffer
     void upload(cudaStream_t s);
+    WGenTab tables() const;
     // W (w_len doubles) = coefficient blocks; waits for the stream and throws if a term had no slot
     void generate(double* W, cudaStream_t s);
     // the blocks of units [u0, u1) (elements [w0, w1) of the whole, written from W on), without the

@@ -7,8 +7,8 @@
 //   Sbar      = L_eff^T ybar per L.S segment       (transpose of contract, tasks.cpp:286-313),
 //   Wbar_u    = Sbar_u T_u^T per unit              (k_wbar, DMMA, in the coefficient-block layout),
 //   coeff_bar = sum over the terms of entry e of Wbar_u(line, slot) * o_val * b_cs * line_scale.
-// The last runs k_wgen's traversal backwards.  One thread per line writes the line's partial sum for
-// every entry of its MPO row (k_wadj).  Then one thread per entry adds the partials of the lines of
+// The last runs k_wgen's traversal backwards.  One thread per (line, entry of its MPO row) writes the
+// line's partial sum for the entry (k_wadj).  Then one thread per entry adds the partials of the lines of
 // its row in increasing line order (k_entry_sum).  There are no atomics, so the result does not
 // vary from run to run.
 #include <cuda_runtime.h>
@@ -21,6 +21,7 @@
 #include "dev_ops.hpp"
 #include "dmma.cuh"
 #include "heff.hpp"
+#include "wgen.cuh"
 
 namespace qcm {
 
@@ -106,67 +107,33 @@ __global__ void __launch_bounds__(NTHR) k_wbar(const UnitD* __restrict__ units, 
     });
 }
 
-constexpr int WA_THR = 128;
-constexpr uint32_t WA_SMAP = 4096;  // (slice id, slot) pairs staged in shared memory
-constexpr uint32_t WA_NST = 64;     // physical states of the basis (CoefGen::validate bounds nst)
-
 // Per line: P[pofs[line] + (e - m_ptr[m])] = sum over the terms of entry e (row m of the line) of
-// Wbar(line, slot) * o_val * b_cs * line_scale; the traversal and slot lookup of k_wgen.
-__global__ void __launch_bounds__(WA_THR) k_wadj(const WGenUnitD* __restrict__ units, const WGenInD* __restrict__ gin,
-                                                 uint32_t nst, const uint32_t* __restrict__ line_major,
-                                                 const double* __restrict__ line_scale,
-                                                 const uint32_t* __restrict__ smap_id, const uint32_t* __restrict__ smap_slot,
-                                                 const uint32_t* __restrict__ m_ptr, const uint32_t* __restrict__ m_other,
-                                                 const uint32_t* __restrict__ m_op, const uint32_t* __restrict__ o_ptr,
-                                                 const uint32_t* __restrict__ o_in, const double* __restrict__ o_val,
-                                                 const int32_t* __restrict__ b_pos, const double* __restrict__ b_cs,
-                                                 uint32_t b_aux, const double* __restrict__ Wb,
-                                                 const uint64_t* __restrict__ pofs, double* __restrict__ P,
-                                                 uint32_t* __restrict__ err) {
-    __shared__ uint32_t sid[WA_SMAP], sslot[WA_SMAP];
-    __shared__ WGenInD sin[WA_NST];
-    const WGenUnitD U = units[blockIdx.x];
-    const bool staged = U.nk <= WA_SMAP;
-    if (staged)
-        for (uint32_t i = threadIdx.x; i < U.nk; i += blockDim.x) {
-            sid[i] = smap_id[U.map0 + i];
-            sslot[i] = smap_slot[U.map0 + i];
+// Wbar(line, slot) * o_val * b_cs * line_scale; the traversal and slot lookup of k_wgen, one thread per entry.
+__global__ void __launch_bounds__(wg::THR) k_wadj(WGenTab t, const double* __restrict__ Wb, const uint64_t* __restrict__ pofs,
+                                                  double* __restrict__ P, uint32_t* __restrict__ err) {
+    __shared__ wg::Shared sh;
+    const WGenUnitD U = t.units[blockIdx.x];
+    const wg::Map map = wg::stage(t, U, blockIdx.x, sh);
+    const double* Wu = Wb + U.w_off;
+    wg::for_entries(t, U, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t) {
+        const uint32_t gl = U.line0 + line, x = t.m_other[e];
+        const double lsc = t.line_scale[gl];
+        const std::size_t q = std::size_t(t.m_op[e]) * t.nst + U.st_out;
+        const uint32_t k1 = t.o_ptr[q + 1];
+        double acc = 0.0;
+        for (uint32_t k = t.o_ptr[q]; k < k1; ++k) {
+            const WGenInD g = sh.sin[t.o_in[k]];
+            if (g.c == WGEN_NONE) continue;
+            const std::size_t bq = std::size_t(g.c) * t.b_aux + x;
+            const int32_t pos = t.b_pos[bq];
+            if (pos < 0) continue;
+            const uint32_t slot = map.slot(g.jbase + uint32_t(pos));
+            if (slot == WGEN_NONE) { atomicOr(err, 1u); continue; }
+            const double d = __dmul_rn(__dmul_rn(t.o_val[k], t.b_cs[bq]), lsc);  // d alpha / d scale_e
+            acc = fma(Wu[line + uint64_t(slot) * U.wld], d, acc);
         }
-    for (uint32_t i = threadIdx.x; i < nst; i += blockDim.x) sin[i] = gin[std::size_t(blockIdx.x) * nst + i];
-    __syncthreads();
-    const uint32_t* ids = staged ? sid : smap_id + U.map0;
-    const uint32_t* slots = staged ? sslot : smap_slot + U.map0;
-    for (uint32_t line = threadIdx.x; line < U.nl; line += blockDim.x) {
-        const uint32_t gl = U.line0 + line;
-        const uint32_t m = line_major[gl];
-        const double lsc = line_scale[gl];
-        const double* Wl = Wb + U.w_off + line;
-        double* Pl = P + pofs[gl];
-        const uint32_t e0 = m_ptr[m];
-        for (uint32_t e = e0; e < m_ptr[m + 1]; ++e) {
-            const uint32_t x = m_other[e], op = m_op[e];
-            const std::size_t q = std::size_t(op) * nst + U.st_out;
-            double acc = 0.0;
-            for (uint32_t k = o_ptr[q]; k < o_ptr[q + 1]; ++k) {
-                const WGenInD g = sin[o_in[k]];
-                if (g.c == WGEN_NONE) continue;
-                const std::size_t bq = std::size_t(g.c) * b_aux + x;
-                const int32_t pos = b_pos[bq];
-                if (pos < 0) continue;
-                const uint32_t id = g.jbase + uint32_t(pos);
-                uint32_t lo = 0, hi = U.nk;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (ids[mid] < id) lo = mid + 1;
-                    else hi = mid;
-                }
-                if (lo >= U.nk || ids[lo] != id) { atomicOr(err, 1u); continue; }
-                const double d = __dmul_rn(__dmul_rn(o_val[k], b_cs[bq]), lsc);  // d alpha / d scale_e
-                acc = fma(Wl[uint64_t(slots[lo]) * U.wld], d, acc);
-            }
-            Pl[e - e0] = acc;
-        }
-    }
+        P[pofs[gl] + (e - e0)] = acc;
+    });
 }
 
 // out[e] = sum over the lines of e's MPO row (increasing line order) of their partial for e
@@ -177,7 +144,17 @@ __global__ void k_entry_sum(uint64_t n_terms, const uint32_t* __restrict__ e_row
         const uint32_t m = e_row[e];
         const uint64_t j = e - m_ptr[m];
         double s = 0.0;
-        for (uint32_t t = rl_ptr[m]; t < rl_ptr[m + 1]; ++t) s += P[pofs[rl_line[t]] + j];
+        uint32_t t = rl_ptr[m];
+        const uint32_t t1 = rl_ptr[m + 1];
+        // eight partials in flight (each is two dependent reads), added in line order
+        for (; t + 8 <= t1; t += 8) {
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = P[pofs[rl_line[t + i]] + j];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s += v[i];
+        }
+        for (; t < t1; ++t) s += P[pofs[rl_line[t]] + j];
         out[e] = s;
     }
 }
@@ -286,11 +263,8 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
     const CoefGen& cg = p.cg;
     QCM_CUDA(cudaMemsetAsync(w.d_err.get(), 0, sizeof(uint32_t), s));
     if (!cg.units.empty())
-        k_wadj<<<unsigned(cg.units.size()), WA_THR, 0, s>>>(
-            cg.d_units.get(), cg.d_gin.get(), cg.nst, cg.d_line_major.get(), cg.d_line_scale.get(), cg.d_smap_id.get(),
-            cg.d_smap_slot.get(), cg.d_m_ptr.get(), cg.d_m_other.get(), cg.d_m_op.get(), cg.d_o_ptr.get(), cg.d_o_in.get(),
-            cg.d_o_val.get(), cg.d_b_pos.get(), cg.d_b_cs.get(), cg.b_aux, w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
-            w.d_err.get());
+        k_wadj<<<unsigned(cg.units.size()), wg::THR, 0, s>>>(cg.tables(), w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
+                                                             w.d_err.get());
     QCM_CUDA(cudaGetLastError());
     const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 255) / 256, 148 * 16));
     k_entry_sum<<<grid, 256, 0, s>>>(w.n_terms, w.d_e_row.get(), cg.d_m_ptr.get(), w.d_rl_ptr.get(), w.d_rl_line.get(),

@@ -28,6 +28,7 @@
 
 #include "dmma.cuh"
 #include "heff.hpp"
+#include "wgen.cuh"
 
 namespace qcm {
 namespace {
@@ -240,63 +241,44 @@ __global__ void __launch_bounds__(NTHR, 5) k_sgemm(const UnitD* __restrict__ uni
     }
 }
 
-// One CTA per unit, one thread per line: the line's coefficient terms (CoefGen), in MPO-entry
-// then operator-term order, summed into W_u.  Products and sums are rounded separately (no
-// contraction), so W_u holds the same values as a host evaluation of the same terms.
-constexpr int WG_THR = 256;  // 256 against 128: streamed applies 3-11 % faster
-constexpr uint32_t WG_SMAP = 4096;  // (slice id, slot) pairs staged in shared memory
-constexpr uint32_t WG_NST = 64;     // physical states of the basis
-__global__ void __launch_bounds__(WG_THR) k_wgen(const WGenUnitD* __restrict__ units, const WGenInD* __restrict__ gin,
-                                                 uint32_t nst, const uint32_t* __restrict__ line_major,
-                                                 const double* __restrict__ line_scale,
-                                                 const uint32_t* __restrict__ smap_id, const uint32_t* __restrict__ smap_slot,
-                                                 const uint32_t* __restrict__ m_ptr, const uint32_t* __restrict__ m_other,
-                                                 const uint32_t* __restrict__ m_op, const double* __restrict__ m_scale,
-                                                 const uint32_t* __restrict__ o_ptr, const uint32_t* __restrict__ o_in,
-                                                 const double* __restrict__ o_val, const int32_t* __restrict__ b_pos,
-                                                 const double* __restrict__ b_cs, uint32_t b_aux, double* __restrict__ W,
-                                                 uint64_t w0, uint32_t* __restrict__ err) {
-    __shared__ uint32_t sid[WG_SMAP], sslot[WG_SMAP];
-    __shared__ WGenInD sin[WG_NST];
-    const WGenUnitD U = units[blockIdx.x];
-    const bool staged = U.nk <= WG_SMAP;
-    if (staged)
-        for (uint32_t i = threadIdx.x; i < U.nk; i += blockDim.x) {
-            sid[i] = smap_id[U.map0 + i];
-            sslot[i] = smap_slot[U.map0 + i];
-        }
-    for (uint32_t i = threadIdx.x; i < nst; i += blockDim.x) sin[i] = gin[std::size_t(blockIdx.x) * nst + i];
-    __syncthreads();
-    const uint32_t* ids = staged ? sid : smap_id + U.map0;
-    const uint32_t* slots = staged ? sslot : smap_slot + U.map0;
-    for (uint32_t line = threadIdx.x; line < U.nl; line += blockDim.x) {
-        const uint32_t m = line_major[U.line0 + line];
-        const double lsc = line_scale[U.line0 + line];
-        double* Wl = W + (U.w_off - w0) + line;
-        for (uint32_t e = m_ptr[m]; e < m_ptr[m + 1]; ++e) {
-            const uint32_t x = m_other[e], op = m_op[e];
-            const double wsc = __dmul_rn(m_scale[e], lsc);
-            const std::size_t q = std::size_t(op) * nst + U.st_out;
-            for (uint32_t k = o_ptr[q]; k < o_ptr[q + 1]; ++k) {
-                const WGenInD g = sin[o_in[k]];
+// One CTA per unit: the coefficient terms of its lines (CoefGen), in MPO-entry then operator-term order, summed
+// into W_u.  Products and sums are rounded separately (no contraction), so W_u holds the same values as a host
+// evaluation of the same terms.  Terms of a line meet in one cell only if their entries share the other MPO
+// index (a slice id is an input state's base plus that index's block position), and those are neighbours in the
+// row: the thread of the first of them adds them all, in order.  Tables that break either premise (an unsorted
+// row, two indices of a boundary cohort on one block: CoefGen::serial) leave the whole row to one thread.
+// One thread per line took 2.07 ms for the 12 M terms of the L=16, M=256 middle bond.
+__global__ void __launch_bounds__(wg::THR) k_wgen(WGenTab t, uint32_t u0, double* __restrict__ W, uint64_t w0,
+                                                  uint32_t* __restrict__ err) {
+    __shared__ wg::Shared sh;
+    const uint32_t unit = u0 + blockIdx.x;
+    const WGenUnitD U = t.units[unit];
+    const wg::Map map = wg::stage(t, U, unit, sh);
+    double* Wu = W + (U.w_off - w0);
+    wg::for_entries(t, U, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t e1) {
+        uint32_t x = t.m_other[e];
+        if (e > e0 && (t.serial || t.m_other[e - 1] == x)) return;  // added by an earlier entry's thread
+        const double lsc = t.line_scale[U.line0 + line];
+        for (uint32_t f = e;;) {
+            const double wsc = __dmul_rn(t.m_scale[f], lsc);
+            const std::size_t q = std::size_t(t.m_op[f]) * t.nst + U.st_out;
+            const uint32_t k1 = t.o_ptr[q + 1];
+            for (uint32_t k = t.o_ptr[q]; k < k1; ++k) {
+                const WGenInD g = sh.sin[t.o_in[k]];
                 if (g.c == WGEN_NONE) continue;
-                const std::size_t bq = std::size_t(g.c) * b_aux + x;
-                const int32_t pos = b_pos[bq];
+                const std::size_t bq = std::size_t(g.c) * t.b_aux + x;
+                const int32_t pos = t.b_pos[bq];
                 if (pos < 0) continue;
-                const double a = __dmul_rn(__dmul_rn(o_val[k], b_cs[bq]), wsc);
-                const uint32_t id = g.jbase + uint32_t(pos);
-                uint32_t lo = 0, hi = U.nk;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (ids[mid] < id) lo = mid + 1;
-                    else hi = mid;
-                }
-                if (lo >= U.nk || ids[lo] != id) { atomicOr(err, 1u); continue; }
-                double* w = Wl + uint64_t(slots[lo]) * U.wld;
+                const double a = __dmul_rn(__dmul_rn(t.o_val[k], t.b_cs[bq]), wsc);
+                const uint32_t slot = map.slot(g.jbase + uint32_t(pos));
+                if (slot == WGEN_NONE) { atomicOr(err, 1u); continue; }
+                double* w = Wu + line + uint64_t(slot) * U.wld;
                 *w = __dadd_rn(*w, a);
             }
+            if (++f >= e1 || (!t.serial && t.m_other[f] != x)) break;
+            x = t.m_other[f];
         }
-    }
+    });
 }
 
 }  // namespace
@@ -305,7 +287,7 @@ void CoefGen::validate() const {
     const std::size_t nu = units.size();
     auto bad = [](const char* what) { throw std::runtime_error(std::string("coefficient tables: ") + what); };
     if (!mt || mt->nst != nst) bad("MPO tables");
-    if (nst > WG_NST || gin.size() != nu * nst || line_scale.size() != line_major.size() || smap_slot.size() != smap_id.size())
+    if (nst > wg::NST || gin.size() != nu * nst || line_scale.size() != line_major.size() || smap_slot.size() != smap_id.size())
         bad("unit tables");
     // the MPO tables were checked when built (indices inside the tensor); here: against the boundary
     const uint32_t nmaj = by_row ? mt->rows : mt->cols, nother = by_row ? mt->cols : mt->rows;
@@ -346,6 +328,18 @@ void CoefGen::upload(cudaStream_t s) {
     d_b_cs.upload(*b_cs, s);
 }
 
+WGenTab CoefGen::tables() const {
+    WGenTab t;
+    t.units = d_units.get(); t.gin = d_gin.get(); t.line_major = d_line_major.get(); t.line_scale = d_line_scale.get();
+    t.smap_id = d_smap_id.get(); t.smap_slot = d_smap_slot.get();
+    t.m_ptr = d_m_ptr.get(); t.m_other = d_m_other.get(); t.m_op = d_m_op.get(); t.m_scale = d_m_scale.get();
+    t.o_ptr = d_o_ptr.get(); t.o_in = d_o_in.get(); t.o_val = d_o_val.get();
+    t.b_pos = d_b_pos.get(); t.b_cs = d_b_cs.get();
+    t.nst = nst; t.b_aux = b_aux;
+    t.serial = serial || !(by_row ? mt->row_sorted : mt->col_sorted);
+    return t;
+}
+
 void CoefGen::generate(double* W, cudaStream_t s) {
     generate_range(W, 0, uint32_t(units.size()), 0, w_len, s);
     check_generated(s);
@@ -360,10 +354,7 @@ void CoefGen::generate_range(double* W, uint32_t u0, uint32_t u1, uint64_t w0, u
         d_err.alloc(1);
         QCM_CUDA(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
     }
-    k_wgen<<<unsigned(u1 - u0), WG_THR, 0, s>>>(d_units.get() + u0, d_gin.get() + std::size_t(u0) * nst, nst, d_line_major.get(),
-                                                d_line_scale.get(), d_smap_id.get(), d_smap_slot.get(), d_m_ptr.get(),
-                                                d_m_other.get(), d_m_op.get(), d_m_scale.get(), d_o_ptr.get(), d_o_in.get(),
-                                                d_o_val.get(), d_b_pos.get(), d_b_cs.get(), b_aux, W, w0, d_err.get());
+    k_wgen<<<unsigned(u1 - u0), wg::THR, 0, s>>>(tables(), u0, W, w0, d_err.get());
     QCM_CUDA(cudaGetLastError());
 }
 

@@ -328,6 +328,13 @@ std::shared_ptr<const MPOTables> build_mpo_tables(const MPOTensor& W) {
         const uint32_t e = W.col_ent[q];
         t->col_other[q] = W.b1[e]; t->col_op[q] = W.op[e]; t->col_scale[q] = W.scale[e];
     }
+    auto sorted = [](const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& other) {
+        for (std::size_t i = 0; i + 1 < ptr.size(); ++i)
+            if (!std::is_sorted(other.begin() + ptr[i], other.begin() + ptr[i + 1])) return false;
+        return true;
+    };
+    t->row_sorted = sorted(t->row_ptr, t->row_other);
+    t->col_sorted = sorted(t->col_ptr, t->col_other);
     return t;
 }
 
@@ -348,11 +355,18 @@ void CoefGen::set_boundary(const BoundaryIndexH& B) {
     b_aux = B.aux;
     b_cs = &B.cscale;
     b_pos.resize(B.offsets.size());
+    serial = false;
+    std::vector<uint32_t> seen(B.aux, 0);  // per block position, the last cohort (+ 1) that used it
     for (uint32_t c = 0; c < B.n_cohorts(); ++c) {
         const int64_t bs = std::max<int64_t>(1, int64_t(B.lsz[c]) * B.rsz[c]);
         for (uint32_t b = 0; b < B.aux; ++b) {
             const int64_t o = B.offsets[std::size_t(c) * B.aux + b];
-            b_pos[std::size_t(c) * B.aux + b] = o < 0 ? -1 : int32_t(o / bs);
+            const int32_t pos = o < 0 ? -1 : int32_t(o / bs);
+            b_pos[std::size_t(c) * B.aux + b] = pos;
+            if (pos < 0) continue;
+            // a cohort of distinct blocks has positions below the number of MPO indices
+            serial |= uint32_t(pos) >= B.aux || seen[std::size_t(pos)] == c + 1;
+            if (uint32_t(pos) < B.aux) seen[std::size_t(pos)] = c + 1;
         }
     }
 }
