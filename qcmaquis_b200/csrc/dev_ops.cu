@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NTHR) k_bgemm(const GemmJob* __restrict__ jobs
     const int wm = warp % S::WM, wn = warp / S::WM;
 #pragma unroll
     for (int i = 0; i < S::FM; ++i) {
-        uint32_t gm = tile.m0 + wm * S::FM * 8 + i * 8 + r;
+        uint32_t gm = tile.m0 + S::row(i, wm) + r;
         if (gm >= J.M) continue;
         uint64_t base = J.c_off;
         if (J.crb) {

@@ -37,6 +37,9 @@ struct Shape {
     static constexpr int BM = WM * FM * 8, BN = WN * FN * 8;
     static constexpr int A_PER = BM * BK / NTHR, B_PER = BN * BK / NTHR;
     static_assert(WM * WN * 32 == NTHR, "4 warps per CTA");
+    // first row of fragment i of a warp in warp row wm: the warp rows take fragments in turn, so that the rows
+    // missing from a tile are missing from all warps alike
+    __host__ __device__ static constexpr int row(int i, int wm) { return (i * WM + wm) * 8; }
 };
 using Sh16 = Shape<1, 4, 2, 4>;  // 16 x 128
 using Sh32 = Shape<1, 4, 4, 4>;  // 32 x 128
@@ -69,7 +72,7 @@ static __device__ __forceinline__ void mma_stage(const double (*A)[S::BM + PAD],
     for (int kk = 0; kk < BK; kk += 4) {
         double a[S::FM], b[S::FN];
 #pragma unroll
-        for (int i = 0; i < S::FM; ++i) a[i] = A[kk + q][wm * S::FM * 8 + i * 8 + r];
+        for (int i = 0; i < S::FM; ++i) a[i] = A[kk + q][S::row(i, wm) + r];
 #pragma unroll
         for (int j = 0; j < S::FN; ++j) b[j] = B[kk + q][wn * S::FN * 8 + j * 8 + r];
 #pragma unroll
@@ -90,13 +93,48 @@ static __device__ __forceinline__ void mma_stage_masked(const double (*A)[S::BM 
         if (!((mask >> (kk / 4)) & 1u)) continue;
         double a[S::FM], b[S::FN];
 #pragma unroll
-        for (int i = 0; i < S::FM; ++i) a[i] = A[kk + q][wm * S::FM * 8 + i * 8 + r];
+        for (int i = 0; i < S::FM; ++i) a[i] = A[kk + q][S::row(i, wm) + r];
 #pragma unroll
         for (int j = 0; j < S::FN; ++j) b[j] = B[kk + q][wn * S::FN * 8 + j * 8 + r];
 #pragma unroll
         for (int i = 0; i < S::FM; ++i)
 #pragma unroll
             for (int j = 0; j < S::FN; ++j) dmma(acc.c[i][j], a[i], b[j]);
+    }
+}
+
+// Operand staged with k fastest (its k elements contiguous in memory): element (x, k) of a stage at x * BK +
+// (k ^ 4 (x mod 4)).  Rows of 128 bytes without padding; the swizzle puts the 4 k's of 4 neighbouring x's in 16
+// different 8-byte banks for the fragment reads, and keeps pairs of k (16-byte copies) together.
+static __device__ __forceinline__ int kfast(int x, int k) { return x * BK + (k ^ ((x & 3) << 2)); }
+
+// One stage with each operand in either layout (AK, BKF: k fastest), leaving out what lies beyond the operands:
+// row fragments past nfm (of the tile's BM / 8) and k groups of 4 past ng.
+template <class S, bool AK, bool BKF>
+static __device__ __forceinline__ void mma_stage_part(const double* A, const double* B, Acc<S>& acc, int warp, int lane, int nfm,
+                                                      int ng) {
+    const int r = lane >> 2, q = lane & 3;
+    const int wm = warp % S::WM, wn = warp / S::WM;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+        if (kk >= 4 * ng) break;
+        double a[S::FM], b[S::FN];
+#pragma unroll
+        for (int i = 0; i < S::FM; ++i) {
+            const int m = S::row(i, wm) + r;
+            a[i] = A[AK ? kfast(m, kk + q) : (kk + q) * (S::BM + PAD) + m];
+        }
+#pragma unroll
+        for (int j = 0; j < S::FN; ++j) {
+            const int n = wn * S::FN * 8 + j * 8 + r;
+            b[j] = B[BKF ? kfast(n, kk + q) : (kk + q) * (S::BN + PAD) + n];
+        }
+#pragma unroll
+        for (int i = 0; i < S::FM; ++i) {
+            if (i * S::WM + wm >= nfm) break;
+#pragma unroll
+            for (int j = 0; j < S::FN; ++j) dmma(acc.c[i][j], a[i], b[j]);
+        }
     }
 }
 
@@ -110,7 +148,7 @@ static __device__ __forceinline__ void for_acc(const Acc<S>& acc, int warp, int 
 #pragma unroll
         for (int j = 0; j < S::FN; ++j)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) f(wm * S::FM * 8 + i * 8 + r, wn * S::FN * 8 + j * 8 + q * 2 + c, acc.c[i][j][c]);
+            for (int c = 0; c < 2; ++c) f(S::row(i, wm) + r, wn * S::FN * 8 + j * 8 + q * 2 + c, acc.c[i][j][c]);
 }
 
 

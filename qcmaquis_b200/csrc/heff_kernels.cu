@@ -25,6 +25,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <stdexcept>
+#include <type_traits>
 
 #include "dmma.cuh"
 #include "heff.hpp"
@@ -34,6 +35,55 @@ namespace qcm {
 namespace {
 
 using namespace dm;
+
+// ---------------------------------------------------------------------------
+// Staging of one operand of a stage (X x BK elements, X = BM or BN) in one of three ways.  get(x, k): pointer to
+// element (x, k); nx, nk: how many x and k of the stage exist (elements past them are zero).
+//   k contiguous in memory: k fastest in shared memory (kfast), 16 bytes at a time if v16 (every k pair starts on
+//     16 bytes and nk is even), else 8;
+//   x contiguous: rows of X + PAD elements per k, 16 bytes at a time if v16 (nx even), else 8.
+template <int X, class Get>
+__device__ __forceinline__ void stage_kfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
+    const int tid = threadIdx.x;
+    if (v16) {
+        constexpr int CH = X * BK / 2;
+        static_assert(CH % NTHR == 0, "whole chunks per thread");
+#pragma unroll
+        for (int rr = 0; rr < CH / NTHR; ++rr) {
+            const int e = tid + rr * NTHR, k = 2 * (e % (BK / 2)), x = e / (BK / 2);
+            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
+            cp16(dst + kfast(x, k), ok ? get(x, k) : any, ok);
+        }
+    } else {
+#pragma unroll
+        for (int rr = 0; rr < X * BK / NTHR; ++rr) {
+            const int e = tid + rr * NTHR, k = e % BK, x = e / BK;
+            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
+            cp8(dst + kfast(x, k), ok ? get(x, k) : any, ok);
+        }
+    }
+}
+template <int X, class Get>
+__device__ __forceinline__ void stage_xfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
+    const int tid = threadIdx.x;
+    if (v16) {
+        constexpr int CH = X * BK / 2;
+#pragma unroll
+        for (int rr = 0; rr < CH / NTHR; ++rr) {
+            const int e = tid + rr * NTHR, x = 2 * (e % (X / 2)), k = e / (X / 2);
+            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
+            cp16(dst + k * (X + PAD) + x, ok ? get(x, k) : any, ok);
+        }
+    } else {
+#pragma unroll
+        for (int rr = 0; rr < X * BK / NTHR; ++rr) {
+            const int e = tid + rr * NTHR, x = e % X, k = e / X;
+            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
+            cp8(dst + k * (X + PAD) + x, ok ? get(x, k) : any, ok);
+        }
+    }
+}
+__device__ __forceinline__ bool aligned16(const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---------------------------------------------------------------------------
 // T-GEMM: one CTA per (job, tile)
@@ -46,57 +96,46 @@ __global__ void __launch_bounds__(NTHR, 5) k_tgemm(const TJobD* __restrict__ job
     const TileD tile = tiles[blockIdx.x];
     const TJobD J = jobs[tile.item];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int c = tid; c < S::BN; c += NTHR) {
-        uint32_t n = tile.n0 + c;
-        uint64_t cb = J.b_off;
-        if (n < J.N) {
-            uint32_t b = n / J.brs, j = n - b * J.brs;
-            cb = J.b_off + uint64_t(b) * J.K * J.brs + (J.tr ? uint64_t(j) : uint64_t(j) * J.K);
-        }
-        colbase[c] = cb;
-    }
-    __syncthreads();
-    const uint64_t kstride = J.tr ? J.brs : 1;
-    auto issue = [&](int sidx, uint32_t k0) {
-        Stage<S>& s = st[sidx];
-#pragma unroll
-        for (int rr = 0; rr < S::A_PER; ++rr) {
-            int e = tid + rr * NTHR;
-            int m = e % S::BM, k = e / S::BM;
-            uint32_t gm = tile.m0 + m, gk = k0 + k;
-            bool ok = gm < J.M && gk < J.K;
-            cp8(&s.A[k][m], ok ? x + J.a_off + gm + uint64_t(gk) * J.lda : x, ok);
-        }
-        if (!J.tr) {
-#pragma unroll
-            for (int rr = 0; rr < S::B_PER; ++rr) {
-                int e = tid + rr * NTHR;
-                int k = e % BK, n = e / BK;
-                uint32_t gn = tile.n0 + n, gk = k0 + k;
-                bool ok = gn < J.N && gk < J.K;
-                cp8(&s.B[k][n], ok ? R + colbase[n] + gk : R, ok);
-            }
-        } else {
-#pragma unroll
-            for (int rr = 0; rr < S::B_PER; ++rr) {
-                int e = tid + rr * NTHR;
-                int n = e % S::BN, k = e / S::BN;
-                uint32_t gn = tile.n0 + n, gk = k0 + k;
-                bool ok = gn < J.N && gk < J.K;
-                cp8(&s.B[k][n], ok ? R + colbase[n] + uint64_t(gk) * kstride : R, ok);
-            }
-        }
-        cp_commit();
-    };
+    const uint32_t nm = min(uint32_t(S::BM), J.M - tile.m0), nn = min(uint32_t(S::BN), J.N - tile.n0);
+    const uint32_t nk = (J.K + BK - 1) / BK;
+    const int nfm = int(nm + 7) / 8;
+    const double* xa = x + J.a_off + tile.m0;
+    const bool a16 = !((J.lda | nm) & 1u) && aligned16(xa);
     Acc<S> acc;
     acc.zero();
-    const uint32_t nk = (J.K + BK - 1) / BK;
-    issue(0, 0);
-    for (uint32_t kc = 0; kc < nk; ++kc) {
-        cp_wait_all();
+    auto loop = [&](auto issue, auto tr) {
+        issue(st[0], 0);
+        for (uint32_t kc = 0; kc < nk; ++kc) {
+            cp_wait_all();
+            __syncthreads();
+            if (kc + 1 < nk) issue(st[(kc + 1) & 1], (kc + 1) * BK);
+            const Stage<S>& s = st[kc & 1];
+            mma_stage_part<S, false, !decltype(tr)::value>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm,
+                                                           int(min(uint32_t(BK), J.K - kc * BK) + 3) / 4);
+        }
+    };
+    if (!J.tr) {
+        // R's columns are K contiguous elements each, one column after the other
+        const double* rb = R + J.b_off + uint64_t(tile.n0) * J.K;
+        const bool b16 = !(J.K & 1u) && aligned16(rb);
+        loop([&](Stage<S>& s, uint32_t k0) {
+            stage_xfast<S::BM>(&s.A[0][0], x, nm, J.K - k0, a16, [&](int m, int k) { return xa + m + uint64_t(k0 + k) * J.lda; });
+            stage_kfast<S::BN>(&s.B[0][0], R, nn, J.K - k0, b16, [&](int n, int k) { return rb + uint64_t(n) * J.K + k0 + k; });
+            cp_commit();
+        }, std::false_type{});
+    } else {
+        // each block transposed: column n of block b at b * K * brs + n % brs, k in steps of brs
+        for (int c = tid; c < S::BN; c += NTHR) {
+            const uint32_t n = tile.n0 + c, b = n / J.brs;
+            colbase[c] = n < J.N ? J.b_off + uint64_t(b) * J.K * J.brs + (n - b * J.brs) : J.b_off;
+        }
         __syncthreads();
-        if (kc + 1 < nk) issue((kc + 1) & 1, (kc + 1) * BK);
-        mma_stage<S>(st[kc & 1].A, st[kc & 1].B, acc, warp, lane);
+        loop([&](Stage<S>& s, uint32_t k0) {
+            stage_xfast<S::BM>(&s.A[0][0], x, nm, J.K - k0, a16, [&](int m, int k) { return xa + m + uint64_t(k0 + k) * J.lda; });
+            stage_xfast<S::BN>(&s.B[0][0], R, nn, J.K - k0, false,
+                               [&](int n, int k) { return R + colbase[n] + uint64_t(k0 + k) * J.brs; });
+            cp_commit();
+        }, std::true_type{});
     }
     // the thread's output columns: FN fragments x 2 columns each; their T offsets once (slice
     // blk at blk * sst, column within it at (n % brs) * M)
@@ -115,7 +154,7 @@ __global__ void __launch_bounds__(NTHR, 5) k_tgemm(const TJobD* __restrict__ job
         }
 #pragma unroll
     for (int i = 0; i < S::FM; ++i) {
-        const uint32_t gm = tile.m0 + wm * S::FM * 8 + i * 8 + r;
+        const uint32_t gm = tile.m0 + S::row(i, wm) + r;
         if (gm >= J.M) continue;
 #pragma unroll
         for (int j = 0; j < S::FN; ++j)
@@ -230,7 +269,7 @@ __global__ void __launch_bounds__(NTHR, 5) k_sgemm(const UnitD* __restrict__ uni
         }
 #pragma unroll
     for (int i = 0; i < S::FM; ++i) {
-        const uint32_t gl = tile.m0 + wm * S::FM * 8 + i * 8 + r;
+        const uint32_t gl = tile.m0 + S::row(i, wm) + r;
         if (gl >= U.nl) continue;
         double* srow = Sm + U.s_off + uint64_t(line_b1[U.line0 + gl]) * U.line_stride;
 #pragma unroll
@@ -384,65 +423,66 @@ __global__ void __launch_bounds__(NTHR) k_lspart(const KItemD* __restrict__ item
     const SegD sg = segs[it.seg];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t M = O.M, Kc = sg.nS * sg.ls_in;
+    const uint32_t nm = min(uint32_t(S::BM), M - ot.m0), nn = min(uint32_t(S::BN), O.N - ot.n0);
+    const int nfm = int(nm + 7) / 8;
     const uint64_t blk = uint64_t(M) * sg.ls_in;
-    // L column bases of a stage's 16 k rows, written two stages ahead so that the loop's barrier
-    // publishes them before their stage is issued
-    auto bases = [&](int sidx, uint32_t k0) {
-        if (tid < BK) {
-            uint32_t kk = k0 + tid;
-            uint64_t kb = sg.l_off;
-            if (kk < it.k1) {
-                uint32_t b = kk / sg.ls_in, j = kk - b * sg.ls_in;
-                kb = sg.l_off + b * blk + (sg.tr ? uint64_t(j) : uint64_t(j) * M);
-            }
-            kbase[sidx][tid] = kb;
-        }
-    };
-    auto issue = [&](int sidx, uint32_t k0) {
-        Stage<S>& s = st[sidx];
-        if (!sg.tr) {
-#pragma unroll
-            for (int rr = 0; rr < S::A_PER; ++rr) {
-                int e = tid + rr * NTHR;
-                int m = e % S::BM, k = e / S::BM;
-                uint32_t gm = ot.m0 + m, gk = k0 + k;
-                bool ok = gm < M && gk < it.k1;
-                cp8(&s.A[k][m], ok ? Lb + kbase[sidx][k] + gm : Lb, ok);
-            }
-        } else {
-#pragma unroll
-            for (int rr = 0; rr < S::A_PER; ++rr) {
-                int e = tid + rr * NTHR;
-                int k = e % BK, m = e / BK;
-                uint32_t gm = ot.m0 + m, gk = k0 + k;
-                bool ok = gm < M && gk < it.k1;
-                cp8(&s.A[k][m], ok ? Lb + kbase[sidx][k] + uint64_t(gm) * sg.ls_in : Lb, ok);
-            }
-        }
-#pragma unroll
-        for (int rr = 0; rr < S::B_PER; ++rr) {
-            int e = tid + rr * NTHR;
-            int k = e % BK, n = e / BK;
-            uint32_t gn = ot.n0 + n, gk = k0 + k;
-            bool ok = gn < O.N && gk < it.k1;
-            cp8(&s.B[k][n], ok ? Sm + sg.s_off + gk + uint64_t(gn) * Kc : Sm, ok);
-        }
-        cp_commit();
-    };
+    // S columns are Kc contiguous elements; pairs of k start on 16 bytes if Kc is even (k0 is)
+    const double* sb = Sm + sg.s_off + uint64_t(ot.n0) * Kc;
+    const bool b16 = !((Kc | it.k0) & 1u) && aligned16(sb);
+    // L's blocks one after the other are M contiguous rows per column
+    const double* la = Lb + sg.l_off + ot.m0;
+    const bool a16 = !((M | nm) & 1u) && aligned16(la);
     Acc<S> acc;
     acc.zero();
     const uint32_t nk = (it.k1 - it.k0 + BK - 1) / BK;
-    bases(0, it.k0);
-    bases(1, it.k0 + BK);
-    __syncthreads();
-    issue(0, it.k0);
-    for (uint32_t kc = 0; kc < nk; ++kc) {
-        cp_wait_all();
+    auto stage_s = [&](Stage<S>& s, uint32_t k0) {
+        stage_kfast<S::BN>(&s.B[0][0], Sm, nn, it.k1 - k0, b16, [&](int n, int k) { return sb + uint64_t(n) * Kc + k0 + k; });
+        cp_commit();
+    };
+    auto mma = [&](uint32_t kc, auto tr) {
+        const Stage<S>& s = st[kc & 1];
+        mma_stage_part<S, decltype(tr)::value, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm,
+                                                     int(min(uint32_t(BK), it.k1 - it.k0 - kc * BK) + 3) / 4);
+    };
+    if (!sg.tr) {
+        auto issue = [&](Stage<S>& s, uint32_t k0) {
+            stage_xfast<S::BM>(&s.A[0][0], Lb, nm, it.k1 - k0, a16, [&](int m, int k) { return la + m + uint64_t(k0 + k) * M; });
+            stage_s(s, k0);
+        };
+        issue(st[0], it.k0);
+        for (uint32_t kc = 0; kc < nk; ++kc) {
+            cp_wait_all();
+            __syncthreads();
+            if (kc + 1 < nk) issue(st[(kc + 1) & 1], it.k0 + (kc + 1) * BK);
+            mma(kc, std::false_type{});
+        }
+    } else {
+        // L^T: element (m, k) of block b = k / ls_in at b * blk + k % ls_in + m * ls_in.  The bases of a stage's 16
+        // k's are written two stages ahead, so that the loop's barrier publishes them before their stage is issued
+        auto bases = [&](int sidx, uint32_t k0) {
+            if (tid < BK) {
+                const uint32_t kk = k0 + tid, b = kk / sg.ls_in;
+                kbase[sidx][tid] = kk < it.k1 ? sg.l_off + b * blk + (kk - b * sg.ls_in) : sg.l_off;
+            }
+        };
+        auto issue = [&](int sidx, uint32_t k0) {
+            Stage<S>& s = st[sidx];
+            stage_kfast<S::BM>(&s.A[0][0], Lb, nm, it.k1 - k0, false,
+                               [&](int m, int k) { return Lb + kbase[sidx][k] + uint64_t(ot.m0 + m) * sg.ls_in; });
+            stage_s(s, k0);
+        };
+        bases(0, it.k0);
+        bases(1, it.k0 + BK);
         __syncthreads();
-        if (kc + 1 < nk) issue((kc + 1) & 1, it.k0 + (kc + 1) * BK);
-        // stage kc's bases were consumed when it was issued: the buffer takes stage kc + 2's
-        if (kc + 2 < nk) bases(kc & 1, it.k0 + (kc + 2) * BK);
-        mma_stage<S>(st[kc & 1].A, st[kc & 1].B, acc, warp, lane);
+        issue(0, it.k0);
+        for (uint32_t kc = 0; kc < nk; ++kc) {
+            cp_wait_all();
+            __syncthreads();
+            if (kc + 1 < nk) issue((kc + 1) & 1, it.k0 + (kc + 1) * BK);
+            // stage kc's bases were consumed when it was issued: the buffer takes stage kc + 2's
+            if (kc + 2 < nk) bases(kc & 1, it.k0 + (kc + 2) * BK);
+            mma(kc, std::true_type{});
+        }
     }
     double* Pt = P + uint64_t(it.slot) * S::BM * S::BN;
     for_acc<S>(acc, warp, lane, [&](int m, int n, double v) { Pt[m + n * S::BM] = v; });
