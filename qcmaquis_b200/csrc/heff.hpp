@@ -286,7 +286,10 @@ struct HeffPlan {
     std::vector<OutD> outs;
     std::vector<OTileD> otiles[N_SHAPES];
     std::vector<KItemD> kitems[N_SHAPES];
-    uint64_t p_len = 0;  // split-K partial tiles (doubles)
+    // split-K partial tiles (doubles); each tile shape's from p_off on (p_apart), or all shapes' in one region
+    // that they take in turn
+    uint64_t p_len = 0, p_off[N_SHAPES] = {};
+    bool p_apart = false;
 
     // reference work count ScheduleNew::total_flops (tasks.cpp:388-398, 777-796)
     double flops = 0, flops_t = 0, flops_ls = 0, flops_s = 0;
@@ -377,6 +380,9 @@ struct HeffPlan {
     ~HeffPlan();
 };
 
+// Places a plan's split-K partials: every tile shape's in a region of its own (one launch for all shapes), unless
+// t_len + s_len + p_len would pass `limit` for that reason alone (then one shared region, a launch per shape)
+void place_partials(HeffPlan& p, uint64_t limit);
 std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& L, const DevBoundary& R, const MPOTensor& W,
                                           const Index& phys, const Index& left, const Index& right, bool bookkeeping);
 // Stages a plan on the device: its coefficient blocks (generated on the device) and, with lists, its

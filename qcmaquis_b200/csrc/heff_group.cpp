@@ -121,9 +121,7 @@ std::unique_ptr<HeffPlan> merge_plans(const std::vector<HeffPlan*>& plans, std::
     g->x_len = xl;
     g->t_len = tl;
     g->s_len = sl;
-    uint64_t pl = 0;
-    for (int sh = 0; sh < N_SHAPES; ++sh) pl = std::max<uint64_t>(pl, kl_items[sh] * shape_bm(sh) * shape_bn(sh));
-    g->p_len = pl;
+    place_partials(*g, ~uint64_t(0));
     static const bool tdbg = std::getenv("QCM_PLAN_TIMING") != nullptr;
     const auto t0 = std::chrono::steady_clock::now();
     upload_merged(*g);

@@ -86,14 +86,36 @@ __device__ __forceinline__ void stage_xfast(double* dst, const double* any, uint
 __device__ __forceinline__ bool aligned16(const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---------------------------------------------------------------------------
+// The tiles of a phase in all its shapes, one launch: the CTA's tile is looked up by running ends in the order
+// 128-, 64-, 32-, 16-row tiles.  A launch per shape left the chip idle at the end of each one: a few long 128-row
+// tiles alone took as long as a tenth of the phase.  Shared memory is the largest shape's; registers are set by
+// the launch bounds in any case.
+template <class D>
+struct TileSet {
+    const D* t[N_SHAPES];
+    uint32_t end[N_SHAPES];  // running ends, shapes from 128 rows down
+    // shape and tile of CTA b (constant indices: the arrays stay in parameter space)
+    __device__ __forceinline__ int find(uint32_t b, D& d) const {
+        if (b < end[SHAPE_128]) { d = t[SHAPE_128][b]; return SHAPE_128; }
+        if (b < end[SHAPE_64]) { d = t[SHAPE_64][b - end[SHAPE_128]]; return SHAPE_64; }
+        if (b < end[SHAPE_32]) { d = t[SHAPE_32][b - end[SHAPE_64]]; return SHAPE_32; }
+        d = t[SHAPE_16][b - end[SHAPE_32]];
+        return SHAPE_16;
+    }
+};
+template <class... S>
+constexpr std::size_t stage_bytes() {
+    std::size_t m = 0;
+    ((m = sizeof(Stage<S>) > m ? sizeof(Stage<S>) : m), ...);
+    return 2 * m;
+}
+
+// ---------------------------------------------------------------------------
 // T-GEMM: one CTA per (job, tile)
 template <class S>
-__global__ void __launch_bounds__(NTHR, 5) k_tgemm(const TJobD* __restrict__ jobs, const TileD* __restrict__ tiles,
-                                                const double* __restrict__ x, const double* __restrict__ R,
-                                                double* __restrict__ T, float* __restrict__ Thi, float* __restrict__ Tlo) {
-    __shared__ Stage<S> st[2];
-    __shared__ uint64_t colbase[S::BN];
-    const TileD tile = tiles[blockIdx.x];
+__device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, const TileD& tile, const TJobD* __restrict__ jobs,
+                                           const double* __restrict__ x, const double* __restrict__ R, double* __restrict__ T,
+                                           float* __restrict__ Thi, float* __restrict__ Tlo) {
     const TJobD J = jobs[tile.item];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nm = min(uint32_t(S::BM), J.M - tile.m0), nn = min(uint32_t(S::BN), J.N - tile.n0);
@@ -179,15 +201,25 @@ __global__ void __launch_bounds__(NTHR, 5) k_tgemm(const TJobD* __restrict__ job
     }
 }
 
+__global__ void __launch_bounds__(NTHR, 5) k_tgemm(TileSet<TileD> set, const TJobD* __restrict__ jobs,
+                                                   const double* __restrict__ x, const double* __restrict__ R,
+                                                   double* __restrict__ T, float* __restrict__ Thi, float* __restrict__ Tlo) {
+    __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64>()];
+    __shared__ uint64_t colbase[128];
+    TileD tile;
+    const int sh = set.find(blockIdx.x, tile);
+    if (sh == SHAPE_64) tgemm_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+    else if (sh == SHAPE_32) tgemm_tile<Sh32>(reinterpret_cast<Stage<Sh32>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+    else tgemm_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+}
+
 // ---------------------------------------------------------------------------
 // S build: one CTA per (unit, line tile, element tile)
 template <class S>
-__global__ void __launch_bounds__(NTHR, 5) k_sgemm(const UnitD* __restrict__ units, const TileD* __restrict__ tiles,
-                                                const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
-                                                const uint16_t* __restrict__ klist, const double* __restrict__ W,
-                                                const double* __restrict__ T, double* __restrict__ Sm, uint64_t w0) {
-    __shared__ Stage<S> st[2];
-    const TileD tile = tiles[blockIdx.x];
+__device__ __forceinline__ void sgemm_tile(Stage<S>* st, const TileD& tile, const UnitD* __restrict__ units,
+                                           const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
+                                           const uint16_t* __restrict__ klist, const double* __restrict__ W,
+                                           const double* __restrict__ T, double* __restrict__ Sm, uint64_t w0) {
     const UnitD U = units[tile.item];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // only the k-steps whose coefficient block (this tile's lines x 16 slices) holds an entry
@@ -278,6 +310,19 @@ __global__ void __launch_bounds__(NTHR, 5) k_sgemm(const UnitD* __restrict__ uni
             for (int c = 0; c < 2; ++c)
                 if (cof[j][c] != 0xffffffffu) srow[cof[j][c]] = acc.c[i][j][c];
     }
+}
+
+__global__ void __launch_bounds__(NTHR, 5) k_sgemm(TileSet<TileD> set, const UnitD* __restrict__ units,
+                                                   const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
+                                                   const uint16_t* __restrict__ klist, const double* __restrict__ W,
+                                                   const double* __restrict__ T, double* __restrict__ Sm, uint64_t w0) {
+    __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64, Sh128>()];
+    TileD tile;
+    const int sh = set.find(blockIdx.x, tile);
+    if (sh == SHAPE_128) sgemm_tile<Sh128>(reinterpret_cast<Stage<Sh128>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
+    else if (sh == SHAPE_64) sgemm_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
+    else if (sh == SHAPE_32) sgemm_tile<Sh32>(reinterpret_cast<Stage<Sh32>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
+    else sgemm_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
 }
 
 // One CTA per unit: the coefficient terms of its lines (CoefGen), in MPO-entry then operator-term order, summed
@@ -411,13 +456,10 @@ namespace {
 // ---------------------------------------------------------------------------
 // L.S GEMM, split-K: item = (output tile, segment, K range) -> partial tile P[item]
 template <class S>
-__global__ void __launch_bounds__(NTHR) k_lspart(const KItemD* __restrict__ items, const OTileD* __restrict__ otiles,
-                                                 const OutD* __restrict__ outs, const SegD* __restrict__ segs,
-                                                 const double* __restrict__ Lb, const double* __restrict__ Sm,
-                                                 double* __restrict__ P) {
-    __shared__ Stage<S> st[2];
-    __shared__ uint64_t kbase[2][BK];
-    const KItemD it = items[blockIdx.x];
+__device__ __forceinline__ void lspart_tile(Stage<S>* st, uint64_t (*kbase)[BK], const KItemD& it, const OTileD* __restrict__ otiles,
+                                            const OutD* __restrict__ outs, const SegD* __restrict__ segs,
+                                            const double* __restrict__ Lb, const double* __restrict__ Sm,
+                                            double* __restrict__ P) {
     const OTileD ot = otiles[it.tile];
     const OutD O = outs[ot.out];
     const SegD sg = segs[it.seg];
@@ -488,92 +530,134 @@ __global__ void __launch_bounds__(NTHR) k_lspart(const KItemD* __restrict__ item
     for_acc<S>(acc, warp, lane, [&](int m, int n, double v) { Pt[m + n * S::BM] = v; });
 }
 
+// what the L.S kernels need of each shape: its output tiles, and its partial tiles in P
+struct OTileSet {
+    const OTileD* t[N_SHAPES];
+    uint64_t part[N_SHAPES];
+};
+__global__ void __launch_bounds__(NTHR, 4) k_lspart(TileSet<KItemD> set, OTileSet ots, const OutD* __restrict__ outs,
+                                                    const SegD* __restrict__ segs, const double* __restrict__ Lb,
+                                                    const double* __restrict__ Sm, double* __restrict__ P) {
+    __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64>()];
+    __shared__ uint64_t kbase[2][BK];
+    KItemD it;
+    const int sh = set.find(blockIdx.x, it);
+    if (sh == SHAPE_64)
+        lspart_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), kbase, it, ots.t[SHAPE_64], outs, segs, Lb, Sm, P + ots.part[SHAPE_64]);
+    else if (sh == SHAPE_32)
+        lspart_tile<Sh32>(reinterpret_cast<Stage<Sh32>*>(raw), kbase, it, ots.t[SHAPE_32], outs, segs, Lb, Sm, P + ots.part[SHAPE_32]);
+    else
+        lspart_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), kbase, it, ots.t[SHAPE_16], outs, segs, Lb, Sm, P + ots.part[SHAPE_16]);
+}
+
 // Sum the partial tiles of each output tile in item order and write y.  Grid: (output tile, 256-element
 // chunk of the tile).
-template <class S>
-__global__ void __launch_bounds__(256) k_lsreduce(const OTileD* __restrict__ otiles, const OutD* __restrict__ outs,
+__global__ void __launch_bounds__(256) k_lsreduce(TileSet<OTileD> set, OTileSet ots, const OutD* __restrict__ outs,
                                                   const double* __restrict__ P, double* __restrict__ y) {
     // one thread per tile element (blockIdx.y: the tile's 256-element chunk): the element's partials are
     // added in item order; the unrolled loop keeps several of its loads in flight
-    const OTileD ot = otiles[blockIdx.x];
+    OTileD ot;
+    const int sh = set.find(blockIdx.x, ot);
+    const uint32_t bm = sh == SHAPE_64 ? Sh64::BM : (sh == SHAPE_32 ? Sh32::BM : Sh16::BM);
+    const uint32_t bn = sh == SHAPE_64 ? Sh64::BN : Sh32::BN;
     const OutD O = outs[ot.out];
-    const int e = int(blockIdx.y) * int(blockDim.x) + int(threadIdx.x);
-    if (e >= S::BM * S::BN) return;
-    const int m = e % S::BM, n = e / S::BM;
-    const uint32_t gm = ot.m0 + m, gn = ot.n0 + n;
+    const uint32_t e = blockIdx.y * blockDim.x + threadIdx.x;
+    if (e >= bm * bn) return;
+    const uint32_t gm = ot.m0 + e % bm, gn = ot.n0 + e / bm;
     if (gm >= O.M || gn >= O.N) return;
-    const double* Pe = P + uint64_t(ot.part0) * S::BM * S::BN + e;
+    const uint64_t p0 = sh == SHAPE_64 ? ots.part[SHAPE_64] : (sh == SHAPE_32 ? ots.part[SHAPE_32] : ots.part[SHAPE_16]);
+    const double* Pe = P + p0 + uint64_t(ot.part0) * bm * bn + e;
     double s = 0.0;
 #pragma unroll 8
-    for (uint32_t p = 0; p < ot.nparts; ++p) s += Pe[uint64_t(p) * S::BM * S::BN];
+    for (uint32_t p = 0; p < ot.nparts; ++p) s += Pe[uint64_t(p) * bm * bn];
     y[O.y_off + gm + uint64_t(gn) * O.M] = s;
 }
 
-template <class S>
-void launch_t(HeffPlan& p, int sh, const double* x, double* Tb, cudaStream_t s, float* Thi = nullptr,
-              float* Tlo = nullptr) {
-    if (!p.ttiles[sh].empty())
-        k_tgemm<S><<<unsigned(p.ttiles[sh].size()), NTHR, 0, s>>>(p.d_tjobs.get(), p.d_ttiles[sh].get(), x,
-                                                                  p.r_data(), Tb, Thi, Tlo);
+// the tiles [a[sh], b[sh]) of every shape (only one shape if `only` >= 0); n: how many in all
+template <class D>
+TileSet<D> tile_set(const DBuf<D>* t, const uint32_t* a, const uint32_t* b, uint32_t& n, int only = -1) {
+    TileSet<D> r;
+    n = 0;
+    for (int sh = N_SHAPES - 1; sh >= 0; --sh) {
+        r.t[sh] = t[sh].get() + a[sh];
+        if (only < 0 || sh == only) n += b[sh] - a[sh];
+        r.end[sh] = n;
+    }
+    return r;
+}
+template <class D>
+TileSet<D> tile_set(const DBuf<D>* t, const std::vector<D>* h, uint32_t& n, int only = -1) {
+    uint32_t a[N_SHAPES] = {}, b[N_SHAPES];
+    for (int sh = 0; sh < N_SHAPES; ++sh) b[sh] = uint32_t(h[sh].size());
+    return tile_set(t, a, b, n, only);
 }
 
-template <class S>
-void launch_s(HeffPlan& p, int sh, const double* Tb, double* Sb, cudaStream_t s) {
-    if (!p.utiles[sh].empty())
-        k_sgemm<S><<<unsigned(p.utiles[sh].size()), NTHR, 0, s>>>(p.d_units.get(), p.d_utiles[sh].get(), p.d_line_b1.get(),
-                                                                  p.d_slice_off.get(), p.d_klist.get(), p.w_data(), Tb, Sb, 0);
+void launch_t(HeffPlan& p, const double* x, double* Tb, cudaStream_t s, float* Thi = nullptr, float* Tlo = nullptr) {
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(p.d_ttiles, p.ttiles, n);
+    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, p.d_tjobs.get(), x, p.r_data(), Tb, Thi, Tlo);
+}
+
+void launch_s(HeffPlan& p, const double* Tb, double* Sb, cudaStream_t s) {
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(p.d_utiles, p.utiles, n);
+    if (n)
+        k_sgemm<<<n, NTHR, 0, s>>>(set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.w_data(), Tb,
+                                   Sb, 0);
 }
 
 // one ket-sector chunk's T-GEMM tiles, S-GEMM tiles and L.S items (T, S and the coefficient blocks from
 // their chunk bases on)
-template <class S>
-void launch_t_chunk(HeffPlan& p, int sh, const HeffPlan::SChunk& c, const double* x, double* Tb, cudaStream_t s) {
-    const uint32_t a = c.tt[0][sh], b = c.tt[1][sh];
-    if (b > a)
-        k_tgemm<S><<<unsigned(b - a), NTHR, 0, s>>>(p.d_tjobs.get(), p.d_ttiles[sh].get() + a, x, p.r_data(), Tb, nullptr,
-                                                    nullptr);
+void launch_t_chunk(HeffPlan& p, const HeffPlan::SChunk& c, const double* x, double* Tb, cudaStream_t s) {
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(p.d_ttiles, c.tt[0], c.tt[1], n);
+    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, p.d_tjobs.get(), x, p.r_data(), Tb, nullptr, nullptr);
 }
 
-template <class S>
-void launch_s_chunk(HeffPlan& p, int sh, const HeffPlan::SChunk& c, uint64_t w0, const double* Tb, double* Sb,
+// the S-GEMM tiles [a[sh], b[sh]), reading coefficient blocks that start at element w0
+void launch_s_tiles(HeffPlan& p, const uint32_t* a, const uint32_t* b, uint64_t w0, const double* Tb, double* Sb,
                     cudaStream_t s) {
-    const uint32_t a = c.ut[0][sh], b = c.ut[1][sh];
-    if (b > a)
-        k_sgemm<S><<<unsigned(b - a), NTHR, 0, s>>>(p.d_units.get(), p.d_utiles[sh].get() + a, p.d_line_b1.get(),
-                                                    p.d_slice_off.get(), p.d_klist.get(), p.d_W.get(), Tb, Sb, w0);
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(p.d_utiles, a, b, n);
+    if (n)
+        k_sgemm<<<n, NTHR, 0, s>>>(set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.d_W.get(), Tb,
+                                   Sb, w0);
 }
 
-template <class S>
-void launch_ls_chunk(HeffPlan& p, int sh, const HeffPlan::SChunk& c, const double* Sb, double* Pb, cudaStream_t s) {
-    const uint32_t a = c.kt[0][sh], b = c.kt[1][sh];
-    if (b > a)
-        k_lspart<S><<<unsigned(b - a), NTHR, 0, s>>>(p.d_kitems[sh].get() + a, p.d_otiles[sh].get(), p.d_outs.get(),
-                                                     p.d_segs.get(), p.l_data(), Sb, Pb + p.pc_off[sh]);
+OTileSet otile_set(const HeffPlan& p) {
+    OTileSet o;
+    for (int sh = 0; sh < N_SHAPES; ++sh) {
+        o.t[sh] = p.d_otiles[sh].get();
+        o.part[sh] = p.sector_chunked() ? p.pc_off[sh] : p.p_off[sh];
+    }
+    return o;
 }
 
-template <class S>
-void launch_lsreduce(HeffPlan& p, int sh, const double* Pb, double* y, cudaStream_t s) {
-    if (p.kitems[sh].empty()) return;
-    const dim3 rg(unsigned(p.otiles[sh].size()), unsigned((S::BM * S::BN + 255) / 256));
-    k_lsreduce<S><<<rg, 256, 0, s>>>(p.d_otiles[sh].get(), p.d_outs.get(), Pb + p.pc_off[sh], y);
+void launch_ls_chunk(HeffPlan& p, const HeffPlan::SChunk& c, const double* Sb, double* Pb, cudaStream_t s) {
+    uint32_t n;
+    const TileSet<KItemD> set = tile_set(p.d_kitems, c.kt[0], c.kt[1], n);
+    if (n) k_lspart<<<n, NTHR, 0, s>>>(set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
 }
 
-// the S-GEMM tiles of one coefficient chunk, reading the chunk's blocks from the plan's scratch
-template <class S>
-void launch_s_range(HeffPlan& p, int sh, const HeffPlan::WChunk& ch, const double* Tb, double* Sb, cudaStream_t s) {
-    if (ch.t1[sh] > ch.t0[sh])
-        k_sgemm<S><<<unsigned(ch.t1[sh] - ch.t0[sh]), NTHR, 0, s>>>(p.d_units.get(), p.d_utiles[sh].get() + ch.t0[sh],
-                                                                    p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(),
-                                                                    p.d_W.get(), Tb, Sb, ch.w0);
+void launch_lsreduce(HeffPlan& p, const double* Pb, double* y, cudaStream_t s, int only = -1) {
+    uint32_t n;
+    const TileSet<OTileD> set = tile_set(p.d_otiles, p.otiles, n, only);
+    const bool tall = only == SHAPE_64 || (only < 0 && !p.otiles[SHAPE_64].empty());
+    const bool mid = only == SHAPE_32 || (only < 0 && !p.otiles[SHAPE_32].empty());
+    const unsigned chunks = tall || mid ? Sh64::BM * Sh64::BN / 256 : Sh16::BM * Sh16::BN / 256;
+    static_assert(Sh64::BM * Sh64::BN == Sh32::BM * Sh32::BN, "chunks per tile");
+    if (n) k_lsreduce<<<dim3(n, chunks), 256, 0, s>>>(set, otile_set(p), p.d_outs.get(), Pb, y);
 }
 
-template <class S>
-void launch_ls(HeffPlan& p, int sh, const double* Sb, double* Pb, double* y, cudaStream_t s) {
-    if (p.kitems[sh].empty()) return;
-    k_lspart<S><<<unsigned(p.kitems[sh].size()), NTHR, 0, s>>>(p.d_kitems[sh].get(), p.d_otiles[sh].get(), p.d_outs.get(),
-                                                               p.d_segs.get(), p.l_data(), Sb, Pb);
-    const dim3 rg(unsigned(p.otiles[sh].size()), unsigned((S::BM * S::BN + 255) / 256));
-    k_lsreduce<S><<<rg, 256, 0, s>>>(p.d_otiles[sh].get(), p.d_outs.get(), Pb, y);
+void launch_ls(HeffPlan& p, const double* Sb, double* Pb, double* y, cudaStream_t s) {
+    // all shapes at once, or (their partials sharing one region) one after the other
+    for (int sh = p.p_apart ? -1 : int(SHAPE_16); sh <= (p.p_apart ? -1 : int(SHAPE_64)); ++sh) {
+        uint32_t n;
+        const TileSet<KItemD> set = tile_set(p.d_kitems, p.kitems, n, sh);
+        if (!n) continue;
+        k_lspart<<<n, NTHR, 0, s>>>(set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
+        launch_lsreduce(p, Pb, y, s, sh);
+    }
 }
 
 }  // namespace
@@ -590,52 +674,33 @@ void apply_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, double
         // chunk by chunk: T, coefficient blocks, S and the L.S partials of its ket sectors; the partials
         // of all chunks summed at the end (the phase events mark the chunk loop and the sum)
         for (const HeffPlan::SChunk& c : p.schunks) {
-            launch_t_chunk<Sh16>(p, SHAPE_16, c, x, Tb, s);
-            launch_t_chunk<Sh32>(p, SHAPE_32, c, x, Tb, s);
-            launch_t_chunk<Sh64>(p, SHAPE_64, c, x, Tb, s);
+            launch_t_chunk(p, c, x, Tb, s);
             if (c.s1 > c.s0) QCM_CUDA(cudaMemsetAsync(Sb, 0, (c.s1 - c.s0) * sizeof(double), s));
             const uint64_t w0 = p.chunk_keeps_w ? 0 : c.w0;  // kept blocks: the whole, from element 0
             if (!p.chunk_keeps_w) p.cg.generate_range(p.d_W.get(), c.u0, c.u1, c.w0, c.w1, s);
-            launch_s_chunk<Sh16>(p, SHAPE_16, c, w0, Tb, Sb, s);
-            launch_s_chunk<Sh32>(p, SHAPE_32, c, w0, Tb, Sb, s);
-            launch_s_chunk<Sh64>(p, SHAPE_64, c, w0, Tb, Sb, s);
-            launch_s_chunk<Sh128>(p, SHAPE_128, c, w0, Tb, Sb, s);
-            launch_ls_chunk<Sh16>(p, SHAPE_16, c, Sb, Pb, s);
-            launch_ls_chunk<Sh32>(p, SHAPE_32, c, Sb, Pb, s);
-            launch_ls_chunk<Sh64>(p, SHAPE_64, c, Sb, Pb, s);
+            launch_s_tiles(p, c.ut[0], c.ut[1], w0, Tb, Sb, s);
+            launch_ls_chunk(p, c, Sb, Pb, s);
         }
         if (ev) QCM_CUDA(cudaEventRecord(ev[1], s));
         if (ev) QCM_CUDA(cudaEventRecord(ev[2], s));
-        launch_lsreduce<Sh16>(p, SHAPE_16, Pb, y, s);
-        launch_lsreduce<Sh32>(p, SHAPE_32, Pb, y, s);
-        launch_lsreduce<Sh64>(p, SHAPE_64, Pb, y, s);
+        launch_lsreduce(p, Pb, y, s);
         if (ev) QCM_CUDA(cudaEventRecord(ev[3], s));
         QCM_CUDA(cudaGetLastError());
         return;
     }
-    launch_t<Sh16>(p, SHAPE_16, x, Tb, s);
-    launch_t<Sh32>(p, SHAPE_32, x, Tb, s);
-    launch_t<Sh64>(p, SHAPE_64, x, Tb, s);
+    launch_t(p, x, Tb, s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[1], s));
     if (p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));  // rows without lines stay 0
     if (p.streamed()) {
         for (const HeffPlan::WChunk& ch : p.wchunks) {
             p.cg.generate_range(p.d_W.get(), ch.u0, ch.u1, ch.w0, ch.w1, s);
-            launch_s_range<Sh16>(p, SHAPE_16, ch, Tb, Sb, s);
-            launch_s_range<Sh32>(p, SHAPE_32, ch, Tb, Sb, s);
-            launch_s_range<Sh64>(p, SHAPE_64, ch, Tb, Sb, s);
-            launch_s_range<Sh128>(p, SHAPE_128, ch, Tb, Sb, s);
+            launch_s_tiles(p, ch.t0, ch.t1, ch.w0, Tb, Sb, s);
         }
     } else {
-        launch_s<Sh16>(p, SHAPE_16, Tb, Sb, s);
-        launch_s<Sh32>(p, SHAPE_32, Tb, Sb, s);
-        launch_s<Sh64>(p, SHAPE_64, Tb, Sb, s);
-        launch_s<Sh128>(p, SHAPE_128, Tb, Sb, s);
+        launch_s(p, Tb, Sb, s);
     }
     if (ev) QCM_CUDA(cudaEventRecord(ev[2], s));
-    launch_ls<Sh16>(p, SHAPE_16, Sb, Pb, y, s);
-    launch_ls<Sh32>(p, SHAPE_32, Sb, Pb, y, s);
-    launch_ls<Sh64>(p, SHAPE_64, Sb, Pb, y, s);
+    launch_ls(p, Sb, Pb, y, s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[3], s));
     QCM_CUDA(cudaGetLastError());
 }
@@ -651,18 +716,14 @@ void apply_mixed_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, 
     double* Tb = p.d_T.get();
     float* Thi = reinterpret_cast<float*>(Tb);
     float* Tlo = tc ? Thi + p.t_len : nullptr;
-    launch_t<Sh16>(p, SHAPE_16, x, Tb, s, Thi, Tlo);
-    launch_t<Sh32>(p, SHAPE_32, x, Tb, s, Thi, Tlo);
-    launch_t<Sh64>(p, SHAPE_64, x, Tb, s, Thi, Tlo);
+    launch_t(p, x, Tb, s, Thi, Tlo);
     if (ev) QCM_CUDA(cudaEventRecord(ev[1], s));
     double* Sb = p.d_S.get();
     if (p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));
     if (tc) run_sgemm_mixed(p, true, p.d_W32s.get(), p.d_W32s.get() + p.w_len, Thi, Tlo, Sb, p.d_merr.get(), s);
     else run_sgemm_mixed(p, false, p.d_W32.get(), nullptr, Thi, nullptr, Sb, p.d_merr.get(), s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[2], s));
-    launch_ls<Sh16>(p, SHAPE_16, Sb, p.d_P.get(), y, s);
-    launch_ls<Sh32>(p, SHAPE_32, Sb, p.d_P.get(), y, s);
-    launch_ls<Sh64>(p, SHAPE_64, Sb, p.d_P.get(), y, s);
+    launch_ls(p, Sb, p.d_P.get(), y, s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[3], s));
     QCM_CUDA(cudaGetLastError());
 }
@@ -675,9 +736,7 @@ void heff_apply_device(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev)
 void heff_tgemm_device(HeffPlan& p, const double* x, double* T) {
     if (!p.lists_staged) throw std::runtime_error("heff T-GEMM: the plan's work lists are not on the device");
     if (p.sector_chunked()) throw std::runtime_error("heff T-GEMM: the plan's apply is chunked by ket sector");
-    launch_t<Sh16>(p, SHAPE_16, x, T, p.stream);
-    launch_t<Sh32>(p, SHAPE_32, x, T, p.stream);
-    launch_t<Sh64>(p, SHAPE_64, x, T, p.stream);
+    launch_t(p, x, T, p.stream);
     QCM_CUDA(cudaGetLastError());
 }
 
@@ -718,50 +777,44 @@ void heff_apply_device_scratch(HeffPlan& p, const double* x, double* y, double* 
 
 void run_tgemm(const TJobD* jobs, const DBuf<TileD>* dtiles, const std::vector<TileD>* htiles, const double* x,
                const double* R, double* T, cudaStream_t s) {
-    if (!htiles[SHAPE_16].empty())
-        k_tgemm<Sh16><<<unsigned(htiles[SHAPE_16].size()), NTHR, 0, s>>>(jobs, dtiles[SHAPE_16].get(), x, R, T, nullptr, nullptr);
-    if (!htiles[SHAPE_32].empty())
-        k_tgemm<Sh32><<<unsigned(htiles[SHAPE_32].size()), NTHR, 0, s>>>(jobs, dtiles[SHAPE_32].get(), x, R, T, nullptr, nullptr);
-    if (!htiles[SHAPE_64].empty())
-        k_tgemm<Sh64><<<unsigned(htiles[SHAPE_64].size()), NTHR, 0, s>>>(jobs, dtiles[SHAPE_64].get(), x, R, T, nullptr, nullptr);
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(dtiles, htiles, n);
+    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, jobs, x, R, T, nullptr, nullptr);
     QCM_CUDA(cudaGetLastError());
 }
 
 void run_sgemm(const UnitD* units, const DBuf<TileD>* dtiles, const std::vector<TileD>* htiles, const uint32_t* line_b1,
                const uint64_t* slice_off, const uint16_t* klist, const double* W, const double* T, double* S,
                cudaStream_t s) {
-    if (!htiles[SHAPE_16].empty())
-        k_sgemm<Sh16><<<unsigned(htiles[SHAPE_16].size()), NTHR, 0, s>>>(units, dtiles[SHAPE_16].get(), line_b1, slice_off, klist, W, T, S, 0);
-    if (!htiles[SHAPE_32].empty())
-        k_sgemm<Sh32><<<unsigned(htiles[SHAPE_32].size()), NTHR, 0, s>>>(units, dtiles[SHAPE_32].get(), line_b1, slice_off, klist, W, T, S, 0);
-    if (!htiles[SHAPE_64].empty())
-        k_sgemm<Sh64><<<unsigned(htiles[SHAPE_64].size()), NTHR, 0, s>>>(units, dtiles[SHAPE_64].get(), line_b1, slice_off, klist, W, T, S, 0);
-    if (!htiles[SHAPE_128].empty())
-        k_sgemm<Sh128><<<unsigned(htiles[SHAPE_128].size()), NTHR, 0, s>>>(units, dtiles[SHAPE_128].get(), line_b1, slice_off, klist, W, T, S, 0);
+    uint32_t n;
+    const TileSet<TileD> set = tile_set(dtiles, htiles, n);
+    if (n) k_sgemm<<<n, NTHR, 0, s>>>(set, units, line_b1, slice_off, klist, W, T, S, 0);
     QCM_CUDA(cudaGetLastError());
 }
 
-
 int heff_launches_per_apply(const HeffPlan& p) {
+    // one launch per phase for all tile shapes (the two L.S kernels per shape if its partials share a region)
+    auto any = [](const uint32_t* a, const uint32_t* b) {
+        for (int sh = 0; sh < N_SHAPES; ++sh)
+            if (b[sh] > a[sh]) return 1;
+        return 0;
+    };
+    auto some = [](const auto* v) {
+        for (int sh = 0; sh < N_SHAPES; ++sh)
+            if (!v[sh].empty()) return 1;
+        return 0;
+    };
     int n = 0;
-    for (int sh = 0; sh < N_SHAPES; ++sh) {
-        n += !p.ttiles[sh].empty();
-        if (!p.streamed()) n += !p.utiles[sh].empty();
-        n += p.kitems[sh].empty() ? 0 : 2;
-    }
-    for (const HeffPlan::WChunk& ch : p.wchunks) {
-        n += ch.u1 > ch.u0;  // the chunk's coefficient generation
-        for (int sh = 0; sh < N_SHAPES; ++sh) n += ch.t1[sh] > ch.t0[sh];
-    }
     if (p.sector_chunked()) {
-        n = 0;
-        for (const HeffPlan::SChunk& c : p.schunks) {
-            n += !p.chunk_keeps_w && c.u1 > c.u0;
-            for (int sh = 0; sh < N_SHAPES; ++sh)
-                n += (c.tt[1][sh] > c.tt[0][sh]) + (c.ut[1][sh] > c.ut[0][sh]) + (c.kt[1][sh] > c.kt[0][sh]);
-        }
-        for (int sh = 0; sh < N_SHAPES; ++sh) n += !p.kitems[sh].empty();  // the partial sums
+        for (const HeffPlan::SChunk& c : p.schunks)
+            n += (!p.chunk_keeps_w && c.u1 > c.u0) + any(c.tt[0], c.tt[1]) + any(c.ut[0], c.ut[1]) + any(c.kt[0], c.kt[1]);
+        return n + some(p.otiles);  // the partial sums
     }
+    n = some(p.ttiles);
+    if (!p.streamed()) n += some(p.utiles);
+    for (const HeffPlan::WChunk& ch : p.wchunks) n += (ch.u1 > ch.u0) + any(ch.t0, ch.t1);  // generation, S-GEMM
+    if (p.p_apart) return n + 2 * some(p.kitems);
+    for (int sh = 0; sh < N_SHAPES; ++sh) n += p.kitems[sh].empty() ? 0 : 2;
     return n;
 }
 

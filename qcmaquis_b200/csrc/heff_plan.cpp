@@ -22,6 +22,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../../include/qcm_b200.h"
 #include "heff.hpp"
 
 namespace qcm {
@@ -400,6 +401,23 @@ void CoefGen::add_unit(uint64_t w_off, uint32_t wld, uint32_t st_out, const uint
     for (uint32_t i = 0; i < g.nk; ++i) { smap_id[m0 + i] = pr[i].first; smap_slot[m0 + i] = pr[i].second; }
     gin.insert(gin.end(), in_row, in_row + nst);
     units.push_back(g);
+}
+
+void place_partials(HeffPlan& p, uint64_t limit) {
+    uint64_t most = 0, sum = 0;
+    for (int sh = 0; sh < N_SHAPES; ++sh) {
+        const uint64_t n = uint64_t(p.kitems[sh].size()) * shape_bm(sh) * shape_bn(sh);
+        p.p_off[sh] = sum;
+        sum += n;
+        most = std::max(most, n);
+    }
+    auto total = [&](uint64_t n) {  // the scratch of an apply, each part rounded up as the allocation-free form does
+        auto r32 = [](uint64_t v) { return (v + 31) / 32 * 32; };
+        return r32(p.t_len) + r32(p.s_len) + r32(n);
+    };
+    p.p_apart = total(sum) <= limit || total(most) > limit;
+    if (!p.p_apart) std::fill(p.p_off, p.p_off + N_SHAPES, 0);
+    p.p_len = p.p_apart ? sum : most;
 }
 
 std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBoundary& Rb, const MPOTensor& W,
@@ -851,9 +869,7 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
                      p->units.size(), (unsigned long long)p->n_alpha,
                      p->utiles[0].size() + p->utiles[1].size() + p->utiles[2].size() + p->utiles[3].size(), double(p->w_len));
     }
-    uint64_t pl = 0;
-    for (int sh = 0; sh < N_SHAPES; ++sh) pl = std::max<uint64_t>(pl, uint64_t(p->kitems[sh].size()) * shape_bm(sh) * shape_bn(sh));
-    p->p_len = pl;
+    place_partials(*p, QCM_NOALLOC_SCRATCH_DOUBLES);
     p->flops = p->flops_t + p->flops_ls + p->flops_s;
     return p;
 }
