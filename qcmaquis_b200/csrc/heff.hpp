@@ -290,6 +290,8 @@ struct HeffPlan {
     // that they take in turn
     uint64_t p_len = 0, p_off[N_SHAPES] = {};
     bool p_apart = false;
+    bool s_covered = true;   // the S-GEMM tiles write every S element that L.S reads (else S is cleared first)
+    bool y_covered = false;  // the output tiles write every element of the vector (else it is cleared first)
 
     // reference work count ScheduleNew::total_flops (tasks.cpp:388-398, 777-796)
     double flops = 0, flops_t = 0, flops_ls = 0, flops_s = 0;

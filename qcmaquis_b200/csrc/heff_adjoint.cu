@@ -253,7 +253,6 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
     double* T = p.d_T.get();
     double* Sb = p.d_S.get();
     heff_tgemm_device(p, x, T);
-    if (p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));
     if (!w.sjobs.empty())
         batched_gemm(w.sjobs, p.L->data.get(), p.L->data.size(), ybar, p.x_len, Sb, p.s_len, w.d_jobs, w.d_jtiles, s);
     if (!w.tiles.empty())

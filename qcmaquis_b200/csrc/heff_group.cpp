@@ -114,6 +114,7 @@ std::unique_ptr<HeffPlan> merge_plans(const std::vector<HeffPlan*>& plans, std::
         g->flops += p.flops; g->flops_t += p.flops_t; g->flops_s += p.flops_s; g->flops_ls += p.flops_ls;
         g->flops_sexec += p.flops_sexec; g->flops_sdense += p.flops_sdense;
         g->n_alpha += p.n_alpha;
+        g->s_covered = g->s_covered && p.s_covered;
         xl += round32(p.x_len);
         tl += round32(p.t_len);
         sl += round32(p.s_len);

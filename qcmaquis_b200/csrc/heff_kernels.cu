@@ -669,13 +669,13 @@ void apply_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, double
     cudaStream_t s = p.stream;
     if (!p.lists_staged) throw std::runtime_error("heff apply: the plan's work lists are not on the device");
     if (ev) QCM_CUDA(cudaEventRecord(ev[0], s));
-    QCM_CUDA(cudaMemsetAsync(y, 0, p.x_len * sizeof(double), s));
+    if (!p.y_covered) QCM_CUDA(cudaMemsetAsync(y, 0, p.x_len * sizeof(double), s));
     if (p.sector_chunked()) {
         // chunk by chunk: T, coefficient blocks, S and the L.S partials of its ket sectors; the partials
         // of all chunks summed at the end (the phase events mark the chunk loop and the sum)
         for (const HeffPlan::SChunk& c : p.schunks) {
             launch_t_chunk(p, c, x, Tb, s);
-            if (c.s1 > c.s0) QCM_CUDA(cudaMemsetAsync(Sb, 0, (c.s1 - c.s0) * sizeof(double), s));
+            if (!p.s_covered && c.s1 > c.s0) QCM_CUDA(cudaMemsetAsync(Sb, 0, (c.s1 - c.s0) * sizeof(double), s));
             const uint64_t w0 = p.chunk_keeps_w ? 0 : c.w0;  // kept blocks: the whole, from element 0
             if (!p.chunk_keeps_w) p.cg.generate_range(p.d_W.get(), c.u0, c.u1, c.w0, c.w1, s);
             launch_s_tiles(p, c.ut[0], c.ut[1], w0, Tb, Sb, s);
@@ -690,7 +690,7 @@ void apply_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, double
     }
     launch_t(p, x, Tb, s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[1], s));
-    if (p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));  // rows without lines stay 0
+    if (!p.s_covered && p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));
     if (p.streamed()) {
         for (const HeffPlan::WChunk& ch : p.wchunks) {
             p.cg.generate_range(p.d_W.get(), ch.u0, ch.u1, ch.w0, ch.w1, s);
@@ -711,7 +711,7 @@ void apply_mixed_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, 
     if (!p.lists_staged) throw std::runtime_error("heff apply: the plan's work lists are not on the device");
     prepare_mixed(p, tc);
     if (ev) QCM_CUDA(cudaEventRecord(ev[0], s));
-    QCM_CUDA(cudaMemsetAsync(y, 0, p.x_len * sizeof(double), s));
+    if (!p.y_covered) QCM_CUDA(cudaMemsetAsync(y, 0, p.x_len * sizeof(double), s));
     // T in FP32, or its hi and lo, lives in the bytes of the FP64 T buffer (t_len doubles = 2 t_len floats)
     double* Tb = p.d_T.get();
     float* Thi = reinterpret_cast<float*>(Tb);
@@ -719,7 +719,8 @@ void apply_mixed_impl(HeffPlan& p, const double* x, double* y, cudaEvent_t* ev, 
     launch_t(p, x, Tb, s, Thi, Tlo);
     if (ev) QCM_CUDA(cudaEventRecord(ev[1], s));
     double* Sb = p.d_S.get();
-    if (p.s_len) QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));
+    if ((tc || !p.s_covered) && p.s_len)  // k_sgemm_tc leaves tiles without steps out
+        QCM_CUDA(cudaMemsetAsync(Sb, 0, p.s_len * sizeof(double), s));
     if (tc) run_sgemm_mixed(p, true, p.d_W32s.get(), p.d_W32s.get() + p.w_len, Thi, Tlo, Sb, p.d_merr.get(), s);
     else run_sgemm_mixed(p, false, p.d_W32.get(), nullptr, Thi, nullptr, Sb, p.d_merr.get(), s);
     if (ev) QCM_CUDA(cudaEventRecord(ev[2], s));

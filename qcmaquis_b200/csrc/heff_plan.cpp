@@ -80,6 +80,7 @@ struct Part {
     std::vector<TileD> utiles[N_SHAPES];  // S-GEMM tiles, item = unit of this part, pad = klist offset
     std::vector<uint16_t> klist;
     double flops_sexec = 0;
+    bool s_covered = true;  // every S row of the part's cohorts is a line of every unit
 };
 
 // Output state of a cohort and its coefficient terms: (line, slice id in the part's T
@@ -151,7 +152,7 @@ void emit_tiles(const UnitD& u, uint32_t item, const TileChoice& c, std::vector<
             if (m) { klist.push_back(uint16_t((ks << 4) | m)); ++cnt; }
         }
         klist[off] = cnt;
-        if (!cnt) continue;
+        // a tile without steps too: its lines' S rows are zero, and nothing else writes them
         for (uint32_t n0 = 0; n0 < u.ne; n0 += bn) utiles[sh].push_back(TileD{item, mt * bm, n0, off});
     }
 }
@@ -171,7 +172,9 @@ void plan_unit_tiles(const UnitD& u, const uint64_t* sig, uint32_t nw, std::vect
     const uint32_t nk = u.nk;
     order.resize(nk);
     for (uint32_t i = 0; i < nk; ++i) order[i] = i;
+    best.sh = SHAPE_64;  // a unit without terms: its tiles write zeros
     if (!u.nl || !u.ne || !nk) return;
+    best.sh = -1;
     const uint32_t nks = checked_ksteps(u), n16 = (u.nl + 15) / 16;
     std::vector<uint64_t> key;
     std::vector<uint32_t> ord(nk);
@@ -512,6 +515,7 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
     std::vector<uint32_t> corder, crank, ctmp;
     std::vector<GRef> gref;
     std::vector<std::pair<uint32_t, uint32_t>> lrows;
+    std::vector<uint8_t> seen;
 #pragma omp for schedule(dynamic, 1)
     for (int oi = 0; oi < int(nl); ++oi) try {
         const uint32_t lb_in = part_order[std::size_t(oi)];
@@ -597,6 +601,13 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
                                                              const std::pair<uint32_t, uint32_t>& b) {
                 return W.row_ptr[a.first + 1] - W.row_ptr[a.first] > W.row_ptr[b.first + 1] - W.row_ptr[b.first];
             });
+            // do the MPO rows and the cohort's S row blocks correspond one to one?
+            seen.assign(nS, 0);
+            bool one_to_one = lrows.size() == nS;
+            for (const auto& lr : lrows) {
+                one_to_one = one_to_one && lr.second < nS && !seen[lr.second];
+                if (one_to_one) seen[lr.second] = 1;
+            }
             const uint32_t nw16 = (uint32_t(lrows.size()) + 1023) / 1024;  // signature words: 64 groups of 16 lines
             // per (unit, input state): the R block positions of the input state's cohort and the
             // slice-id base of its T job (rp = null: no T job)
@@ -662,12 +673,25 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
             }
             if (n_alpha == 0) continue;
             P.n_alpha += n_alpha;
+            P.s_covered = P.s_covered && one_to_one;
             const uint64_t s_off = P.s_len;
             P.s_len += (uint64_t(K_c) * stripe + 31) / 32 * 32;
             for (std::size_t ui = 0; ui < nu; ++ui) {
                 U& u = units[ui];
                 P.flops_s += 2.0 * ls_in * u.ms * double(u.nterms);
-                if (!u.nterms) continue;
+                const uint32_t nl_terms = uint32_t(u.lines.size());
+                // the cohort's blocks without a term for this unit are lines without coefficients, after the others:
+                // the S-GEMM writes their zeros, so that S needs no clearing before an apply (at L=24, M=512 they
+                // are 1 % of S, and clearing it took 0.16 ms of 3.7)
+                if (one_to_one) {
+                    std::size_t next = 0;
+                    for (const auto& lr : lrows) {
+                        if (next < nl_terms && u.lines[next] == lr.second) { ++next; continue; }
+                        u.lines.push_back(lr.second);
+                        u.rows.push_back(lr.first);
+                    }
+                }
+                if (u.lines.empty()) continue;
                 slices.assign(u.sl.begin(), u.sl.end());
                 // slot order and S-GEMM tiling from the slot signatures
                 UnitD ud{};
@@ -723,9 +747,9 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
                         P.flops_sexec += 2.0 * 4.0 * g * shape_bm(sh) * shape_bn(sh);
                     }
                 P.units.push_back(ud);
-                P.g_elems += uint64_t(ud.ne) * ud.nl;
+                P.g_elems += uint64_t(ud.ne) * nl_terms;
                 P.g_reads += uint64_t(ud.ne) * u.nterms;
-                P.flops_sdense += 2.0 * ud.nl * ud.nk * double(ud.ne);  // padding lines not counted
+                P.flops_sdense += 2.0 * nl_terms * ud.nk * double(ud.ne);  // padding lines not counted
             }
             P.flops_ls += 2.0 * ls_out * ls_in * double(nS) * stripe;
             SegD sg{};
@@ -757,6 +781,7 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
                  b.kl + uint32_t(P.klist.size()), b.bk + P.bk_alpha.size(), {}};
         for (int sh = 0; sh < N_SHAPES; ++sh) n.tile[sh] = b.tile[sh] + P.utiles[sh].size();
         p->flops_sexec += P.flops_sexec;
+        p->s_covered = p->s_covered && P.s_covered;
     }
     const Base& tot = base[nl];
     p->part_job.resize(nl + 1); p->part_unit.resize(nl + 1);
@@ -860,6 +885,10 @@ std::unique_ptr<HeffPlan> build_heff_plan(const DevBoundary& Lb, const DevBounda
         }
         p->outs.push_back(o);
     }
+    uint64_t y_len = 0;
+    for (const OutD& o : p->outs)
+        if (o.seg_count) y_len += uint64_t(o.M) * o.N;
+    p->y_covered = y_len == p->x_len;
     if (tdbg) {
         double psum = 0, pmax = 0;
         for (double t : part_s) { psum += t; pmax = std::max(pmax, t); }
