@@ -439,7 +439,7 @@ struct BStepPlan {
         uint64_t b = dbytes(d_tjobs) + dbytes(sb.d_units) + dbytes(sb.d_klist) + dbytes(sb.d_line_b1) + dbytes(sb.d_slice_off);
         for (int k = 0; k < N_SHAPES; ++k) b += dbytes(d_ttiles[k]) + dbytes(sb.d_utiles[k]);
         const CoefGen& g = sb.cg;
-        b += dbytes(g.d_units) + dbytes(g.d_gin) + dbytes(g.d_line_major) + dbytes(g.d_smap_id) + dbytes(g.d_smap_slot) +
+        b += dbytes(g.d_tasks) + dbytes(g.d_units) + dbytes(g.d_gin) + dbytes(g.d_line_major) + dbytes(g.d_smap_id) + dbytes(g.d_smap_slot) +
              dbytes(g.d_m_ptr) + dbytes(g.d_m_other) + dbytes(g.d_m_op) + dbytes(g.d_o_ptr) + dbytes(g.d_o_in) +
              dbytes(g.d_line_scale) + dbytes(g.d_m_scale) + dbytes(g.d_o_val) + dbytes(g.d_b_cs) + dbytes(g.d_b_pos);
         return b;

@@ -201,8 +201,13 @@ struct MPOTables {
 };
 std::shared_ptr<const MPOTables> build_mpo_tables(const MPOTensor& W);
 
+// one CTA's share of a unit's (line, MPO entry) pairs: those numbered i0 .. i0 + WGEN_PAIRS - 1
+struct WGenTaskD { uint32_t unit, i0; };
+constexpr uint32_t WGEN_PAIRS = 2048;
+
 // the coefficient-generation tables on the device (CoefGen::tables)
 struct WGenTab {
+    const WGenTaskD* tasks;
     const WGenUnitD* units;
     const WGenInD* gin;
     const uint32_t* line_major;
@@ -232,6 +237,8 @@ struct CoefGen {
     bool serial = false;  // two MPO indices of one boundary cohort share a block
     uint64_t w_len = 0;
 
+    std::vector<uint32_t> task_ptr;  // per unit, its first task (made by upload; one past the last unit too)
+    DBuf<WGenTaskD> d_tasks;
     DBuf<WGenUnitD> d_units;
     DBuf<WGenInD> d_gin;
     DBuf<uint32_t> d_line_major, d_smap_id, d_smap_slot, d_m_ptr, d_m_other, d_m_op, d_o_ptr, d_o_in, d_err;

@@ -112,10 +112,11 @@ __global__ void __launch_bounds__(NTHR) k_wbar(const UnitD* __restrict__ units, 
 __global__ void __launch_bounds__(wg::THR) k_wadj(WGenTab t, const double* __restrict__ Wb, const uint64_t* __restrict__ pofs,
                                                   double* __restrict__ P, uint32_t* __restrict__ err) {
     __shared__ wg::Shared sh;
-    const WGenUnitD U = t.units[blockIdx.x];
-    const wg::Map map = wg::stage(t, U, blockIdx.x, sh);
+    const WGenTaskD task = t.tasks[blockIdx.x];
+    const WGenUnitD U = t.units[task.unit];
+    const wg::Map map = wg::stage(t, U, task.unit, sh);
     const double* Wu = Wb + U.w_off;
-    wg::for_entries(t, U, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t) {
+    wg::for_entries(t, U, task.i0, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t) {
         const uint32_t gl = U.line0 + line, x = t.m_other[e];
         const double lsc = t.line_scale[gl];
         const std::size_t q = std::size_t(t.m_op[e]) * t.nst + U.st_out;
@@ -261,8 +262,8 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
     QCM_CUDA(cudaGetLastError());
     const CoefGen& cg = p.cg;
     QCM_CUDA(cudaMemsetAsync(w.d_err.get(), 0, sizeof(uint32_t), s));
-    if (!cg.units.empty())
-        k_wadj<<<unsigned(cg.units.size()), wg::THR, 0, s>>>(cg.tables(), w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
+    if (!cg.task_ptr.empty() && cg.task_ptr.back())
+        k_wadj<<<cg.task_ptr.back(), wg::THR, 0, s>>>(cg.tables(), w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
                                                              w.d_err.get());
     QCM_CUDA(cudaGetLastError());
     const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 255) / 256, 148 * 16));

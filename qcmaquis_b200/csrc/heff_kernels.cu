@@ -325,29 +325,30 @@ __global__ void __launch_bounds__(NTHR, 5) k_sgemm(TileSet<TileD> set, const Uni
     else sgemm_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
 }
 
-// One CTA per unit: the coefficient terms of its lines (CoefGen), in MPO-entry then operator-term order, summed
+// One CTA per task: the coefficient terms of a unit's lines (CoefGen), in MPO-entry then operator-term order, summed
 // into W_u.  Products and sums are rounded separately (no contraction), so W_u holds the same values as a host
 // evaluation of the same terms.  Terms of a line meet in one cell only if their entries share the other MPO
 // index (a slice id is an input state's base plus that index's block position), and those are neighbours in the
 // row: the thread of the first of them adds them all, in order.  Tables that break either premise (an unsorted
 // row, two indices of a boundary cohort on one block: CoefGen::serial) leave the whole row to one thread.
-// One thread per line took 2.07 ms for the 12 M terms of the L=16, M=256 middle bond.
-__global__ void __launch_bounds__(wg::THR) k_wgen(WGenTab t, uint32_t u0, double* __restrict__ W, uint64_t w0,
+__global__ void __launch_bounds__(wg::THR) k_wgen(WGenTab t, uint32_t task0, double* __restrict__ W, uint64_t w0,
                                                   uint32_t* __restrict__ err) {
     __shared__ wg::Shared sh;
-    const uint32_t unit = u0 + blockIdx.x;
-    const WGenUnitD U = t.units[unit];
-    const wg::Map map = wg::stage(t, U, unit, sh);
+    const WGenTaskD task = t.tasks[task0 + blockIdx.x];
+    const WGenUnitD U = t.units[task.unit];
+    const wg::Map map = wg::stage(t, U, task.unit, sh);
     double* Wu = W + (U.w_off - w0);
-    wg::for_entries(t, U, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t e1) {
+    wg::for_entries(t, U, task.i0, sh, [&](uint32_t line, uint32_t e, uint32_t e0, uint32_t e1) {
         uint32_t x = t.m_other[e];
         if (e > e0 && (t.serial || t.m_other[e - 1] == x)) return;  // added by an earlier entry's thread
         const double lsc = t.line_scale[U.line0 + line];
         for (uint32_t f = e;;) {
+            const bool more = f + 1 < e1 && (t.serial || t.m_other[f + 1] == x);
             const double wsc = __dmul_rn(t.m_scale[f], lsc);
             const std::size_t q = std::size_t(t.m_op[f]) * t.nst + U.st_out;
-            const uint32_t k1 = t.o_ptr[q + 1];
-            for (uint32_t k = t.o_ptr[q]; k < k1; ++k) {
+            const uint32_t k0 = t.o_ptr[q], k1 = t.o_ptr[q + 1];
+            const bool alone = !more && f == e && k1 == k0 + 1;  // the only term of its cell
+            for (uint32_t k = k0; k < k1; ++k) {
                 const WGenInD g = sh.sin[t.o_in[k]];
                 if (g.c == WGEN_NONE) continue;
                 const std::size_t bq = std::size_t(g.c) * t.b_aux + x;
@@ -357,10 +358,10 @@ __global__ void __launch_bounds__(wg::THR) k_wgen(WGenTab t, uint32_t u0, double
                 const uint32_t slot = map.slot(g.jbase + uint32_t(pos));
                 if (slot == WGEN_NONE) { atomicOr(err, 1u); continue; }
                 double* w = Wu + line + uint64_t(slot) * U.wld;
-                *w = __dadd_rn(*w, a);
+                *w = __dadd_rn(alone ? 0.0 : *w, a);
             }
-            if (++f >= e1 || (!t.serial && t.m_other[f] != x)) break;
-            x = t.m_other[f];
+            if (!more) break;
+            x = t.m_other[++f];
         }
     });
 }
@@ -395,6 +396,24 @@ void CoefGen::validate() const {
 
 void CoefGen::upload(cudaStream_t s) {
     validate();
+    {
+        const std::vector<uint32_t>& ptr = by_row ? mt->row_ptr : mt->col_ptr;
+        std::vector<WGenTaskD> tasks;
+        task_ptr.resize(units.size() + 1);
+        for (std::size_t i = 0; i < units.size(); ++i) {
+            task_ptr[i] = uint32_t(tasks.size());
+            uint64_t pairs = 0;
+            for (uint32_t l = 0; l < units[i].nl; ++l) {
+                const uint32_t m = line_major[units[i].line0 + l];
+                pairs += ptr[m + 1] - ptr[m];
+            }
+            if (pairs > 0xffffffffu - WGEN_PAIRS) throw std::runtime_error("coefficient tables: too many terms in a unit");
+            for (uint64_t p = 0; p < pairs; p += WGEN_PAIRS) tasks.push_back(WGenTaskD{uint32_t(i), uint32_t(p)});
+        }
+        task_ptr[units.size()] = uint32_t(tasks.size());
+        d_tasks.upload(tasks, s);
+        QCM_CUDA(cudaStreamSynchronize(s));  // the list is local
+    }
     d_units.upload(units, s);
     d_gin.upload(gin, s);
     d_line_major.upload(line_major, s);
@@ -414,7 +433,7 @@ void CoefGen::upload(cudaStream_t s) {
 
 WGenTab CoefGen::tables() const {
     WGenTab t;
-    t.units = d_units.get(); t.gin = d_gin.get(); t.line_major = d_line_major.get(); t.line_scale = d_line_scale.get();
+    t.tasks = d_tasks.get(); t.units = d_units.get(); t.gin = d_gin.get(); t.line_major = d_line_major.get(); t.line_scale = d_line_scale.get();
     t.smap_id = d_smap_id.get(); t.smap_slot = d_smap_slot.get();
     t.m_ptr = d_m_ptr.get(); t.m_other = d_m_other.get(); t.m_op = d_m_op.get(); t.m_scale = d_m_scale.get();
     t.o_ptr = d_o_ptr.get(); t.o_in = d_o_in.get(); t.o_val = d_o_val.get();
@@ -432,13 +451,15 @@ void CoefGen::generate(double* W, cudaStream_t s) {
 void CoefGen::generate_range(double* W, uint32_t u0, uint32_t u1, uint64_t w0, uint64_t w1, cudaStream_t s) {
     if (w1 > w0) QCM_CUDA(cudaMemsetAsync(W, 0, (w1 - w0) * sizeof(double), s));
     if (u1 <= u0) return;
-    if (d_units.size() < units.size()) throw std::runtime_error("coefficient tables: not uploaded");
+    if (d_units.size() < units.size() || task_ptr.size() != units.size() + 1)
+        throw std::runtime_error("coefficient tables: not uploaded");
     if (u1 > units.size()) throw std::runtime_error("coefficient tables: unit range outside the plan");
     if (d_err.size() < 1) {
         d_err.alloc(1);
         QCM_CUDA(cudaMemsetAsync(d_err.get(), 0, sizeof(uint32_t), s));
     }
-    k_wgen<<<unsigned(u1 - u0), wg::THR, 0, s>>>(tables(), u0, W, w0, d_err.get());
+    const uint32_t t0 = task_ptr[u0], t1 = task_ptr[u1];
+    if (t1 > t0) k_wgen<<<t1 - t0, wg::THR, 0, s>>>(tables(), t0, W, w0, d_err.get());
     QCM_CUDA(cudaGetLastError());
 }
 
@@ -829,7 +850,7 @@ void release_plan_device(HeffPlan& p) {
     p.d_merr.reset(); p.d_x.reset(); p.d_y.reset();
     p.adj.reset();
     CoefGen& g = p.cg;
-    g.d_units.reset(); g.d_gin.reset(); g.d_line_major.reset(); g.d_smap_id.reset(); g.d_smap_slot.reset();
+    g.d_tasks.reset(); g.d_units.reset(); g.d_gin.reset(); g.d_line_major.reset(); g.d_smap_id.reset(); g.d_smap_slot.reset();
     g.d_m_ptr.reset(); g.d_m_other.reset(); g.d_m_op.reset(); g.d_o_ptr.reset(); g.d_o_in.reset(); g.d_err.reset();
     g.d_line_scale.reset(); g.d_m_scale.reset(); g.d_o_val.reset(); g.d_b_cs.reset(); g.d_b_pos.reset();
     p.lists_staged = false;
@@ -840,7 +861,7 @@ void release_plan_scratch(HeffPlan& p) {
     p.d_W32.reset(); p.d_W32s.reset(); p.d_merr.reset();
     p.adj.reset();
     CoefGen& g = p.cg;
-    g.d_units.reset(); g.d_gin.reset(); g.d_line_major.reset(); g.d_smap_id.reset(); g.d_smap_slot.reset();
+    g.d_tasks.reset(); g.d_units.reset(); g.d_gin.reset(); g.d_line_major.reset(); g.d_smap_id.reset(); g.d_smap_slot.reset();
     g.d_m_ptr.reset(); g.d_m_other.reset(); g.d_m_op.reset(); g.d_o_ptr.reset(); g.d_o_in.reset(); g.d_err.reset();
     g.d_line_scale.reset(); g.d_m_scale.reset(); g.d_o_val.reset(); g.d_b_cs.reset(); g.d_b_pos.reset();
 }

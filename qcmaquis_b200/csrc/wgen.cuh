@@ -1,8 +1,10 @@
 // Traversal of the coefficient terms of an S-build unit, shared by the generation of its coefficient block
-// (k_wgen) and the adjoint's sums over it (k_wadj): one CTA per unit, one thread per (line, MPO entry) pair.
-// Rows of the MPO differ in length by two orders of magnitude and a term is a chain of dependent table reads, so
-// the pairs of a unit are numbered through (a scan of the row lengths) and dealt out to the threads one by one:
-// the longest row no longer decides, and neighbouring threads read neighbouring entries.
+// (k_wgen) and the adjoint's sums over it (k_wadj): one thread per (line, MPO entry) pair.
+// Rows of the MPO differ in length by two orders of magnitude, units by three, and a term is a chain of dependent
+// table reads: latency binds, so what counts is how many pairs are in flight.  The pairs of a unit are numbered
+// through (a scan of the row lengths), cut into tasks of WGEN_PAIRS pairs, a CTA each, and dealt out to its threads
+// one by one: neither the longest row nor the largest unit decides, and neighbouring threads read neighbouring
+// entries.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -53,10 +55,11 @@ static __device__ __forceinline__ Map stage(const WGenTab& t, const WGenUnitD& U
     return Map{staged ? sh.sid : t.smap_id + U.map0, staged ? sh.sslot : t.smap_slot + U.map0, U.nk};
 }
 
-// body(line, entry, first entry of the line's row, one past its last) for every pair of the unit
+// body(line, entry, first entry of the line's row, one past its last) for the pairs [i0, i0 + WGEN_PAIRS) of the unit
 template <class Body>
-static __device__ __forceinline__ void for_entries(const WGenTab& t, const WGenUnitD& U, Shared& sh, Body body) {
-    for (uint32_t l0 = 0; l0 < U.nl; l0 += LINES) {
+static __device__ __forceinline__ void for_entries(const WGenTab& t, const WGenUnitD& U, uint32_t i0, Shared& sh, Body body) {
+    uint32_t base = 0;  // pairs of the lines before l0
+    for (uint32_t l0 = 0; l0 < U.nl && base < i0 + WGEN_PAIRS; l0 += LINES) {
         const uint32_t n = min(LINES, U.nl - l0);
         for (uint32_t l = threadIdx.x; l < n; l += blockDim.x) {
             const uint32_t m = t.line_major[U.line0 + l0 + l];
@@ -67,21 +70,22 @@ static __device__ __forceinline__ void for_entries(const WGenTab& t, const WGenU
         if (threadIdx.x == 0) sh.pre[0] = 0;
         __syncthreads();
         if (threadIdx.x < 32) {
-            uint32_t base = 0;
+            uint32_t carry = 0;
             for (uint32_t l = threadIdx.x; l < (n + 31) / 32 * 32; l += 32) {
                 uint32_t v = l < n ? sh.pre[l + 1] : 0;
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t w = __shfl_up_sync(0xffffffffu, v, o);
                     if (int(threadIdx.x) >= o) v += w;
                 }
-                v += base;
+                v += carry;
                 if (l < n) sh.pre[l + 1] = v;
-                base = __shfl_sync(0xffffffffu, v, 31);
+                carry = __shfl_sync(0xffffffffu, v, 31);
             }
         }
         __syncthreads();
         const uint32_t total = sh.pre[n];
-        for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+        const uint32_t a0 = i0 > base ? i0 - base : 0, a1 = min(total, i0 + WGEN_PAIRS - base);
+        for (uint32_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
             uint32_t lo = 0, hi = n;  // the last line with pre[line] <= i (an empty row's successor wins)
             while (hi - lo > 1) {
                 const uint32_t mid = (lo + hi) >> 1;
@@ -91,6 +95,7 @@ static __device__ __forceinline__ void for_entries(const WGenTab& t, const WGenU
             const uint32_t a = sh.row0[lo];
             body(l0 + lo, a + (i - sh.pre[lo]), a, a + (sh.pre[lo + 1] - sh.pre[lo]));
         }
+        base += total;
         __syncthreads();
     }
 }
