@@ -38,6 +38,7 @@
 #include <stdexcept>
 
 #include "heff.hpp"
+#include "tiles.cuh"
 
 namespace qcm {
 namespace {
@@ -96,13 +97,11 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 }
 
 template <class S, bool PRE>
-__global__ void __launch_bounds__(XTHR) k_sgemm_x3(const UnitD* __restrict__ units, const TileD* __restrict__ tiles,
-                                                   const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
-                                                   const uint16_t* __restrict__ klist, const float* __restrict__ Wh,
-                                                   const float* __restrict__ Wl, const float* __restrict__ Th,
-                                                   const float* __restrict__ Tl, double* __restrict__ Sm) {
-    __shared__ XStage<S, PRE> st[2];
-    const TileD tile = tiles[blockIdx.x];
+__device__ __forceinline__ void x3_tile(XStage<S, PRE>* st, const TileD& tile, const UnitD* __restrict__ units,
+                                        const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
+                                        const uint16_t* __restrict__ klist, const float* __restrict__ Wh,
+                                        const float* __restrict__ Wl, const float* __restrict__ Th,
+                                        const float* __restrict__ Tl, double* __restrict__ Sm) {
     const UnitD U = units[tile.item];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -239,6 +238,29 @@ __global__ void __launch_bounds__(XTHR) k_sgemm_x3(const UnitD* __restrict__ uni
                 for (int c = 0; c < 2; ++c)
                     if (cof[j][c] != 0xffffffffu) srow[cof[j][c]] = double(acc[i][j][2 * h + c]);
         }
+}
+
+// all shapes in one launch (PRE: the 64 x 64 and 128 x 32 tiles, the others run on tcgen05)
+template <bool PRE>
+__global__ void __launch_bounds__(XTHR, 5) k_sgemm_x3(TileSet<TileD> set, const UnitD* __restrict__ units,
+                                                      const uint32_t* __restrict__ line_b1,
+                                                      const uint64_t* __restrict__ slice_off, const uint16_t* __restrict__ klist,
+                                                      const float* __restrict__ Wh, const float* __restrict__ Wl,
+                                                      const float* __restrict__ Th, const float* __restrict__ Tl,
+                                                      double* __restrict__ Sm) {
+    constexpr std::size_t wide = sizeof(XStage<X64, PRE>) > sizeof(XStage<X128, PRE>) ? sizeof(XStage<X64, PRE>) : sizeof(XStage<X128, PRE>);
+    constexpr std::size_t flat = sizeof(XStage<X16, PRE>) > sizeof(XStage<X32, PRE>) ? sizeof(XStage<X16, PRE>) : sizeof(XStage<X32, PRE>);
+    __shared__ __align__(16) unsigned char raw[2 * (PRE || wide > flat ? wide : flat)];
+    TileD tile;
+    const int sh = set.find(blockIdx.x, tile);
+    if (sh == SHAPE_128)
+        x3_tile<X128, PRE>(reinterpret_cast<XStage<X128, PRE>*>(raw), tile, units, line_b1, slice_off, klist, Wh, Wl, Th, Tl, Sm);
+    else if (sh == SHAPE_64)
+        x3_tile<X64, PRE>(reinterpret_cast<XStage<X64, PRE>*>(raw), tile, units, line_b1, slice_off, klist, Wh, Wl, Th, Tl, Sm);
+    else if (!PRE && sh == SHAPE_32)
+        x3_tile<X32, false>(reinterpret_cast<XStage<X32, false>*>(raw), tile, units, line_b1, slice_off, klist, Wh, Wl, Th, Tl, Sm);
+    else if (!PRE)
+        x3_tile<X16, false>(reinterpret_cast<XStage<X16, false>*>(raw), tile, units, line_b1, slice_off, klist, Wh, Wl, Th, Tl, Sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -457,12 +479,16 @@ __global__ void k_split(const double* __restrict__ x, float* __restrict__ hi, fl
     }
 }
 
-template <class S, bool PRE>
-void launch_x3(const HeffPlan& p, int sh, const float* Wh, const float* Wl, const float* Th, const float* Tl, double* Sm,
+// the tiles of the shapes from `lowest` up
+template <bool PRE>
+void launch_x3(const HeffPlan& p, int lowest, const float* Wh, const float* Wl, const float* Th, const float* Tl, double* Sm,
                cudaStream_t s) {
-    if (p.utiles[sh].empty()) return;
-    k_sgemm_x3<S, PRE><<<unsigned(p.utiles[sh].size()), XTHR, 0, s>>>(p.d_units.get(), p.d_utiles[sh].get(), p.d_line_b1.get(),
-                                                                  p.d_slice_off.get(), p.d_klist.get(), Wh, Wl, Th, Tl, Sm);
+    uint32_t a[N_SHAPES] = {}, b[N_SHAPES] = {}, n;
+    for (int sh = lowest; sh < N_SHAPES; ++sh) b[sh] = uint32_t(p.utiles[sh].size());
+    const TileSet<TileD> set = tile_set(p.d_utiles, a, b, n);
+    if (n)
+        k_sgemm_x3<PRE><<<n, XTHR, 0, s>>>(set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), Wh, Wl,
+                                           Th, Tl, Sm);
 }
 
 template <int BML>
@@ -497,14 +523,10 @@ void run_sgemm_mixed(const HeffPlan& p, bool tc, const float* Wh, const float* W
         // hi / lo operands: tcgen05 for the 16- and 32-line tiles, mma.sync for the others
         launch_tc<16>(p, SHAPE_16, Wh, Wl, Th, Tl, Sm, err, s);
         launch_tc<32>(p, SHAPE_32, Wh, Wl, Th, Tl, Sm, err, s);
-        launch_x3<X64, true>(p, SHAPE_64, Wh, Wl, Th, Tl, Sm, s);
-        launch_x3<X128, true>(p, SHAPE_128, Wh, Wl, Th, Tl, Sm, s);
+        launch_x3<true>(p, SHAPE_64, Wh, Wl, Th, Tl, Sm, s);
     } else {
         // single FP32 operands, split at the fragment loads
-        launch_x3<X16, false>(p, SHAPE_16, Wh, nullptr, Th, nullptr, Sm, s);
-        launch_x3<X32, false>(p, SHAPE_32, Wh, nullptr, Th, nullptr, Sm, s);
-        launch_x3<X64, false>(p, SHAPE_64, Wh, nullptr, Th, nullptr, Sm, s);
-        launch_x3<X128, false>(p, SHAPE_128, Wh, nullptr, Th, nullptr, Sm, s);
+        launch_x3<false>(p, SHAPE_16, Wh, nullptr, Th, nullptr, Sm, s);
     }
     QCM_CUDA(cudaGetLastError());
 }
