@@ -84,6 +84,27 @@ __device__ __forceinline__ void stage_xfast(double* dst, const double* any, uint
         }
     }
 }
+// An apply's kernels are launched as programmatic dependents of one another: each lets the next one start once
+// all its own CTAs run (grid_trigger), so that the next kernel's CTAs load their descriptors into the slots that
+// the last wave leaves empty, and waits (grid_wait) for the one before it to be complete before it touches anything
+// that a kernel writes.  What is read before grid_wait (tiles, jobs, units, k-step lists) is written by copies when a
+// plan is staged, never by a kernel.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+template <class... P, class... X>
+void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned block, cudaStream_t s, X... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    QCM_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 __device__ __forceinline__ bool aligned16(const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---------------------------------------------------------------------------
@@ -101,6 +122,7 @@ __device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, cons
                                            const double* __restrict__ x, const double* __restrict__ R, double* __restrict__ T,
                                            float* __restrict__ Thi, float* __restrict__ Tlo) {
     const TJobD J = jobs[tile.item];
+    grid_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nm = min(uint32_t(S::BM), J.M - tile.m0), nn = min(uint32_t(S::BN), J.N - tile.n0);
     const uint32_t nk = (J.K + BK - 1) / BK;
@@ -190,6 +212,7 @@ __global__ void __launch_bounds__(NTHR, 5) k_tgemm(TileSet<TileD> set, const TJo
                                                    double* __restrict__ T, float* __restrict__ Thi, float* __restrict__ Tlo) {
     __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64>()];
     __shared__ uint64_t colbase[128];
+    grid_trigger();
     TileD tile;
     const int sh = set.find(blockIdx.x, tile);
     if (sh == SHAPE_64) tgemm_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
@@ -209,6 +232,7 @@ __device__ __forceinline__ void sgemm_tile(Stage<S>* st, const TileD& tile, cons
     // only the k-steps whose coefficient block (this tile's lines x 16 slices) holds an entry
     const uint16_t* ks = klist + tile.pad;
     const uint32_t nsteps = ks[0];
+    grid_wait();
     const double* Wu = W + (U.w_off - w0);  // W holds the coefficient blocks from element w0 on
     // 16-byte chunks (2 doubles): W_u columns (ld wld, rows nl .. wld - 1 zero) and T slices (sst
     // apart, 16-byte aligned) are read 16 bytes at a time; a chunk past the slice's ne elements
@@ -301,6 +325,7 @@ __global__ void __launch_bounds__(NTHR, 5) k_sgemm(TileSet<TileD> set, const Uni
                                                    const uint16_t* __restrict__ klist, const double* __restrict__ W,
                                                    const double* __restrict__ T, double* __restrict__ Sm, uint64_t w0) {
     __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64, Sh128>()];
+    grid_trigger();
     TileD tile;
     const int sh = set.find(blockIdx.x, tile);
     if (sh == SHAPE_128) sgemm_tile<Sh128>(reinterpret_cast<Stage<Sh128>*>(raw), tile, units, line_b1, slice_off, klist, W, T, Sm, w0);
@@ -468,6 +493,7 @@ __device__ __forceinline__ void lspart_tile(Stage<S>* st, uint64_t (*kbase)[BK],
     const OTileD ot = otiles[it.tile];
     const OutD O = outs[ot.out];
     const SegD sg = segs[it.seg];
+    grid_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t M = O.M, Kc = sg.nS * sg.ls_in;
     const uint32_t nm = min(uint32_t(S::BM), M - ot.m0), nn = min(uint32_t(S::BN), O.N - ot.n0);
@@ -545,6 +571,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_lspart(TileSet<KItemD> set, OTileSe
                                                     const double* __restrict__ Sm, double* __restrict__ P) {
     __shared__ __align__(16) unsigned char raw[stage_bytes<Sh16, Sh32, Sh64>()];
     __shared__ uint64_t kbase[2][BK];
+    grid_trigger();
     KItemD it;
     const int sh = set.find(blockIdx.x, it);
     if (sh == SHAPE_64)
@@ -561,11 +588,13 @@ __global__ void __launch_bounds__(256) k_lsreduce(TileSet<OTileD> set, OTileSet 
                                                   const double* __restrict__ P, double* __restrict__ y) {
     // one thread per tile element (blockIdx.y: the tile's 256-element chunk): the element's partials are
     // added in item order; the unrolled loop keeps several of its loads in flight
+    grid_trigger();
     OTileD ot;
     const int sh = set.find(blockIdx.x, ot);
     const uint32_t bm = sh == SHAPE_64 ? Sh64::BM : (sh == SHAPE_32 ? Sh32::BM : Sh16::BM);
     const uint32_t bn = sh == SHAPE_64 ? Sh64::BN : Sh32::BN;
     const OutD O = outs[ot.out];
+    grid_wait();
     const uint32_t e = blockIdx.y * blockDim.x + threadIdx.x;
     if (e >= bm * bn) return;
     const uint32_t gm = ot.m0 + e % bm, gn = ot.n0 + e / bm;
@@ -581,14 +610,14 @@ __global__ void __launch_bounds__(256) k_lsreduce(TileSet<OTileD> set, OTileSet 
 void launch_t(HeffPlan& p, const double* x, double* Tb, cudaStream_t s, float* Thi = nullptr, float* Tlo = nullptr) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_ttiles, p.ttiles, n);
-    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, p.d_tjobs.get(), x, p.r_data(), Tb, Thi, Tlo);
+    if (n) launch_dependent(k_tgemm, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, Thi, Tlo);
 }
 
 void launch_s(HeffPlan& p, const double* Tb, double* Sb, cudaStream_t s) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_utiles, p.utiles, n);
     if (n)
-        k_sgemm<<<n, NTHR, 0, s>>>(set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.w_data(), Tb,
+        launch_dependent(k_sgemm, dim3(n), NTHR, s, set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.w_data(), Tb,
                                    Sb, 0);
 }
 
@@ -597,7 +626,7 @@ void launch_s(HeffPlan& p, const double* Tb, double* Sb, cudaStream_t s) {
 void launch_t_chunk(HeffPlan& p, const HeffPlan::SChunk& c, const double* x, double* Tb, cudaStream_t s) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_ttiles, c.tt[0], c.tt[1], n);
-    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, p.d_tjobs.get(), x, p.r_data(), Tb, nullptr, nullptr);
+    if (n) launch_dependent(k_tgemm, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, nullptr, nullptr);
 }
 
 // the S-GEMM tiles [a[sh], b[sh]), reading coefficient blocks that start at element w0
@@ -606,7 +635,7 @@ void launch_s_tiles(HeffPlan& p, const uint32_t* a, const uint32_t* b, uint64_t 
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_utiles, a, b, n);
     if (n)
-        k_sgemm<<<n, NTHR, 0, s>>>(set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.d_W.get(), Tb,
+        launch_dependent(k_sgemm, dim3(n), NTHR, s, set, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), p.d_klist.get(), p.d_W.get(), Tb,
                                    Sb, w0);
 }
 
@@ -622,7 +651,7 @@ OTileSet otile_set(const HeffPlan& p) {
 void launch_ls_chunk(HeffPlan& p, const HeffPlan::SChunk& c, const double* Sb, double* Pb, cudaStream_t s) {
     uint32_t n;
     const TileSet<KItemD> set = tile_set(p.d_kitems, c.kt[0], c.kt[1], n);
-    if (n) k_lspart<<<n, NTHR, 0, s>>>(set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
+    if (n) launch_dependent(k_lspart, dim3(n), NTHR, s, set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
 }
 
 void launch_lsreduce(HeffPlan& p, const double* Pb, double* y, cudaStream_t s, int only = -1) {
@@ -632,7 +661,7 @@ void launch_lsreduce(HeffPlan& p, const double* Pb, double* y, cudaStream_t s, i
     const bool mid = only == SHAPE_32 || (only < 0 && !p.otiles[SHAPE_32].empty());
     const unsigned chunks = tall || mid ? Sh64::BM * Sh64::BN / 256 : Sh16::BM * Sh16::BN / 256;
     static_assert(Sh64::BM * Sh64::BN == Sh32::BM * Sh32::BN, "chunks per tile");
-    if (n) k_lsreduce<<<dim3(n, chunks), 256, 0, s>>>(set, otile_set(p), p.d_outs.get(), Pb, y);
+    if (n) launch_dependent(k_lsreduce, dim3(n, chunks), 256, s, set, otile_set(p), p.d_outs.get(), Pb, y);
 }
 
 void launch_ls(HeffPlan& p, const double* Sb, double* Pb, double* y, cudaStream_t s) {
@@ -641,7 +670,7 @@ void launch_ls(HeffPlan& p, const double* Sb, double* Pb, double* y, cudaStream_
         uint32_t n;
         const TileSet<KItemD> set = tile_set(p.d_kitems, p.kitems, n, sh);
         if (!n) continue;
-        k_lspart<<<n, NTHR, 0, s>>>(set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
+        launch_dependent(k_lspart, dim3(n), NTHR, s, set, otile_set(p), p.d_outs.get(), p.d_segs.get(), p.l_data(), Sb, Pb);
         launch_lsreduce(p, Pb, y, s, sh);
     }
 }
