@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(32) k_brr(int ns, int it, const double* __rest
         V[r][c] = r == c ? 1.0 : 0.0;
     }
     __syncwarp();
+    double last = 0.0;  // off-diagonal part of the sweep before
     for (int sweep = 0; sweep < 100; ++sweep) {
         double off = 0.0, tot = 0.0;
         for (int e = lane; e < n * n; e += 32) {
@@ -121,7 +122,8 @@ __global__ void __launch_bounds__(32) k_brr(int ns, int it, const double* __rest
             off += __shfl_xor_sync(0xffffffffu, off, o);
             tot += __shfl_xor_sync(0xffffffffu, tot, o);
         }
-        if (off <= 1e-32 * tot || off == 0.0) break;
+        if (jacobi_done(off, tot, last, sweep)) break;
+        last = off;
         for (int p = 0; p < n - 1; ++p)
             for (int q = p + 1; q < n; ++q) {
                 const double apq = A[p][q];

@@ -124,11 +124,13 @@ void sym_lowest_eigenpair(const double* M, int ldm, int n, double& w, std::vecto
     for (int i = 0; i < n; ++i) V[i + std::size_t(i) * n] = 1.0;
     auto a = [&](int i, int j) -> double& { return A[i + std::size_t(j) * n]; };
     // cyclic Jacobi (Golub & Van Loan, Algorithm 8.5.3) until the off-diagonal part is negligible
+    double last = 0.0;  // off-diagonal part of the sweep before
     for (int sweep = 0; sweep < 100; ++sweep) {
         double off = 0.0, tot = 0.0;
         for (int j = 0; j < n; ++j)
             for (int i = 0; i < n; ++i) { tot += a(i, j) * a(i, j); if (i != j) off += a(i, j) * a(i, j); }
-        if (off <= 1e-32 * tot || off == 0.0) break;
+        if (jacobi_done(off, tot, last, sweep)) break;
+        last = off;
         for (int p = 0; p < n - 1; ++p)
             for (int q = p + 1; q < n; ++q) {
                 double apq = a(p, q);

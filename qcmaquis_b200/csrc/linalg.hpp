@@ -116,6 +116,13 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
                 uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, std::unique_ptr<SideStreams>& side,
                 cudaStream_t s, uint32_t* P = nullptr, uint64_t p_len = 0);
 
+// Does a cyclic Jacobi diagonalisation end before sweep `sweep`?  off, tot: sums of squares of the off-diagonal and of
+// all elements; last: off before the previous sweep.  Sweeps converge quadratically down to rounding (off about
+// n^2 eps^2 tot, which can lie above 1e-32 tot for good): there a sweep no longer halves off, and no later one
+// improves the result.  Waiting for 1e-32 alone ran most matrices of more than 8 rows to the limit of 100 sweeps.
+__host__ __device__ inline bool jacobi_done(double off, double tot, double last, int sweep) {
+    return off == 0.0 || off <= 1e-32 * tot || (sweep > 0 && off >= 0.5 * last && off <= 1e-28 * tot);
+}
 // Lowest eigenpair of the symmetric n x n matrix held in the upper triangle of
 // M (column-major, leading dimension ldm); cyclic Jacobi rotations, FP64.
 // Replaces the dsyevx(range='I', il=iu=1) call of ietl/jacobi.h:476-516.
