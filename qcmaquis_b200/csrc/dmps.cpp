@@ -424,7 +424,7 @@ void preconditioned_svd(Ctx& c, const DBlocks& both, BlockSVD& r, int* zero_coun
         pl += kk;
         qj.push_back(QrJob{both.off[k], qo, xo, wq, m, n, tall ? 0u : 1u, QR_PIVOT | (tall ? QR_RT : 0u), po});
         wq += qr_scratch(m, n, !tall);
-        sj.push_back(SvdJob{xo, xo, r.so[k], xo, wj, kk, kk, uint32_t(k), 0});
+        sj.push_back(SvdJob{xo, xo, r.so[k], xo, wj, kk, kk, uint32_t(k), 0, 0});
         wj += jacobi_svd_scratch(kk, kk);
         GemmJob g{};
         g.alpha = 1.0; g.beta = 0.0;

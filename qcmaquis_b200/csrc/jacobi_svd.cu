@@ -17,6 +17,11 @@
 // to all of them (distributed shared memory), and after one cluster barrier each CTA adds the partials in rank
 // order and derives the same rotations, one thread per pair.  A second cluster barrier per round (the partials
 // may be overwritten) is split: it is arrived at before the rotations and waited for after them.
+//
+// The largest blocks (more than about 420 columns on 16 CTAs) leave no shared memory for Q, and rotating it in L2
+// took three quarters of their time.  Nothing in the iteration reads Q, and its rows take the same rotations
+// independently of one another: these blocks write their rotations to a log, and k_jacobi_rows applies it to slices
+// of rows that fit shared memory, LOG_SWEEPS sweeps at a time.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -42,8 +47,11 @@ constexpr uint32_t JMAX_CLUSTER = 16;
 // Where a block's work arrays live in a cluster of nc CTAs: per CTA hr rows of G and hq rows of Q (even, so
 // that columns start on 16 bytes), each in shared memory if it fits there after the fixed part (norms, rotation
 // angles, partial dot products, ranks), else in the block's scratch (L2-resident).
+// In a cluster the columns are ldg and ldq apart, 64 bytes off a multiple of 128 if that takes at most a quarter more:
+// four lanes read a short column, and two neighbouring columns' lanes then share no bank.
+// Two buffers of partials (a round needs no second barrier then), or one if G fits only beside one.
 struct JacobiLayout {
-    uint32_t hr, hq, fixed;
+    uint32_t hr, hq, ldg, ldq, fixed, nbuf;
     bool g_smem, q_smem;
 };
 __host__ __device__ inline JacobiLayout jacobi_layout(uint32_t r, uint32_t c, uint32_t nc, uint32_t smem_doubles) {
@@ -51,23 +59,43 @@ __host__ __device__ inline JacobiLayout jacobi_layout(uint32_t r, uint32_t c, ui
     l.hr = ((r + nc - 1) / nc + 1) / 2 * 2;
     l.hq = ((c + nc - 1) / nc + 1) / 2 * 2;
     const uint32_t np = (c + 1) / 2;
-    l.fixed = (c + 2 * np + nc * np + (c + 1) / 2 + 3) / 2 * 2;
-    const uint64_t g = uint64_t(l.hr) * c, q = uint64_t(l.hq) * c;
-    l.g_smem = l.fixed + g <= smem_doubles;
-    l.q_smem = l.g_smem && l.fixed + g + q <= smem_doubles;
-    return l;
+    auto padded = [nc](uint32_t h) {
+        const uint32_t p = (h + 7) / 16 * 16 + 8;
+        return nc > 1 && 4 * p <= 5 * h ? p : h;
+    };
+    l.ldg = padded(l.hr);
+    l.ldq = padded(l.hq);
+    const uint64_t g = uint64_t(l.ldg) * c, q = uint64_t(l.ldq) * c;
+    for (l.nbuf = nc > 1 ? 2 : 1;; l.nbuf = 1) {
+        l.fixed = (c + 2 * np + l.nbuf * nc * (np + (np & 1u)) + (c + 1) / 2 + 3) / 2 * 2;
+        l.g_smem = l.fixed + g <= smem_doubles;
+        l.q_smem = l.g_smem && l.fixed + g + q <= smem_doubles;
+        if (l.g_smem || l.nbuf == 1) return l;
+    }
 }
 
 // CTAs per block: about 36 rows of each column per CTA.  There a round's shared-memory time (under 1 us up to
-// 100 columns, 2 us at 500) is near its fixed part (barriers, square root and division chain); splitting
-// further only adds CTAs that wait.
+// 100 columns, 2 us at 500) is near its fixed part (barriers, square root chain); splitting further only adds
+// CTAs that wait.  Up to 88 columns one CTA, which has no exchange and one barrier a round.
 inline uint32_t jacobi_cluster(uint32_t r, uint32_t c) {
-    if (c <= 48) return 1;
+    if (c <= 88) return 1;
     const uint32_t rows = std::max(r, c);
     uint32_t nc = 2;
     while (nc < JMAX_CLUSTER && rows > 36 * nc) nc *= 2;
     return nc;
 }
+
+constexpr int LOG_SWEEPS = 4;       // sweeps per launch of a logged block
+constexpr uint32_t ROWS_SLICE = 16;  // rows of Q per CTA of k_jacobi_rows
+constexpr int ROWS_THR = 512;
+static_assert(JMAX_SWEEPS % LOG_SWEEPS == 0, "whole launches");
+// Logged blocks: log: per block (l_off of its job) LOG_SWEEPS sweeps of c' - 1 rounds of c'/2 rotations (cosine, sine);
+// meta: per block of the launch the sweeps of this launch and whether the block is done; launch: their number so far.
+struct JacobiLog {
+    double2* log;
+    int* meta;
+    int launch;
+};
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
@@ -102,39 +130,82 @@ __device__ __forceinline__ void rotate(double2* x, double2* y, uint32_t n2, doub
     }
 }
 
+// cosine cs and sine sn of the rotation that makes two columns orthogonal, and t = sn / cs, from their squared norms
+// al, be and dot product ga: zeta = d / h, d = beta - alpha, h = 2 gamma.  With w = 1 / sqrt(d^2 + h^2) the double
+// angle's cosine is |d| w and its sine h w (sign of d), so c^2 = (1 + |d| w) / 2, s = h w / (2 c) and t = s / c: two
+// reciprocal square roots in the round's serial chain.  d^2 + h^2 outside the range takes the quotients themselves.
+__device__ __forceinline__ void rotation(double al, double be, double ga, double& cs, double& sn, double& tt) {
+    const double d = be - al, h = 2.0 * ga, dh = fma(d, d, h * h);
+    if (dh > 1e-280 && dh < 1e300) {
+        const double w = rsqrt(dh), c2 = fma(0.5 * fabs(d), w, 0.5), rs = rsqrt(c2);
+        cs = c2 * rs;
+        sn = (d >= 0.0 ? 0.5 * h : -0.5 * h) * w * rs;
+        tt = sn * rs;
+    } else {
+        const double zeta = d / h;
+        tt = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+        cs = rsqrt(1.0 + tt * tt);
+        sn = cs * tt;
+    }
+}
+
+// dot product of two columns of 2 n2 elements by a group of gs lanes (all 32 lanes call it; x, y only read if act)
+__device__ __forceinline__ double group_dot(const double2* x, const double2* y, uint32_t n2, uint32_t hl, uint32_t gs, bool act) {
+    double a = 0.0, b = 0.0;
+    if (act)
+        for (uint32_t i = hl; i < n2; i += gs) {
+            const double2 u = x[i], v = y[i];
+            a = fma(u.x, v.x, a);
+            b = fma(u.y, v.y, b);
+        }
+    return group_sum(a + b, gs);
+}
+
+// where a launch's blocks keep their work arrays (known at compile time: shared-memory addresses are a third of the
+// kernel's instructions)
+enum JacobiMode { J_SMEM, J_LOGGED, J_LOGGED_L2 };  // G and Q in shared memory; G there and Q logged; G in the scratch
+
+template <int MODE>
 __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
                                                      double* __restrict__ U, double* __restrict__ S, double* __restrict__ V,
-                                                     double* __restrict__ Wg, uint32_t smem_doubles,
-                                                     int* __restrict__ zero_count, int* __restrict__ sweeps_used) {
+                                                     double* __restrict__ Wg, int* __restrict__ zero_count,
+                                                     int* __restrict__ sweeps_used, JacobiLog lg) {
     extern __shared__ __align__(16) double smem[];
     __shared__ int rotated;
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t nc = cl.num_blocks(), rank = cl.block_rank();
     const SvdJob J = jobs[blockIdx.x / nc];
+    constexpr bool logged = MODE != J_SMEM;
+    int* meta = lg.meta + 2 * (blockIdx.x / nc);
+    if (logged && lg.launch > 0 && meta[1]) return;  // the whole cluster: done in an earlier launch
     const bool tall = J.m >= J.n;
     const uint32_t r = tall ? J.m : J.n, c = tall ? J.n : J.m;
-    const JacobiLayout l = jacobi_layout(r, c, nc, smem_doubles);
-    const uint32_t hr = l.hr, hq = l.hq, cp = c + (c & 1u), np = cp / 2;
-    double* nrm = smem;         // c
-    double* rcs = nrm + c;      // np, then np sines
-    double* rsn = rcs + np;
-    double* part = rsn + np;    // nc x np partial dot products, by rank
-    uint32_t* rank_of = reinterpret_cast<uint32_t*>(part + nc * np);  // c
-    double* scratch = Wg + J.w_off + uint64_t(rank) * (hr + hq) * c;
-    double* G = l.g_smem ? smem + l.fixed : scratch;
-    double* Q = l.q_smem ? smem + l.fixed + uint64_t(hr) * c : scratch + uint64_t(hr) * c;
+    const JacobiLayout l = jacobi_layout(r, c, nc, JSMEM_DOUBLES);  // as the launch does
+    const uint32_t hr = l.hr, hq = l.hq, ldg = l.ldg, ldq = l.ldq, cp = c + (c & 1u), np = cp / 2, npe = np + (np & 1u);
+    double2* rot = reinterpret_cast<double2*>(smem);  // np: the round's rotations (cosine, sine)
+    double* part = smem + 2 * np;                     // nbuf x nc x npe partial dot products, by rank
+    double* nrm = part + l.nbuf * nc * npe;           // c
+    uint32_t* rank_of = reinterpret_cast<uint32_t*>(nrm + c);  // c
+    double* scratch = Wg + J.w_off + uint64_t(rank) * (ldg + ldq) * c;
+    double* G = MODE == J_LOGGED_L2 ? scratch : smem + l.fixed;
+    double* Q = smem + l.fixed + ldg * c;  // unless logged
     const uint32_t nthr = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr / 32;
     const uint32_t r0 = rank * hr, q0 = rank * hq;  // first rows of this CTA
-    // G = A or A^T, Q = I
+    // G = A or A^T, Q = I (a logged block goes on from the G it left in the scratch)
     const double* a = A + J.a_off;
-    for (uint32_t i = tid; i < hr * c; i += nthr) {
-        const uint32_t col = i / hr, row = r0 + (i - col * hr);
-        G[i] = row >= r ? 0.0 : (tall ? a[row + uint64_t(col) * J.m] : a[col + uint64_t(row) * J.m]);
+    if (!logged || lg.launch == 0) {
+        for (uint32_t i = tid; i < hr * c; i += nthr) {
+            const uint32_t col = i / hr, k = i - col * hr, row = r0 + k;
+            G[col * ldg + k] = row >= r ? 0.0 : (tall ? a[row + uint64_t(col) * J.m] : a[col + uint64_t(row) * J.m]);
+        }
+    } else if (MODE == J_LOGGED) {
+        for (uint32_t i = tid; i < ldg * c; i += nthr) G[i] = scratch[i];
     }
-    for (uint32_t i = tid; i < hq * c; i += nthr) {
-        const uint32_t col = i / hq;
-        Q[i] = q0 + (i - col * hq) == col ? 1.0 : 0.0;
-    }
+    if (!logged)
+        for (uint32_t i = tid; i < hq * c; i += nthr) {
+            const uint32_t col = i / hq, k = i - col * hq;
+            Q[col * ldq + k] = q0 + k == col ? 1.0 : 0.0;
+        }
     __syncthreads();
     const double tol2 = (JEPS * double(r)) * (JEPS * double(r));
     auto cluster_sync = [&] {
@@ -145,41 +216,68 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
             __syncthreads();
         }
     };
-    // a value of rank `rank` at part[rank][t] of every CTA, written by the first nc of the group's lanes
-    auto send = [&](uint32_t t, double v, uint32_t hl, uint32_t gs) {
-        if (nc == 1) {
-            if (hl == 0) part[t] = v;
-            return;
-        }
-        for (uint32_t d = hl; d < nc; d += gs) cl.map_shared_rank(part, d)[rank * np + t] = v;
+    // An exchange: every CTA's partial of item t goes to its row of the buffer in all CTAs (put, by the group's lanes);
+    // after the barrier (arrived) gather adds them in rank order.  With one buffer it may be filled again once all CTAs
+    // have gathered: they arrive at a second barrier then (gathered), waited for before the next put (free).
+    uint32_t par = 0;  // this exchange's buffer
+    auto put = [&](uint32_t t, double v, uint32_t hl, uint32_t gs) {
+        double* b = part + (par * nc + rank) * npe + t;
+        for (uint32_t d = hl; d < nc; d += gs) *cl.map_shared_rank(b, d) = v;
     };
     auto gather = [&](uint32_t t) {
-        double s = part[t];
-        for (uint32_t d = 1; d < nc; ++d) s += part[d * np + t];
+        const double* b = part + par * nc * npe + t;
+        double s = b[0];
+        for (uint32_t d = 1; d < nc; ++d) s += b[d * npe];
         return s;
+    };
+    bool wait_free = false;  // one buffer: the exchange before is still being gathered
+    auto free = [&] {
+        if (wait_free) cluster_wait();
+        wait_free = false;
+    };
+    auto gathered = [&] {  // all lanes of a warp together
+        if (l.nbuf == 2) {
+            par ^= 1;
+        } else {
+            cluster_arrive();
+            wait_free = true;
+        }
     };
     // nrm[j] = |G_j|^2 over all rows, half the columns at a time (the partials' buffer holds np values)
     auto column_norms = [&] {
         for (uint32_t j0 = 0; j0 < c; j0 += np) {
             const uint32_t j1 = min(c, j0 + np);
+            if (nc > 1) free();
             for (uint32_t j = j0 + warp; j < j1; j += nwarp) {
-                const double* g = G + uint64_t(j) * hr;
+                const double* g = G + j * ldg;
                 double x = 0.0;
                 for (uint32_t i = lane; i < hr; i += 32) x = fma(g[i], g[i], x);
-                send(j - j0, warp_sum(x), lane, 32);
+                x = warp_sum(x);
+                if (nc > 1) put(j - j0, x, lane, 32);
+                else if (lane == 0) nrm[j] = x;
             }
             cluster_sync();
+            if (nc == 1) continue;
             for (uint32_t j = j0 + tid; j < j1; j += nthr) nrm[j] = gather(j - j0);
-            cluster_sync();
+            __syncwarp();
+            gathered();
         }
+        __syncthreads();
     };
-    // lanes per pair: enough groups for all pairs of a round in one pass if the columns are long enough to
-    // keep the lanes busy (two elements per lane and step)
+    // lanes per pair: the least passes over the pairs times steps along a column (two elements per lane), a pass's
+    // fixed part counted as four steps
     uint32_t gs = 16;
-    while (gs > 4 && (np * gs > nthr || hr / 2 < gs)) gs >>= 1;
+    for (uint32_t g = 16, best = 0xffffffffu; g >= 4; g >>= 1) {
+        const uint32_t cost = (np * g + nthr - 1) / nthr * ((hr / 2 + g - 1) / g + 4);
+        if (cost < best) { best = cost; gs = g; }
+    }
     const uint32_t grp = tid / gs, hl = tid % gs, ngrp = nthr / gs;
-    for (int sweep = 0; sweep < JMAX_SWEEPS && c > 1; ++sweep) {
+    const int sweep0 = logged ? lg.launch * LOG_SWEEPS : 0, sweep1 = logged ? sweep0 + LOG_SWEEPS : JMAX_SWEEPS;
+    int sweep = sweep0;
+    bool done = c <= 1;
+    for (; sweep < sweep1 && !done; ++sweep) {
         if (tid == 0) rotated = 0;
+        double2* lgs = logged ? lg.log + J.l_off + uint64_t(sweep - sweep0) * (cp - 1) * np : nullptr;
         column_norms();
         for (uint32_t k = 0; k + 1 < cp; ++k) {
             // every lane runs the same number of passes so the group shuffles never diverge
@@ -187,21 +285,33 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
                 const uint32_t t = pass * ngrp + grp;
                 uint32_t p = 0, q = 0;
                 const bool act = t < np && pair_of(t, k, cp, c, p, q);
-                double ga = 0.0;
-                if (act) {
-                    const double2* gp = reinterpret_cast<const double2*>(G + uint64_t(p) * hr);
-                    const double2* gq = reinterpret_cast<const double2*>(G + uint64_t(q) * hr);
-                    double g2 = 0.0;
-                    for (uint32_t i = hl; i < hr / 2; i += gs) {
-                        const double2 x = gp[i], y = gq[i];
-                        ga = fma(x.x, y.x, ga);
-                        g2 = fma(x.y, y.y, g2);
+                double2* gp = reinterpret_cast<double2*>(G + p * ldg);
+                double2* gq = reinterpret_cast<double2*>(G + q * ldg);
+                const double ga = group_dot(gp, gq, hr / 2, hl, gs, act);
+                if (nc == 1) {
+                    // a block of one CTA needs no exchange: each group rotates its pair at once, one barrier a round
+                    const double al = act ? nrm[p] : 0.0, be = act ? nrm[q] : 0.0;
+                    if (act && ga * ga > tol2 * (al * be)) {
+                        double cs, sn, tt;
+                        rotation(al, be, ga, cs, sn, tt);
+                        rotate(gp, gq, hr / 2, cs, sn, hl, gs);
+                        rotate(reinterpret_cast<double2*>(Q + p * ldq), reinterpret_cast<double2*>(Q + q * ldq),
+                               hq / 2, cs, sn, hl, gs);
+                        if (hl == 0) {
+                            nrm[p] = al - tt * ga;
+                            nrm[q] = be + tt * ga;
+                            rotated = 1;
+                        }
                     }
-                    ga += g2;
+                    __syncwarp();
+                    continue;
                 }
-                ga = group_sum(ga, gs);
-                if (pass == 0 && k > 0 && nc > 1) cluster_wait();  // the previous round's partials have been read
-                if (act) send(t, ga, hl, gs);
+                if (pass == 0) free();
+                if (act) put(t, ga, hl, gs);
+            }
+            if (nc == 1) {
+                __syncthreads();
+                continue;
             }
             cluster_sync();
             for (uint32_t t = tid; t < np; t += nthr) {
@@ -210,49 +320,49 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
                 if (pair_of(t, k, cp, c, p, q)) {
                     const double ga = gather(t), al = nrm[p], be = nrm[q];
                     if (ga * ga > tol2 * (al * be)) {
-                        // t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), zeta = d / h, d = beta - alpha, h = 2 gamma,
-                        // multiplied through by |h| (one square root and one division) unless d^2 + h^2 could
-                        // overflow
-                        const double d = be - al, h = 2.0 * ga;
                         double tt;
-                        if (fabs(d) < 1e150 && fabs(h) < 1e150) {
-                            tt = (d >= 0.0 ? h : -h) / (fabs(d) + sqrt(fma(d, d, h * h)));
-                        } else {
-                            const double zeta = d / h;
-                            tt = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                        }
-                        cs = rsqrt(1.0 + tt * tt);
-                        sn = cs * tt;
+                        rotation(al, be, ga, cs, sn, tt);
                         nrm[p] = al - tt * ga;
                         nrm[q] = be + tt * ga;
                         rotated = 1;
                     }
                 }
-                rcs[t] = cs;
-                rsn[t] = sn;
+                rot[t] = make_double2(cs, sn);
+                if (logged && t % nc == rank) lgs[uint64_t(k) * np + t] = make_double2(cs, sn);
             }
             __syncwarp();
-            if (nc > 1) cluster_arrive();  // waited for before the next partials are sent
+            gathered();
             __syncthreads();
             for (uint32_t t = grp; t < np; t += ngrp) {
-                const double cs = rcs[t], sn = rsn[t];
+                const double2 cs = rot[t];
                 uint32_t p, q;
-                if ((cs == 1.0 && sn == 0.0) || !pair_of(t, k, cp, c, p, q)) continue;
-                rotate(reinterpret_cast<double2*>(G + uint64_t(p) * hr), reinterpret_cast<double2*>(G + uint64_t(q) * hr),
-                       hr / 2, cs, sn, hl, gs);
-                rotate(reinterpret_cast<double2*>(Q + uint64_t(p) * hq), reinterpret_cast<double2*>(Q + uint64_t(q) * hq),
-                       hq / 2, cs, sn, hl, gs);
+                if ((cs.x == 1.0 && cs.y == 0.0) || !pair_of(t, k, cp, c, p, q)) continue;
+                rotate(reinterpret_cast<double2*>(G + p * ldg), reinterpret_cast<double2*>(G + q * ldg),
+                       hr / 2, cs.x, cs.y, hl, gs);
+                if (!logged)
+                    rotate(reinterpret_cast<double2*>(Q + p * ldq), reinterpret_cast<double2*>(Q + q * ldq),
+                           hq / 2, cs.x, cs.y, hl, gs);
             }
             __syncthreads();
         }
-        if (nc > 1) cluster_wait();
         const int any = rotated;
         __syncthreads();
-        if (sweeps_used && rank == 0 && tid == 0) sweeps_used[J.id] = sweep + 1;
-        if (!any) break;
+        done = !any;
+    }
+    if (sweeps_used && rank == 0 && tid == 0) sweeps_used[J.id] = sweep;
+    if (logged) {
+        done = done || sweep == JMAX_SWEEPS;
+        if (rank == 0 && tid == 0) { meta[0] = sweep - sweep0; meta[1] = done ? 1 : 0; }
+        if (!done) {
+            if (MODE == J_LOGGED)
+                for (uint32_t i = tid; i < ldg * c; i += nthr) scratch[i] = G[i];
+            if (nc > 1) free();
+            return;  // every CTA of the cluster has passed its last exchange
+        }
     }
     // sigma_j = |G_j| and its rank in descending order (ties by index)
     column_norms();
+    if (nc > 1) free();
     for (uint32_t j = tid; j < c; j += nthr) nrm[j] = sqrt(nrm[j]);
     __syncthreads();
     double* sv = S + J.s_off;
@@ -266,6 +376,7 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
         }
         rank_of[j] = rk;
         if (rank == 0) {
+            if (logged) lg.log[J.l_off + uint64_t(LOG_SWEEPS) * (cp - 1) * np + j].x = double(rk);
             sv[rk] = x;
             zeros += x == 0.0 ? 1 : 0;
         }
@@ -276,15 +387,67 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
     double* Gout = tall ? U + J.u_off : V + J.v_off;   // r x c, ld r
     double* Qout = tall ? V + J.v_off : U + J.u_off;   // c x c, ld c
     for (uint32_t i = tid; i < hr * c; i += nthr) {
-        const uint32_t col = i / hr, row = r0 + (i - col * hr);
+        const uint32_t col = i / hr, k = i - col * hr, row = r0 + k;
         if (row >= r) continue;
         const double sg = nrm[col];
-        Gout[row + uint64_t(rank_of[col]) * r] = sg > 0.0 ? G[i] / sg : 0.0;
+        Gout[row + uint64_t(rank_of[col]) * r] = sg > 0.0 ? G[col * ldg + k] / sg : 0.0;
     }
+    if (logged) return;
     for (uint32_t i = tid; i < hq * c; i += nthr) {
-        const uint32_t col = i / hq, row = q0 + (i - col * hq);
-        if (row < c) Qout[row + uint64_t(rank_of[col]) * c] = Q[i];
+        const uint32_t col = i / hq, k = i - col * hq, row = q0 + k;
+        if (row < c) Qout[row + uint64_t(rank_of[col]) * c] = Q[col * ldq + k];
     }
+}
+
+// The logged rotations of k_jacobi_svd's last launch applied to ROWS_SLICE rows of Q (grid: slice, block).  Between
+// launches Q waits in its output buffer, its columns in their own order; when its block is done they are written
+// in the order of the singular values.  One half-warp per pair, a lane per row: the columns of a pair are two
+// conflict-free rows of shared memory, whose bandwidth binds.
+__global__ void __launch_bounds__(ROWS_THR) k_jacobi_rows(const SvdJob* __restrict__ jobs, double* __restrict__ U,
+                                                          double* __restrict__ V, JacobiLog lg, int launch) {
+    extern __shared__ __align__(16) double q[];  // [column][ROWS_SLICE]
+    const SvdJob J = jobs[blockIdx.y];
+    const bool tall = J.m >= J.n;
+    const uint32_t c = tall ? J.n : J.m, cp = c + (c & 1u), np = cp / 2;
+    const uint32_t row0 = blockIdx.x * ROWS_SLICE;
+    const int nsweeps = lg.meta[2 * blockIdx.y], done = lg.meta[2 * blockIdx.y + 1];
+    if (row0 >= c || done > 1) return;  // 2: written by an earlier launch
+    double* Qout = tall ? V + J.v_off : U + J.u_off;  // c x c, ld c
+    const uint32_t lane = threadIdx.x % ROWS_SLICE, grp = threadIdx.x / ROWS_SLICE, ngrp = ROWS_THR / ROWS_SLICE;
+    const uint32_t row = row0 + lane;
+    for (uint32_t j = grp; j < c; j += ngrp)
+        q[j * ROWS_SLICE + lane] = launch == 0 ? (row == j ? 1.0 : 0.0) : (row < c ? Qout[row + uint64_t(j) * c] : 0.0);
+    __syncthreads();
+    const double2* log = lg.log + J.l_off;
+    for (int sweep = 0; sweep < nsweeps; ++sweep)
+        for (uint32_t k = 0; k + 1 < cp; ++k) {
+            for (uint32_t t = grp; t < np; t += ngrp) {
+                const double2 cs = log[t];
+                uint32_t p, r;
+                if ((cs.x == 1.0 && cs.y == 0.0) || !pair_of(t, k, cp, c, p, r)) continue;
+                const double x = q[p * ROWS_SLICE + lane], y = q[r * ROWS_SLICE + lane];
+                q[p * ROWS_SLICE + lane] = cs.x * x - cs.y * y;
+                q[r * ROWS_SLICE + lane] = cs.y * x + cs.x * y;
+            }
+            log += np;
+            __syncthreads();
+        }
+    const double2* rank_of = lg.log + J.l_off + uint64_t(LOG_SWEEPS) * (cp - 1) * np;
+    if (row < c)
+        for (uint32_t j = grp; j < c; j += ngrp)
+            Qout[row + uint64_t(done ? uint32_t(rank_of[j].x) : j) * c] = q[j * ROWS_SLICE + lane];
+}
+
+// after k_jacobi_rows: blocks that are done are not touched again
+__global__ void k_jacobi_mark(int* meta, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && meta[2 * i + 1]) meta[2 * i + 1] = 2;
+}
+
+// log entries of a block (double2): its rotations, then the rank of every column
+uint64_t log_entries(uint32_t c) {
+    const uint64_t cp = c + (c & 1u);
+    return uint64_t(LOG_SWEEPS) * (cp - 1) * (cp / 2) + c;
 }
 
 }  // namespace
@@ -319,7 +482,7 @@ void SideStreams::join(cudaStream_t to) {
 
 uint64_t jacobi_svd_scratch(uint32_t m, uint32_t n) {
     const uint64_t r = std::max(m, n), c = std::min(m, n);
-    const uint64_t d = (r + c + 4 * JMAX_CLUSTER) * c;  // every CTA's rows rounded up to even
+    const uint64_t d = (r + c + 2 * 18 * JMAX_CLUSTER) * c;  // every CTA's rows, padded (at most 17 each)
     return (d + 31) / 32 * 32;  // whole multiples of 32 doubles: the next block's scratch stays 16-byte aligned
 }
 
@@ -327,9 +490,11 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
                         uint64_t s_len, double* V, uint64_t v_len, double* W, uint64_t w_len, int* zero_count,
                         DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, int* sweeps_used) {
     // one launch per cluster size, the largest first (they take longest), each on a stream of its own
-    constexpr int NCLS = 5;  // 16, 8, 4, 2, 1 CTAs per block
-    static_assert(JMAX_CLUSTER >> (NCLS - 1) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
+    constexpr int NCLS = 7;  // 16 logged (G in L2, in shared memory), then 16, 8, 4, 2, 1 CTAs per block
+    static_assert(JMAX_CLUSTER >> (NCLS - 3) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
     std::vector<SvdJob> cls[NCLS];
+    uint64_t log_len = 0;
+    uint32_t log_cols = 0;
     uint32_t nid = 0;
     for (const SvdJob& j : jobs) {
         nid = std::max(nid, j.id + 1);
@@ -342,10 +507,21 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
         if (j.w_off % 2) throw std::runtime_error("batched_jacobi_svd: scratch offset not 16-byte aligned");
         if (uint64_t(j.m) * j.n > 0x7fffffffu) throw std::runtime_error("batched_jacobi_svd: block too large");
         const uint32_t nc = jacobi_cluster(std::max(j.m, j.n), uint32_t(k));
-        int i = 0;
+        int i = 2;
         for (uint32_t x = JMAX_CLUSTER; x > nc; x /= 2) ++i;
+        if (!jacobi_layout(std::max(j.m, j.n), uint32_t(k), nc, JSMEM_DOUBLES).q_smem) {
+            i = jacobi_layout(std::max(j.m, j.n), uint32_t(k), JMAX_CLUSTER, JSMEM_DOUBLES).g_smem ? 1 : 0;
+            log_cols = std::max(log_cols, uint32_t(k));
+        }
         cls[i].push_back(j);
+        if (i < 2) {
+            cls[i].back().l_off = log_len;
+            log_len += log_entries(uint32_t(k));
+        }
     }
+    DBuf<double2> log(log_len);
+    DBuf<int> metas(2 * (cls[0].size() + cls[1].size()));
+    if (metas.size()) QCM_CUDA(cudaMemsetAsync(metas.get(), 0, metas.size() * sizeof(int), s));
     if (nid) QCM_CUDA(cudaMemsetAsync(zero_count, 0, nid * sizeof(int), s));
     std::vector<SvdJob> all;
     int used = 0;
@@ -359,8 +535,10 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     }
     if (all.empty()) return;
     jobbuf.upload(all, s);
-    QCM_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(JSMEM_DOUBLES * sizeof(double))));
-    QCM_CUDA(cudaFuncSetAttribute(k_jacobi_svd, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (auto* k : {k_jacobi_svd<J_SMEM>, k_jacobi_svd<J_LOGGED>, k_jacobi_svd<J_LOGGED_L2>}) {
+        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(JSMEM_DOUBLES * sizeof(double))));
+        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     if (used > 1 && !side) side = std::make_unique<SideStreams>();
     if (used > 1) side->fork(s);
     std::size_t first = 0;
@@ -368,15 +546,15 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < NCLS && err == cudaSuccess; ++i) {
         if (cls[i].empty()) continue;
-        const uint32_t nc = JMAX_CLUSTER >> i;
+        const uint32_t nc = i < 2 ? JMAX_CLUSTER : JMAX_CLUSTER >> (i - 2);
         // shared memory of the launch's largest block (everything that fits), threads by its pairs per round
         uint64_t sm = 0;
         uint32_t lanes = 0;
         for (const SvdJob& j : cls[i]) {
             const uint32_t r = std::max(j.m, j.n), c = std::min(j.m, j.n);
             const JacobiLayout l = jacobi_layout(r, c, nc, JSMEM_DOUBLES);
-            sm = std::max(sm, l.fixed + (l.g_smem ? uint64_t(l.hr) * c : 0) + (l.q_smem ? uint64_t(l.hq) * c : 0));
-            lanes = std::max(lanes, (c + 1) / 2 * 8);
+            sm = std::max(sm, l.fixed + (i > 0 ? uint64_t(l.ldg) * c : 0) + (i > 1 ? uint64_t(l.ldq) * c : 0));
+            lanes = std::max(lanes, (c + 1) / 2 * (nc == 1 ? 16 : 8));
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(unsigned(cls[i].size()) * nc);
@@ -389,8 +567,27 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        err = cudaLaunchKernelEx(&cfg, k_jacobi_svd, static_cast<const SvdJob*>(jobbuf.get() + first), A, U, S, V, W,
-                                 uint32_t(sm), zero_count, sweeps_used);
+        const SvdJob* dj = jobbuf.get() + first;
+        if (i > 1) {
+            err = cudaLaunchKernelEx(&cfg, k_jacobi_svd<J_SMEM>, dj, A, U, S, V, W, zero_count, sweeps_used,
+                                     JacobiLog{nullptr, nullptr, 0});
+        } else {
+            // LOG_SWEEPS sweeps, then their rotations applied to Q, up to the limit of sweeps (launches after the last
+            // block is done return at once)
+            const std::size_t qb = std::size_t(log_cols) * ROWS_SLICE * sizeof(double);
+            err = cudaFuncSetAttribute(k_jacobi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(qb));
+            const dim3 qg((log_cols + ROWS_SLICE - 1) / ROWS_SLICE, unsigned(cls[i].size()));
+            auto* kernel = i == 0 ? k_jacobi_svd<J_LOGGED_L2> : k_jacobi_svd<J_LOGGED>;
+            int* meta = metas.get() + (i == 0 ? 0 : 2 * cls[0].size());
+            for (int x = 0; x < JMAX_SWEEPS / LOG_SWEEPS && err == cudaSuccess; ++x) {
+                const JacobiLog lg{log.get(), meta, x};
+                err = cudaLaunchKernelEx(&cfg, kernel, dj, A, U, S, V, W, zero_count, sweeps_used, lg);
+                if (err != cudaSuccess) break;
+                k_jacobi_rows<<<qg, ROWS_THR, qb, cfg.stream>>>(dj, U, V, lg, x);
+                k_jacobi_mark<<<unsigned((cls[i].size() + 127) / 128), 128, 0, cfg.stream>>>(meta, int(cls[i].size()));
+                err = cudaGetLastError();
+            }
+        }
         first += cls[i].size();
         ++lane;
     }

@@ -57,7 +57,7 @@ struct Solver {
 void svd_thin_lane(Solver& sv, int l, const double* A, int m, int n, double* U, double* S, double* V, int* info);
 // Streams beside a main one, for launches that run at the same time (fork from / join to the main stream).
 struct SideStreams {
-    static constexpr int N = 4;
+    static constexpr int N = 6;
     cudaStream_t s[N] = {};
     cudaEvent_t fork_ev = nullptr, done[N] = {};
     SideStreams();
@@ -78,6 +78,7 @@ struct SvdJob {
     uint64_t a_off, u_off, s_off, v_off, w_off;  // w_off: scratch of jacobi_svd_scratch(m, n) doubles
     uint32_t m, n;
     uint32_t id, pad;  // zero_count[id] receives the block's number of zero singular values
+    uint64_t l_off;    // set by batched_jacobi_svd
 };
 uint64_t jacobi_svd_scratch(uint32_t m, uint32_t n);
 // Symmetric eigendecomposition (divide and conquer, lower triangle) on lane `l`: A (n x n, ld n)

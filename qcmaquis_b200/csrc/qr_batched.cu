@@ -48,9 +48,11 @@ constexpr uint32_t QR_PIV_MAX = 1024;           // columns of a pivoted factoris
 constexpr uint32_t QR_SMEM_DOUBLES = 28400;     // dynamic shared memory per CTA (222 KiB; 2.4 KiB static)
 constexpr uint32_t QR_MAX_CLUSTER = 16;
 
-// CTAs per block: 64 columns of 64 rows are two passes of the 32 warps, about what a step's barriers cost
+// CTAs per block: 64 columns of 64 rows are two passes of the 32 warps, about what a step's barriers cost; a cluster's
+// barrier costs more than a CTA's, and up to about 112 columns of 112 rows one CTA is the faster
 inline uint32_t qr_cluster(uint32_t mm, uint32_t nn) {
     const uint64_t e = uint64_t(mm) * nn;
+    if (e <= 112 * 112) return 1;
     uint32_t nc = 1;
     while (nc < QR_MAX_CLUSTER && nc * 2 <= nn && e > uint64_t(64 * 64) * nc * nc) nc *= 2;
     return nc;
@@ -90,9 +92,9 @@ struct QrCand {
     uint32_t pos, col;
 };
 __device__ __forceinline__ bool better(double va, uint32_t pa, double vb, uint32_t pb) { return va > vb || (va == vb && pa < pb); }
-// the best candidate of the warp's lanes, in every lane
-__device__ __forceinline__ QrCand warp_best(QrCand c) {
-    for (int o = 16; o > 0; o >>= 1) {
+// the best candidate of each aligned group of n lanes (a power of two), in all of them
+__device__ __forceinline__ QrCand warp_best(QrCand c, int n) {
+    for (int o = n / 2; o > 0; o >>= 1) {
         QrCand d;
         d.val = __shfl_xor_sync(0xffffffffu, c.val, o);
         d.tail = __shfl_xor_sync(0xffffffffu, c.tail, o);
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
         if (warp == 0) {
             QrCand c = wbest[lane < nwarp ? lane : 0];
             if (lane >= nwarp) { c.val = -2.0; c.pos = 0xffffffffu; }
-            c = warp_best(c);
+            c = warp_best(c, 32);
             if (nc == 1) {
                 if (lane == 0) cand[step & 1][0] = c;
             } else if (lane < nc) {
@@ -194,8 +196,7 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
     thr = 64.0 * 2.220446049250313e-16 * sqrt(thr);
     for (uint32_t j = 0; j < k; ++j) {
         // the pivot, the same in every warp of every CTA
-        QrCand pv = lane < nc ? cand[j & 1][lane] : none;
-        pv = warp_best(pv);
+        QrCand pv = warp_best(cand[j & 1][lane & (nc - 1)], int(nc));
         if (pv.pos >= nn) {
             // no candidate compared (NaN columns remain): the column at position j, its values undefined
             pv.pos = j;
