@@ -86,15 +86,45 @@ __global__ void __launch_bounds__(NTHR) k_bgemm(const GemmJob* __restrict__ jobs
     }
 }
 
-__global__ void k_bcopy(const CopyJob* __restrict__ jobs, uint32_t njobs, const double* __restrict__ src,
-                        double* __restrict__ dst) {
+// One CTA per (job, strip of 32 source columns): a warp per column, its rows over the lanes (no division per element);
+// a transposing copy passes 32 x 32 tiles through shared memory, so that both sides move whole lines.  Small copies in
+// one launch: launches, and waits after them, were the cost.  A truncation of the 75 two-site blocks at L=24, M=512 with
+// its results read back: 6.4 ms with a copy and a wait per block and result, 5.4 ms gathered and read in one copy each.
+constexpr int CP_COLS = 32;
+__global__ void __launch_bounds__(256) k_bcopy(const CopyJob* __restrict__ jobs, const double* __restrict__ src,
+                                               double* __restrict__ dst, const double* __restrict__ scale) {
+    __shared__ double tile[CP_COLS][33];
     const CopyJob J = jobs[blockIdx.x];
-    const uint64_t n = uint64_t(J.rows) * J.cols;
-    for (uint64_t e = threadIdx.x; e < n; e += blockDim.x) {
-        uint32_t j = uint32_t(e / J.rows), i = uint32_t(e - uint64_t(j) * J.rows);
-        double v = src[J.src_off + i + uint64_t(J.rev ? J.cols - 1 - j : j) * J.src_ld];
-        if (!J.trans) dst[J.dst_off + i + uint64_t(j) * J.dst_ld] = v;
-        else dst[J.dst_off + j + uint64_t(i) * J.dst_ld] = v;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto column = [&](uint32_t j) { return src + J.src_off + uint64_t(J.rev ? J.cols - 1 - j : j) * J.src_ld; };
+    auto factor = [&](uint32_t j) { return J.scaled ? scale[J.s_off + j] : 1.0; };
+    for (uint64_t strip = uint64_t(blockIdx.y) * CP_COLS; strip < J.cols; strip += uint64_t(gridDim.y) * CP_COLS) {
+        const uint32_t j0 = uint32_t(strip), j1 = uint32_t(min(uint64_t(J.cols), strip + CP_COLS));
+        if (!J.trans) {
+            for (uint32_t j = j0 + warp; j < j1; j += 8) {
+                const double* c = column(j);
+                double* d = dst + J.dst_off + uint64_t(j) * J.dst_ld;
+                if (J.scaled) {
+                    const double f = factor(j);
+                    for (uint32_t i = lane; i < J.rows; i += 32) d[i] = c[i] * f;
+                } else {
+                    for (uint32_t i = lane; i < J.rows; i += 32) d[i] = c[i];
+                }
+            }
+            continue;
+        }
+        for (uint32_t i0 = 0; i0 < J.rows; i0 += 32) {
+            for (uint32_t j = j0 + warp; j < j1; j += 8)
+                if (i0 + lane < J.rows) tile[j - j0][lane] = column(j)[i0 + lane];
+            __syncthreads();
+            const uint32_t j = j0 + lane;
+            if (j < j1)
+                for (uint32_t i = i0 + warp; i < min(J.rows, i0 + 32); i += 8) {
+                    const double v = tile[lane][i - i0];
+                    dst[J.dst_off + j + uint64_t(i) * J.dst_ld] = J.scaled ? v * factor(j) : v;
+                }
+            __syncthreads();
+        }
     }
 }
 
@@ -162,14 +192,6 @@ __global__ void k_fill(double* p, uint64_t n, double v) {
     for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) p[i] = v;
 }
 
-__global__ void k_scale(double* A, uint32_t rows, uint32_t cols, uint32_t lda, const double* __restrict__ d, int by_row) {
-    const uint64_t n = uint64_t(rows) * cols;
-    for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < n; e += uint64_t(gridDim.x) * blockDim.x) {
-        uint32_t j = uint32_t(e / rows), i = uint32_t(e - uint64_t(j) * rows);
-        A[i + uint64_t(j) * lda] *= by_row ? d[i] : d[j];
-    }
-}
-
 unsigned grid_for(uint64_t n, unsigned bs = 256) {
     uint64_t g = (n + bs - 1) / bs;
     return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, 148 * 16)));
@@ -207,26 +229,27 @@ void batched_gemm(const std::vector<GemmJob>& jobs, const double* A, uint64_t a_
     jobbuf.upload(jobs, s);
     tilebuf.upload(reinterpret_cast<const uint32_t*>(tiles.data()), tiles.size() * 4, s);
     k_bgemm<<<unsigned(tiles.size()), NTHR, 0, s>>>(jobbuf.get(), reinterpret_cast<const GTile*>(tilebuf.get()), A, B, C);
+    // no wait: the lists are pageable, so their upload has left them when it returns, and the next call's upload
+    // into the same buffers is ordered behind this launch on the stream
     QCM_CUDA(cudaGetLastError());
-    // job/tile buffers are reused by the next call: keep the host order simple by finishing here
-    QCM_CUDA(cudaStreamSynchronize(s));
 }
 
 void batched_copy(const std::vector<CopyJob>& jobs, const double* src, uint64_t src_len, double* dst, uint64_t dst_len,
-                  DBuf<CopyJob>& jobbuf, cudaStream_t s) {
+                  DBuf<CopyJob>& jobbuf, cudaStream_t s, const double* scale, uint64_t scale_len) {
     if (jobs.empty()) return;
+    uint32_t cols = 0;
     for (const CopyJob& j : jobs) {
         check_extent(j.src_off, j.rows, j.cols, j.src_ld, src_len, "copy source");
         if (j.trans) check_extent(j.dst_off, j.cols, j.rows, j.dst_ld, dst_len, "copy destination");
         else check_extent(j.dst_off, j.rows, j.cols, j.dst_ld, dst_len, "copy destination");
+        if (j.scaled && (!scale || j.s_off + j.cols > scale_len)) throw std::runtime_error("device work list out of bounds: copy factors");
+        if (j.rows) cols = std::max(cols, j.cols);
     }
-    uint64_t mx = 0;
-    for (auto& j : jobs) mx = std::max<uint64_t>(mx, uint64_t(j.rows) * j.cols);
-    if (mx == 0) return;
+    if (!cols) return;
+    if (cols > 65535u * CP_COLS) throw std::runtime_error("copy: too many columns");
     jobbuf.upload(jobs, s);
-    k_bcopy<<<unsigned(jobs.size()), 256, 0, s>>>(jobbuf.get(), unsigned(jobs.size()), src, dst);
+    k_bcopy<<<dim3(unsigned(jobs.size()), (cols + CP_COLS - 1) / CP_COLS), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
     QCM_CUDA(cudaGetLastError());
-    QCM_CUDA(cudaStreamSynchronize(s));
 }
 
 void dev_dots(const double* V, uint64_t ldv, uint32_t m, const double* w, uint64_t n, double* out, double* scratch,
@@ -259,18 +282,6 @@ void dev_axpy_dscalar(const double* a_dev, double sa, const double* x, double* y
 void dev_fill(double* p, uint64_t n, double v, cudaStream_t s) {
     if (!n) return;
     k_fill<<<grid_for(n), 256, 0, s>>>(p, n, v);
-    QCM_CUDA(cudaGetLastError());
-}
-
-void dev_scale_rows(double* A, uint32_t rows, uint32_t cols, uint32_t lda, const double* d, cudaStream_t s) {
-    if (!rows || !cols) return;
-    k_scale<<<grid_for(uint64_t(rows) * cols), 256, 0, s>>>(A, rows, cols, lda, d, 1);
-    QCM_CUDA(cudaGetLastError());
-}
-
-void dev_scale_cols(double* A, uint32_t rows, uint32_t cols, uint32_t lda, const double* d, cudaStream_t s) {
-    if (!rows || !cols) return;
-    k_scale<<<grid_for(uint64_t(rows) * cols), 256, 0, s>>>(A, rows, cols, lda, d, 0);
     QCM_CUDA(cudaGetLastError());
 }
 

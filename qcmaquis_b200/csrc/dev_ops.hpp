@@ -28,10 +28,13 @@ struct GemmJob {
 
 // dst[dst_off + i + j*dst_ld] = src[src_off + i + j*src_ld] (i < rows, j < cols);
 // with trans: dst[dst_off + j + i*dst_ld] = src[...] (transposed copy);
-// with rev: source column j is read from column cols - 1 - j (reversed column order)
+// with rev: source column j is read from column cols - 1 - j (reversed column order);
+// with scaled: the values of source column j times the launch's scale[s_off + j]
 struct CopyJob {
     uint64_t src_off, dst_off;
     uint32_t rows, cols, src_ld, dst_ld, trans, rev;
+    uint32_t scaled = 0;
+    uint64_t s_off = 0;
 };
 
 // Runs a list of GEMM jobs (all operands addressed from the three base pointers, whose
@@ -41,7 +44,7 @@ struct CopyJob {
 void batched_gemm(const std::vector<GemmJob>& jobs, const double* A, uint64_t a_len, const double* B, uint64_t b_len,
                   double* C, uint64_t c_len, DBuf<GemmJob>& jobbuf, DBuf<uint32_t>& tilebuf, cudaStream_t s);
 void batched_copy(const std::vector<CopyJob>& jobs, const double* src, uint64_t src_len, double* dst, uint64_t dst_len,
-                  DBuf<CopyJob>& jobbuf, cudaStream_t s);
+                  DBuf<CopyJob>& jobbuf, cudaStream_t s, const double* scale = nullptr, uint64_t scale_len = 0);
 // throws unless the rows x cols column-major sub-matrix at off (leading dimension ld) lies in [0, len)
 void check_extent(uint64_t off, uint64_t rows, uint64_t cols, uint64_t ld, uint64_t len, const char* what);
 
@@ -61,8 +64,5 @@ void dev_axpby(double a, const double* x, double b, double* y, uint64_t n, cudaS
 void dev_axpy_dscalar(const double* a_dev, double sa, const double* x, double* y, uint64_t n, cudaStream_t s);
 // p[i] = v
 void dev_fill(double* p, uint64_t n, double v, cudaStream_t s);
-// scale rows (row_scale) or columns of a column-major block: A(i,j) *= d[i] or d[j]
-void dev_scale_rows(double* A, uint32_t rows, uint32_t cols, uint32_t lda, const double* d, cudaStream_t s);
-void dev_scale_cols(double* A, uint32_t rows, uint32_t cols, uint32_t lda, const double* d, cudaStream_t s);
 
 }  // namespace qcm

@@ -610,19 +610,12 @@ TruncResults DTwoSite::split_from(Ctx& c, bool l2r, const BlockSVD& sv, std::siz
     std::size_t i = 0;
     for (std::size_t k = 0; k < nb; ++k) {
         if (!keep[k]) continue;
-        ju.push_back(CopyJob{uo[k], m1.b.off[i], both.rows[k], keep[k], both.rows[k], both.rows[k], 0, 0});
-        jv.push_back(CopyJob{vo[k], m2.b.off[i], both.cols[k], keep[k], both.cols[k], keep[k], 1, 0});
+        ju.push_back(CopyJob{uo[k], m1.b.off[i], both.rows[k], keep[k], both.rows[k], both.rows[k], 0, 0, !l2r, so[k]});
+        jv.push_back(CopyJob{vo[k], m2.b.off[i], both.cols[k], keep[k], both.cols[k], keep[k], 1, 0, l2r, so[k]});
         ++i;
     }
-    batched_copy(ju, U.get(), ul, m1.b.d.get(), m1.b.total, c.cjobs, c.s);
-    batched_copy(jv, V.get(), vl, m2.b.d.get(), m2.b.total, c.cjobs, c.s);
-    i = 0;
-    for (std::size_t k = 0; k < nb; ++k) {
-        if (!keep[k]) continue;
-        if (l2r) dev_scale_rows(m2.b.d.get() + m2.b.off[i], keep[k], both.cols[k], keep[k], S.get() + so[k], c.s);
-        else dev_scale_cols(m1.b.d.get() + m1.b.off[i], both.rows[k], keep[k], both.rows[k], S.get() + so[k], c.s);
-        ++i;
-    }
+    batched_copy(ju, U.get(), ul, m1.b.d.get(), m1.b.total, c.cjobs, c.s, S.get(), sv.s_len);
+    batched_copy(jv, V.get(), vl, m2.b.d.get(), m2.b.total, c.cjobs, c.s, S.get(), sv.s_len);
     QCM_CUDA(cudaStreamSynchronize(c.s));  // the decomposition's buffers may be released on return
     return tr;
 }
