@@ -33,31 +33,69 @@ namespace {
 constexpr int BJ_THR = 256;
 constexpr int BJ_MAXIT = 16;  // subspace slots of the batched solve
 
+constexpr int DOT_THR = 1024;  // threads of a dot's CTA
+constexpr int DOT_ILP = 4;     // entries of each operand in flight per thread
+
 __device__ double block_sum(double v, double* sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (lane == 0) sh[w] = v;
     __syncthreads();
     double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int i = 0; i < BJ_THR / 32; ++i) r += sh[i];
+    if (w == 0) {
+        r = lane < DOT_THR / 32 ? sh[lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
+    }
     __syncthreads();
     return r;  // valid in thread 0
 }
 
-// out[k * ns + i] = <A_k, B> over solve i's entries, k < nk (A_k = A + k * ld).  Grid (nk, ns).
-__global__ void __launch_bounds__(BJ_THR) k_bdots(const double* __restrict__ A, uint64_t ld, const double* __restrict__ B,
-                                                  const uint64_t* __restrict__ xo, const uint64_t* __restrict__ xn,
-                                                  int ns, double* __restrict__ out) {
-    __shared__ double sh[BJ_THR / 32];
+// f(j) for this thread's entries j < n, DOT_ILP of them in one unrolled body
+template <class F>
+__device__ __forceinline__ void for_entries(uint64_t n, F f) {
+    uint64_t j = threadIdx.x;
+    for (; j + (DOT_ILP - 1) * DOT_THR < n; j += DOT_ILP * DOT_THR)
+#pragma unroll
+        for (int u = 0; u < DOT_ILP; ++u) f(j + u * DOT_THR, u);
+    for (; j < n; j += DOT_THR) f(j, 0);
+}
+
+// out[k * ns + i] = <A_k, B> over solve i's entries, k < nk (A_k = A + k * ld).  Grid (nk, ns): one CTA per dot, so its
+// time is a thread's chain of loads: 1024 threads with four entries each in flight, and the three dots of the
+// residual in one launch (k_bdots3).  8 iterations of 16 solves (L=12, M=128): 16.93 ms with 256 threads and one entry
+// in flight, 16.60 ms so.
+__global__ void __launch_bounds__(DOT_THR) k_bdots(const double* __restrict__ A, uint64_t ld, const double* __restrict__ B,
+                                                   const uint64_t* __restrict__ xo, const uint64_t* __restrict__ xn,
+                                                   int ns, double* __restrict__ out) {
+    __shared__ double sh[DOT_THR / 32];
     const int k = blockIdx.x, i = blockIdx.y;
     const double* a = A + uint64_t(k) * ld + xo[i];
     const double* b = B + xo[i];
-    const uint64_t n = xn[i];
-    double v = 0.0;
-    for (uint64_t j = threadIdx.x; j < n; j += BJ_THR) v = fma(a[j], b[j], v);
-    v = block_sum(v, sh);
-    if (threadIdx.x == 0) out[uint64_t(k) * ns + i] = v;
+    double v[DOT_ILP] = {};
+    for_entries(xn[i], [&](uint64_t j, int u) { v[u] = fma(a[j], b[j], v[u]); });
+    const double d = block_sum((v[0] + v[1]) + (v[2] + v[3]), sh);
+    if (threadIdx.x == 0) out[uint64_t(k) * ns + i] = d;
+}
+
+// d3[i] = |R_i|^2, d3[ns + i] = <R_i, U_i>, d3[2 ns + i] = |U_i|^2.  Grid ns.
+__global__ void __launch_bounds__(DOT_THR) k_bdots3(const double* __restrict__ R, const double* __restrict__ U,
+                                                    const uint64_t* __restrict__ xo, const uint64_t* __restrict__ xn,
+                                                    int ns, double* __restrict__ d3) {
+    __shared__ double sh[DOT_THR / 32];
+    const int i = blockIdx.x;
+    const double* r = R + xo[i];
+    const double* u = U + xo[i];
+    double v[3][DOT_ILP] = {};
+    for_entries(xn[i], [&](uint64_t j, int c) {
+        const double rj = r[j], uj = u[j];
+        v[0][c] = fma(rj, rj, v[0][c]);
+        v[1][c] = fma(rj, uj, v[1][c]);
+        v[2][c] = fma(uj, uj, v[2][c]);
+    });
+    for (int m = 0; m < 3; ++m) {
+        const double d = block_sum((v[m][0] + v[m][1]) + (v[m][2] + v[m][3]), sh);
+        if (threadIdx.x == 0) d3[m * ns + i] = d;
+    }
 }
 
 // Y_i = beta * Y_i + sa * sum_{k < nk} c[k * ns + i] * A_k,i  (+ sg * g[i] * G_i if G).  Grid (chunks, ns).
@@ -245,21 +283,19 @@ void jacobi_davidson_batched(HeffPlan& g, const std::vector<uint64_t>& xo, const
         double* t = Vi(it);
         // classical Gram-Schmidt against V[0..it), twice
         for (int pass = 0; pass < (it > 0 ? 2 : 0); ++pass) {
-            k_bdots<<<dim3(unsigned(it), unsigned(ns)), BJ_THR, 0, s>>>(V, ld, t, dxo.get(), dxn.get(), ns, dots);
+            k_bdots<<<dim3(unsigned(it), unsigned(ns)), DOT_THR, 0, s>>>(V, ld, t, dxo.get(), dxn.get(), ns, dots);
             k_blincomb<<<eg, BJ_THR, 0, s>>>(V, ld, it, dots, ns, -1.0, 1.0, nullptr, nullptr, 0.0, t, dxo.get(),
                                              dxn.get());
         }
-        k_bdots<<<dim3(1, unsigned(ns)), BJ_THR, 0, s>>>(t, ld, t, dxo.get(), dxn.get(), ns, nrm2);
+        k_bdots<<<dim3(1, unsigned(ns)), DOT_THR, 0, s>>>(t, ld, t, dxo.get(), dxn.get(), ns, nrm2);
         k_bnormalise<<<eg, BJ_THR, 0, s>>>(t, nrm2, dxo.get(), dxn.get());
         heff_apply_device(g, t, VAi(it));
-        k_bdots<<<dim3(unsigned(it + 1), unsigned(ns)), BJ_THR, 0, s>>>(V, ld, VAi(it), dxo.get(), dxn.get(), ns, Mcol);
+        k_bdots<<<dim3(unsigned(it + 1), unsigned(ns)), DOT_THR, 0, s>>>(V, ld, VAi(it), dxo.get(), dxn.get(), ns, Mcol);
         k_brr<<<unsigned(ns), 32, 0, s>>>(ns, it, Mcol, Mp, theta, sv);
         // u = V s; r = VA s - theta u
         k_blincomb<<<eg, BJ_THR, 0, s>>>(V, ld, it + 1, sv, ns, 1.0, 0.0, nullptr, nullptr, 0.0, U, dxo.get(), dxn.get());
         k_blincomb<<<eg, BJ_THR, 0, s>>>(VA, ld, it + 1, sv, ns, 1.0, 0.0, U, theta, -1.0, R, dxo.get(), dxn.get());
-        k_bdots<<<dim3(1, unsigned(ns)), BJ_THR, 0, s>>>(R, ld, R, dxo.get(), dxn.get(), ns, d3);
-        k_bdots<<<dim3(1, unsigned(ns)), BJ_THR, 0, s>>>(R, ld, U, dxo.get(), dxn.get(), ns, d3 + nsu);
-        k_bdots<<<dim3(1, unsigned(ns)), BJ_THR, 0, s>>>(U, ld, U, dxo.get(), dxn.get(), ns, d3 + 2 * nsu);
+        k_bdots3<<<unsigned(ns), DOT_THR, 0, s>>>(R, U, dxo.get(), dxn.get(), ns, d3);
         QCM_CUDA(cudaMemsetAsync(active, 0, sizeof(int), s));
         k_bconv<<<sg, 128, 0, s>>>(ns, it, it == maxiter - 1, tol, d3, theta, state, devv, dit, cr, cu, keep, active);
         k_bkeep<<<eg, BJ_THR, 0, s>>>(U, X, keep, dxo.get(), dxn.get());
