@@ -11,7 +11,7 @@
 //               cohort is stored as its Hermitian partner)         (tasks.cpp:707-752)
 //   k_wgen    : W_u (lines x slices) = the unit's MPO coefficient terms summed into
 //               a dense block, once per plan, from the MPO, operator and boundary
-//               tables (one thread per line)
+//               tables (one thread per MPO entry of a line)
 //   k_sgemm   : S rows of a cohort unit = W_u * T slices.
 //               Replaces the alpha-weighted gather (gpu_dgemm_ddot.cu:282-359,
 //               tasks.cpp:466-494) by a tensor-core GEMM.
@@ -43,20 +43,21 @@ using namespace dm;
 //   k contiguous in memory: k fastest in shared memory (kfast), 16 bytes at a time if v16 (every k pair starts on
 //     16 bytes and nk is even), else 8;
 //   x contiguous: rows of X + PAD elements per k, 16 bytes at a time if v16 (nx even), else 8.
-template <int X, class Get>
+// UNROLL copies in one loop body.
+template <int X, int UNROLL, class Get>
 __device__ __forceinline__ void stage_kfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
     const int tid = threadIdx.x;
     if (v16) {
         constexpr int CH = X * BK / 2;
         static_assert(CH % NTHR == 0, "whole chunks per thread");
-#pragma unroll
+#pragma unroll UNROLL
         for (int rr = 0; rr < CH / NTHR; ++rr) {
             const int e = tid + rr * NTHR, k = 2 * (e % (BK / 2)), x = e / (BK / 2);
             const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
             cp16(dst + kfast(x, k), ok ? get(x, k) : any, ok);
         }
     } else {
-#pragma unroll
+#pragma unroll UNROLL
         for (int rr = 0; rr < X * BK / NTHR; ++rr) {
             const int e = tid + rr * NTHR, k = e % BK, x = e / BK;
             const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
@@ -64,19 +65,19 @@ __device__ __forceinline__ void stage_kfast(double* dst, const double* any, uint
         }
     }
 }
-template <int X, class Get>
+template <int X, int UNROLL, class Get>
 __device__ __forceinline__ void stage_xfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
     const int tid = threadIdx.x;
     if (v16) {
         constexpr int CH = X * BK / 2;
-#pragma unroll
+#pragma unroll UNROLL
         for (int rr = 0; rr < CH / NTHR; ++rr) {
             const int e = tid + rr * NTHR, x = 2 * (e % (X / 2)), k = e / (X / 2);
             const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
             cp16(dst + k * (X + PAD) + x, ok ? get(x, k) : any, ok);
         }
     } else {
-#pragma unroll
+#pragma unroll UNROLL
         for (int rr = 0; rr < X * BK / NTHR; ++rr) {
             const int e = tid + rr * NTHR, x = e % X, k = e / X;
             const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
@@ -116,8 +117,14 @@ constexpr std::size_t stage_bytes() {
 }
 
 // ---------------------------------------------------------------------------
-// T-GEMM: one CTA per (job, tile)
-template <class S>
+// T-GEMM: one CTA per (job, tile).  K is one ket sector, a few steps, and the three shapes' tiles run side by side: what
+// bounds it is how fast its code is fetched (two thirds of the stalled cycles of a small launch) and its operands
+// arrive, not the MMAs.  So the copies stand at one place of the loop for all steps, A's for both layouts of R, and
+// each form of T (OUT) has a kernel of its own: 0.757 -> 0.688 ms at L=24, M=512, 3.66 -> 3.34 ms at M=1024 (14.5 ->
+// 16.0 TFLOP/s), 0.124 -> 0.109 ms at L=16, M=256.  Runs of tiles per CTA, or both first stages issued before the
+// first wait, take more code and were slower (0.96 and 0.78 ms at M=512).
+enum class TOut { F64, F32, TF32_PAIR };  // T in FP64; in FP32; as a TF32 pair
+template <class S, TOut OUT>
 __device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, const TileD& tile, const TJobD* __restrict__ jobs,
                                            const double* __restrict__ x, const double* __restrict__ R, double* __restrict__ T,
                                            float* __restrict__ Thi, float* __restrict__ Tlo) {
@@ -131,39 +138,43 @@ __device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, cons
     const bool a16 = !((J.lda | nm) & 1u) && aligned16(xa);
     Acc<S> acc;
     acc.zero();
-    auto loop = [&](auto issue, auto tr) {
-        issue(st[0], 0);
-        for (uint32_t kc = 0; kc < nk; ++kc) {
-            cp_wait_all();
-            __syncthreads();
-            if (kc + 1 < nk) issue(st[(kc + 1) & 1], (kc + 1) * BK);
-            const Stage<S>& s = st[kc & 1];
-            mma_stage_part<S, false, !decltype(tr)::value>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm,
-                                                           int(min(uint32_t(BK), J.K - kc * BK) + 3) / 4);
-        }
-    };
-    if (!J.tr) {
-        // R's columns are K contiguous elements each, one column after the other
-        const double* rb = R + J.b_off + uint64_t(tile.n0) * J.K;
-        const bool b16 = !(J.K & 1u) && aligned16(rb);
-        loop([&](Stage<S>& s, uint32_t k0) {
-            stage_xfast<S::BM>(&s.A[0][0], x, nm, J.K - k0, a16, [&](int m, int k) { return xa + m + uint64_t(k0 + k) * J.lda; });
-            stage_kfast<S::BN>(&s.B[0][0], R, nn, J.K - k0, b16, [&](int n, int k) { return rb + uint64_t(n) * J.K + k0 + k; });
-            cp_commit();
-        }, std::false_type{});
-    } else {
-        // each block transposed: column n of block b at b * K * brs + n % brs, k in steps of brs
+    // R's columns are K contiguous elements each, one column after the other; or (tr) each block is transposed: column
+    // n of block b at b * K * brs + n % brs, k in steps of brs
+    const bool tr = J.tr;
+    if (tr) {
         for (int c = tid; c < S::BN; c += NTHR) {
             const uint32_t n = tile.n0 + c, b = n / J.brs;
             colbase[c] = n < J.N ? J.b_off + uint64_t(b) * J.K * J.brs + (n - b * J.brs) : J.b_off;
         }
         __syncthreads();
-        loop([&](Stage<S>& s, uint32_t k0) {
-            stage_xfast<S::BM>(&s.A[0][0], x, nm, J.K - k0, a16, [&](int m, int k) { return xa + m + uint64_t(k0 + k) * J.lda; });
-            stage_xfast<S::BN>(&s.B[0][0], R, nn, J.K - k0, false,
-                               [&](int n, int k) { return R + colbase[n] + uint64_t(k0 + k) * J.brs; });
+    }
+    const double* rb = R + J.b_off + uint64_t(tile.n0) * J.K;
+    // pairs of k (tr: of columns of one block) start on 16 bytes
+    const bool b16 = !((tr ? J.brs : J.K) & 1u) && aligned16(tr ? R + J.b_off : rb);
+    // Turn kc multiplies step kc and, before, starts the copies of step kc + 1: one place in the code for the copies
+#pragma unroll 1
+    for (int kc = -1; kc < int(nk); ++kc) {
+        if (kc >= 0) {
+            cp_wait_all();
+            __syncthreads();
+        }
+        if (kc + 1 < int(nk)) {
+            Stage<S>& s = st[(kc + 1) & 1];
+            const uint32_t k0 = uint32_t(kc + 1) * BK;
+            stage_xfast<S::BM, 8>(&s.A[0][0], x, nm, J.K - k0, a16, [&](int m, int k) { return xa + m + uint64_t(k0 + k) * J.lda; });
+            if (!tr)
+                stage_kfast<S::BN, 16>(&s.B[0][0], R, nn, J.K - k0, b16, [&](int n, int k) { return rb + uint64_t(n) * J.K + k0 + k; });
+            else
+                stage_xfast<S::BN, 16>(&s.B[0][0], R, nn, J.K - k0, b16,
+                                   [&](int n, int k) { return R + colbase[n] + uint64_t(k0 + k) * J.brs; });
             cp_commit();
-        }, std::true_type{});
+        }
+        if (kc >= 0) {
+            const Stage<S>& s = st[kc & 1];
+            const int ng = int(min(uint32_t(BK), J.K - kc * BK) + 3) / 4;
+            if (!tr) mma_stage_part<S, false, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm, ng);
+            else mma_stage_part<S, false, false>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm, ng);
+        }
     }
     // the thread's output columns: FN fragments x 2 columns each; their T offsets once (slice
     // blk at blk * sst, column within it at (n % brs) * M)
@@ -191,9 +202,9 @@ __device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, cons
                 if (!cok[j][c]) continue;
                 const double v = acc.c[i][j][c];
                 const uint64_t o = cof[j][c] + gm;
-                if (Thi && !Tlo) {
+                if constexpr (OUT == TOut::F32) {
                     Thi[o] = float(v);  // mixed form: T in FP32, split by the S build
-                } else if (Thi) {
+                } else if constexpr (OUT == TOut::TF32_PAIR) {
                     // mixed form (tensor-memory path): T as TF32 hi + lo (round to nearest)
                     uint32_t h, l;
                     asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(h) : "f"(float(v)));
@@ -207,6 +218,7 @@ __device__ __forceinline__ void tgemm_tile(Stage<S>* st, uint64_t* colbase, cons
     }
 }
 
+template <TOut OUT>
 __global__ void __launch_bounds__(NTHR, 5) k_tgemm(TileSet<TileD> set, const TJobD* __restrict__ jobs,
                                                    const double* __restrict__ x, const double* __restrict__ R,
                                                    double* __restrict__ T, float* __restrict__ Thi, float* __restrict__ Tlo) {
@@ -215,9 +227,9 @@ __global__ void __launch_bounds__(NTHR, 5) k_tgemm(TileSet<TileD> set, const TJo
     grid_trigger();
     TileD tile;
     const int sh = set.find(blockIdx.x, tile);
-    if (sh == SHAPE_64) tgemm_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
-    else if (sh == SHAPE_32) tgemm_tile<Sh32>(reinterpret_cast<Stage<Sh32>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
-    else tgemm_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+    if (sh == SHAPE_64) tgemm_tile<Sh64, OUT>(reinterpret_cast<Stage<Sh64>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+    else if (sh == SHAPE_32) tgemm_tile<Sh32, OUT>(reinterpret_cast<Stage<Sh32>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
+    else tgemm_tile<Sh16, OUT>(reinterpret_cast<Stage<Sh16>*>(raw), colbase, tile, jobs, x, R, T, Thi, Tlo);
 }
 
 // ---------------------------------------------------------------------------
@@ -484,7 +496,9 @@ void CoefGen::check_generated(cudaStream_t s) {
 namespace {
 
 // ---------------------------------------------------------------------------
-// L.S GEMM, split-K: item = (output tile, segment, K range) -> partial tile P[item]
+// L.S GEMM, split-K: item = (output tile, segment, K range) -> partial tile P[item].  Its copies are a loop of two per
+// turn at one place for all steps (see k_tgemm): no register is spilled any more, 0.450 -> 0.441 ms at L=24, M=512,
+// 0.092 -> 0.083 ms at L=16, M=256.  Rows past the output's are not stored: k_lsreduce does not read them.
 template <class S>
 __device__ __forceinline__ void lspart_tile(Stage<S>* st, uint64_t (*kbase)[BK], const KItemD& it, const OTileD* __restrict__ otiles,
                                             const OutD* __restrict__ outs, const SegD* __restrict__ segs,
@@ -508,57 +522,51 @@ __device__ __forceinline__ void lspart_tile(Stage<S>* st, uint64_t (*kbase)[BK],
     Acc<S> acc;
     acc.zero();
     const uint32_t nk = (it.k1 - it.k0 + BK - 1) / BK;
-    auto stage_s = [&](Stage<S>& s, uint32_t k0) {
-        stage_kfast<S::BN>(&s.B[0][0], Sm, nn, it.k1 - k0, b16, [&](int n, int k) { return sb + uint64_t(n) * Kc + k0 + k; });
-        cp_commit();
-    };
-    auto mma = [&](uint32_t kc, auto tr) {
-        const Stage<S>& s = st[kc & 1];
-        mma_stage_part<S, decltype(tr)::value, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm,
-                                                     int(min(uint32_t(BK), it.k1 - it.k0 - kc * BK) + 3) / 4);
-    };
-    if (!sg.tr) {
-        auto issue = [&](Stage<S>& s, uint32_t k0) {
-            stage_xfast<S::BM>(&s.A[0][0], Lb, nm, it.k1 - k0, a16, [&](int m, int k) { return la + m + uint64_t(k0 + k) * M; });
-            stage_s(s, k0);
-        };
-        issue(st[0], it.k0);
-        for (uint32_t kc = 0; kc < nk; ++kc) {
-            cp_wait_all();
-            __syncthreads();
-            if (kc + 1 < nk) issue(st[(kc + 1) & 1], it.k0 + (kc + 1) * BK);
-            mma(kc, std::false_type{});
+    // L^T (tr): element (m, k) of block b = k / ls_in at b * blk + k % ls_in + m * ls_in.  The bases of a stage's 16
+    // k's are written two stages ahead, so that the loop's barrier publishes them before their stage is issued
+    const bool tr = sg.tr;
+    auto bases = [&](int sidx, uint32_t k0) {
+        if (tid < BK) {
+            const uint32_t kk = k0 + tid, b = kk / sg.ls_in;
+            kbase[sidx][tid] = kk < it.k1 ? sg.l_off + b * blk + (kk - b * sg.ls_in) : sg.l_off;
         }
-    } else {
-        // L^T: element (m, k) of block b = k / ls_in at b * blk + k % ls_in + m * ls_in.  The bases of a stage's 16
-        // k's are written two stages ahead, so that the loop's barrier publishes them before their stage is issued
-        auto bases = [&](int sidx, uint32_t k0) {
-            if (tid < BK) {
-                const uint32_t kk = k0 + tid, b = kk / sg.ls_in;
-                kbase[sidx][tid] = kk < it.k1 ? sg.l_off + b * blk + (kk - b * sg.ls_in) : sg.l_off;
-            }
-        };
-        auto issue = [&](int sidx, uint32_t k0) {
-            Stage<S>& s = st[sidx];
-            stage_kfast<S::BM>(&s.A[0][0], Lb, nm, it.k1 - k0, false,
-                               [&](int m, int k) { return Lb + kbase[sidx][k] + uint64_t(ot.m0 + m) * sg.ls_in; });
-            stage_s(s, k0);
-        };
+    };
+    if (tr) {
         bases(0, it.k0);
         bases(1, it.k0 + BK);
         __syncthreads();
-        issue(0, it.k0);
-        for (uint32_t kc = 0; kc < nk; ++kc) {
+    }
+#pragma unroll 1
+    for (int kc = -1; kc < int(nk); ++kc) {
+        if (kc >= 0) {
             cp_wait_all();
             __syncthreads();
-            if (kc + 1 < nk) issue((kc + 1) & 1, it.k0 + (kc + 1) * BK);
+        }
+        if (kc + 1 < int(nk)) {
+            const int sidx = (kc + 1) & 1;
+            Stage<S>& s = st[sidx];
+            const uint32_t k0 = it.k0 + uint32_t(kc + 1) * BK;
+            if (!tr)
+                stage_xfast<S::BM, 2>(&s.A[0][0], Lb, nm, it.k1 - k0, a16, [&](int m, int k) { return la + m + uint64_t(k0 + k) * M; });
+            else
+                stage_kfast<S::BM, 2>(&s.A[0][0], Lb, nm, it.k1 - k0, false,
+                                   [&](int m, int k) { return Lb + kbase[sidx][k] + uint64_t(ot.m0 + m) * sg.ls_in; });
+            stage_kfast<S::BN, 2>(&s.B[0][0], Sm, nn, it.k1 - k0, b16, [&](int n, int k) { return sb + uint64_t(n) * Kc + k0 + k; });
+            cp_commit();
+        }
+        if (kc >= 0) {
             // stage kc's bases were consumed when it was issued: the buffer takes stage kc + 2's
-            if (kc + 2 < nk) bases(kc & 1, it.k0 + (kc + 2) * BK);
-            mma(kc, std::true_type{});
+            if (tr && kc + 2 < int(nk)) bases(kc & 1, it.k0 + uint32_t(kc + 2) * BK);
+            const Stage<S>& s = st[kc & 1];
+            const int ng = int(min(uint32_t(BK), it.k1 - it.k0 - kc * BK) + 3) / 4;
+            if (!tr) mma_stage_part<S, false, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm, ng);
+            else mma_stage_part<S, true, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm, ng);
         }
     }
     double* Pt = P + uint64_t(it.slot) * S::BM * S::BN;
-    for_acc<S>(acc, warp, lane, [&](int m, int n, double v) { Pt[m + n * S::BM] = v; });
+    for_acc<S>(acc, warp, lane, [&](int m, int n, double v) {
+        if (uint32_t(m) < nm) Pt[m + n * S::BM] = v;
+    });
 }
 
 // what the L.S kernels need of each shape: its output tiles, and its partial tiles in P
@@ -610,7 +618,8 @@ __global__ void __launch_bounds__(256) k_lsreduce(TileSet<OTileD> set, OTileSet 
 void launch_t(HeffPlan& p, const double* x, double* Tb, cudaStream_t s, float* Thi = nullptr, float* Tlo = nullptr) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_ttiles, p.ttiles, n);
-    if (n) launch_dependent(k_tgemm, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, Thi, Tlo);
+    const auto kernel = Tlo ? k_tgemm<TOut::TF32_PAIR> : (Thi ? k_tgemm<TOut::F32> : k_tgemm<TOut::F64>);
+    if (n) launch_dependent(kernel, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, Thi, Tlo);
 }
 
 void launch_s(HeffPlan& p, const double* Tb, double* Sb, cudaStream_t s) {
@@ -626,7 +635,7 @@ void launch_s(HeffPlan& p, const double* Tb, double* Sb, cudaStream_t s) {
 void launch_t_chunk(HeffPlan& p, const HeffPlan::SChunk& c, const double* x, double* Tb, cudaStream_t s) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(p.d_ttiles, c.tt[0], c.tt[1], n);
-    if (n) launch_dependent(k_tgemm, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, nullptr, nullptr);
+    if (n) launch_dependent(k_tgemm<TOut::F64>, dim3(n), NTHR, s, set, p.d_tjobs.get(), x, p.r_data(), Tb, nullptr, nullptr);
 }
 
 // the S-GEMM tiles [a[sh], b[sh]), reading coefficient blocks that start at element w0
@@ -795,7 +804,7 @@ void run_tgemm(const TJobD* jobs, const DBuf<TileD>* dtiles, const std::vector<T
                const double* R, double* T, cudaStream_t s) {
     uint32_t n;
     const TileSet<TileD> set = tile_set(dtiles, htiles, n);
-    if (n) k_tgemm<<<n, NTHR, 0, s>>>(set, jobs, x, R, T, nullptr, nullptr);
+    if (n) k_tgemm<TOut::F64><<<n, NTHR, 0, s>>>(set, jobs, x, R, T, nullptr, nullptr);
     QCM_CUDA(cudaGetLastError());
 }
 
