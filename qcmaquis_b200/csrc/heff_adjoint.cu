@@ -8,9 +8,8 @@
 //   Wbar_u    = Sbar_u T_u^T per unit              (k_wbar, DMMA, in the coefficient-block layout),
 //   coeff_bar = sum over the terms of entry e of Wbar_u(line, slot) * o_val * b_cs * line_scale.
 // The last runs k_wgen's traversal backwards.  One thread per (line, entry of its MPO row) writes the
-// line's partial sum for the entry (k_wadj).  Then one thread per entry adds the partials of the lines of
-// its row in increasing line order (k_entry_sum).  There are no atomics, so the result does not
-// vary from run to run.
+// line's partial sum for the entry (k_wadj).  Then the partials of the lines of the entry's row are added in a
+// fixed order (k_entry_sum).  There are no atomics, so the result does not vary from run to run.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,13 +20,14 @@
 #include "dev_ops.hpp"
 #include "dmma.cuh"
 #include "heff.hpp"
+#include "tiles.cuh"
 #include "wgen.cuh"
 
 namespace qcm {
 
 struct HeffAdjointWork {
-    std::vector<TileD> tiles;  // k_wbar: (unit, first line, first slot) per 64 x 64 tile of Wbar
-    DBuf<TileD> d_tiles;
+    std::vector<TileD> tiles[N_SHAPES];  // k_wbar: (unit, first line, first slot) per tile of Wbar
+    DBuf<TileD> d_tiles[N_SHAPES];
     DBuf<double> d_Wb;          // Wbar, the coefficient-block layout (w_len doubles)
     DBuf<double> d_P;           // per line, one partial per entry of its MPO row
     DBuf<uint64_t> d_pofs;      // per line: offset of its partials in P
@@ -42,69 +42,69 @@ struct HeffAdjointWork {
 namespace {
 
 using namespace dm;
-using SW = Sh64;
 
-// Wbar_u(line, slot) = sum_e Sbar(S row block line_b1[line], element e) * T(slice of slot, e); one CTA
-// per 64 x 64 tile, K = the unit's elements.
-__global__ void __launch_bounds__(NTHR) k_wbar(const UnitD* __restrict__ units, const TileD* __restrict__ tiles,
-                                               const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
-                                               const double* __restrict__ Sb, const double* __restrict__ T,
-                                               double* __restrict__ Wb) {
-    __shared__ Stage<SW> st[2];
-    __shared__ uint64_t soff[SW::BN], lrow[SW::BM];
-    const TileD tile = tiles[blockIdx.x];
-    const UnitD U = units[tile.item];
+// Wbar_u(line, slot) = sum_e Sbar(S row block line_b1[line], element e) * T(slice of slot, e); one CTA per tile (shapes as
+// the T-GEMM's, by the unit's lines), K = the unit's elements.  Elements are contiguous in both operands: both are staged
+// with k fastest, 16 bytes at a time where the strides are even.  A thread copies the same k of every row, so an
+// element's place in its S row (a division) is found once per step.  0.64 ms with 64 x 64 tiles throughout, 8-byte
+// copies and a division per element; 0.52 ms so (L=16, M=256: 14 TFLOP/s, K of 91 elements a tile on average).
+template <class S>
+__device__ __forceinline__ void wbar_tile(Stage<S>* st, uint64_t* soff, uint64_t* lrow, const TileD& tile, const UnitD& U,
+                                          const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
+                                          const double* __restrict__ Sb, const double* __restrict__ T, double* __restrict__ Wb) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int c = tid; c < SW::BN; c += NTHR) {
-        const uint32_t n = tile.n0 + c;
-        soff[c] = n < U.nk ? slice_off[U.slice0 + n] : 0;
-    }
+    const uint32_t nm = min(uint32_t(S::BM), U.nl - tile.m0), nn = min(uint32_t(S::BN), U.nk - tile.n0);
+    for (uint32_t c = tid; c < nn; c += NTHR) soff[c] = slice_off[U.slice0 + tile.n0 + c];
     // S row block of each line of the tile (the rows k_sgemm writes for it)
-    for (int c = tid; c < SW::BM; c += NTHR) {
-        const uint32_t l = tile.m0 + c;
-        lrow[c] = l < U.nl ? U.s_off + uint64_t(line_b1[U.line0 + l]) * U.line_stride : 0;
-    }
+    for (uint32_t c = tid; c < nm; c += NTHR) lrow[c] = U.s_off + uint64_t(line_b1[U.line0 + tile.m0 + c]) * U.line_stride;
     __syncthreads();
-    auto issue = [&](int sidx, uint32_t k0) {
-        Stage<SW>& s = st[sidx];
-        // element-fastest thread order: consecutive threads read consecutive rows of a slice column
-#pragma unroll
-        for (int rr = 0; rr < SW::A_PER; ++rr) {
-            const int e = tid + rr * NTHR;
-            const int k = e % BK, m = e / BK;
-            const uint32_t gm = tile.m0 + m, ge = k0 + k;
-            const bool ok = gm < U.nl && ge < U.ne;
-            uint64_t a = 0;
-            if (ok) {
-                const uint32_t c = ge / U.erows, r = ge - c * U.erows;
-                a = lrow[m] + r + uint64_t(c) * U.col_stride;
-            }
-            cp8(&s.A[k][m], Sb + a, ok);
-        }
-#pragma unroll
-        for (int rr = 0; rr < SW::B_PER; ++rr) {
-            const int e = tid + rr * NTHR;
-            const int k = e % BK, n = e / BK;
-            const uint32_t gn = tile.n0 + n, ge = k0 + k;
-            const bool ok = gn < U.nk && ge < U.ne;
-            cp8(&s.B[k][n], ok ? T + soff[n] + ge : T, ok);
-        }
-        cp_commit();
-    };
-    Acc<SW> acc;
+    // slices start on 16 bytes; pairs of elements of an S row do if all its strides are even
+    const bool a16 = !((U.ne | U.erows | U.col_stride | U.line_stride | U.s_off) & 1u) && !(reinterpret_cast<uintptr_t>(Sb) & 15u);
+    const bool b16 = !(U.ne & 1u);
+    const uint32_t ka = a16 ? 2 * (tid % (BK / 2)) : tid % BK;  // this thread's k in stage_kfast
+    static_assert(NTHR % BK == 0, "the same k in every round");
+    const int nfm = int(nm + 7) / 8;
+    Acc<S> acc;
     acc.zero();
     const uint32_t nk = (U.ne + BK - 1) / BK;
-    if (nk) issue(0, 0);
-    for (uint32_t kc = 0; kc < nk; ++kc) {
-        cp_wait_all();
-        __syncthreads();
-        if (kc + 1 < nk) issue((kc + 1) & 1, (kc + 1) * BK);
-        mma_stage<SW>(st[kc & 1].A, st[kc & 1].B, acc, warp, lane);
+#pragma unroll 1
+    for (int kc = -1; kc < int(nk); ++kc) {
+        if (kc >= 0) {
+            cp_wait_all();
+            __syncthreads();
+        }
+        if (kc + 1 < int(nk)) {
+            Stage<S>& s = st[(kc + 1) & 1];
+            const uint32_t k0 = uint32_t(kc + 1) * BK, col = (k0 + ka) / U.erows;
+            const uint64_t at = (k0 + ka - col * U.erows) + uint64_t(col) * U.col_stride;
+            stage_kfast<S::BM, 4>(&s.A[0][0], Sb, nm, U.ne - k0, a16, [&](int m, int) { return Sb + lrow[m] + at; });
+            stage_kfast<S::BN, 4>(&s.B[0][0], T, nn, U.ne - k0, b16, [&](int n, int k) { return T + soff[n] + k0 + k; });
+            cp_commit();
+        }
+        if (kc >= 0) {
+            const Stage<S>& s = st[kc & 1];
+            mma_stage_part<S, true, true>(&s.A[0][0], &s.B[0][0], acc, warp, lane, nfm,
+                                          int(min(uint32_t(BK), U.ne - kc * BK) + 3) / 4);
+        }
     }
-    for_acc<SW>(acc, warp, lane, [&](int m, int n, double v) {
-        const uint32_t gm = tile.m0 + m, gn = tile.n0 + n;
-        if (gm < U.nl && gn < U.nk) Wb[U.w_off + gm + uint64_t(gn) * U.wld] = v;
+    for_acc<S>(acc, warp, lane, [&](int m, int n, double v) {
+        if (uint32_t(m) < nm && uint32_t(n) < nn) Wb[U.w_off + tile.m0 + m + uint64_t(tile.n0 + n) * U.wld] = v;
     });
+}
+
+__global__ void __launch_bounds__(NTHR, 4) k_wbar(TileSet<TileD> set, const UnitD* __restrict__ units,
+                                                  const uint32_t* __restrict__ line_b1, const uint64_t* __restrict__ slice_off,
+                                                  const double* __restrict__ Sb, const double* __restrict__ T,
+                                                  double* __restrict__ Wb) {
+    __shared__ __align__(16) unsigned char raw[2 * std::max({sizeof(Stage<Sh16>), sizeof(Stage<Sh32>), sizeof(Stage<Sh64>)})];
+    __shared__ uint64_t soff[Sh16::BN], lrow[Sh64::BM];
+    static_assert(Sh32::BN <= Sh16::BN && Sh64::BN <= Sh16::BN);
+    TileD tile;
+    const int sh = set.find(blockIdx.x, tile);
+    const UnitD U = units[tile.item];
+    if (sh == SHAPE_64) wbar_tile<Sh64>(reinterpret_cast<Stage<Sh64>*>(raw), soff, lrow, tile, U, line_b1, slice_off, Sb, T, Wb);
+    else if (sh == SHAPE_32) wbar_tile<Sh32>(reinterpret_cast<Stage<Sh32>*>(raw), soff, lrow, tile, U, line_b1, slice_off, Sb, T, Wb);
+    else wbar_tile<Sh16>(reinterpret_cast<Stage<Sh16>*>(raw), soff, lrow, tile, U, line_b1, slice_off, Sb, T, Wb);
 }
 
 // Per line: P[pofs[line] + (e - m_ptr[m])] = sum over the terms of entry e (row m of the line) of
@@ -137,26 +137,42 @@ __global__ void __launch_bounds__(wg::THR) k_wadj(WGenTab t, const double* __res
     });
 }
 
-// out[e] = sum over the lines of e's MPO row (increasing line order) of their partial for e
-__global__ void k_entry_sum(uint64_t n_terms, const uint32_t* __restrict__ e_row, const uint32_t* __restrict__ m_ptr,
-                            const uint32_t* __restrict__ rl_ptr, const uint32_t* __restrict__ rl_line,
-                            const uint64_t* __restrict__ pofs, const double* __restrict__ P, double* __restrict__ out) {
-    for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < n_terms; e += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t m = e_row[e];
-        const uint64_t j = e - m_ptr[m];
+// out[e] = sum over the lines of e's MPO row of their partial for e.  A CTA takes 32 entries (a lane each: neighbouring
+// entries of a row have neighbouring partials) and its 8 warps an eighth of the lines each, whose sums are added in
+// warp order: the order does not vary from run to run.  A row's lines are a chain of dependent reads, thousands for
+// some rows: with one thread per entry the longest took 127 us of the 1.9 ms at L=16, M=256.
+constexpr int ES_WARPS = 8;
+__global__ void __launch_bounds__(32 * ES_WARPS) k_entry_sum(uint64_t n_terms, const uint32_t* __restrict__ e_row,
+                                                             const uint32_t* __restrict__ m_ptr, const uint32_t* __restrict__ rl_ptr,
+                                                             const uint32_t* __restrict__ rl_line, const uint64_t* __restrict__ pofs,
+                                                             const double* __restrict__ P, double* __restrict__ out) {
+    __shared__ double part[ES_WARPS][32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (uint64_t e0 = uint64_t(blockIdx.x) * 32; e0 < n_terms; e0 += uint64_t(gridDim.x) * 32) {
+        const uint64_t e = e0 + lane;
         double s = 0.0;
-        uint32_t t = rl_ptr[m];
-        const uint32_t t1 = rl_ptr[m + 1];
-        // eight partials in flight (each is two dependent reads), added in line order
-        for (; t + 8 <= t1; t += 8) {
-            double v[8];
+        if (e < n_terms) {
+            const uint32_t m = e_row[e], r0 = rl_ptr[m], nl = rl_ptr[m + 1] - r0, share = (nl + ES_WARPS - 1) / ES_WARPS;
+            const uint64_t j = e - m_ptr[m];
+            uint32_t t = r0 + min(nl, w * share);
+            const uint32_t t1 = r0 + min(nl, (w + 1) * share);
+            // eight partials in flight (each is two dependent reads), added in line order
+            for (; t + 8 <= t1; t += 8) {
+                double v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = P[pofs[rl_line[t + i]] + j];
+                for (int i = 0; i < 8; ++i) v[i] = P[pofs[rl_line[t + i]] + j];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) s += v[i];
+                for (int i = 0; i < 8; ++i) s += v[i];
+            }
+            for (; t < t1; ++t) s += P[pofs[rl_line[t]] + j];
         }
-        for (; t < t1; ++t) s += P[pofs[rl_line[t]] + j];
-        out[e] = s;
+        part[w][lane] = s;
+        __syncthreads();
+        if (w == 0 && e < n_terms) {
+            for (int i = 1; i < ES_WARPS; ++i) s += part[i][lane];
+            out[e] = s;
+        }
+        __syncthreads();
     }
 }
 
@@ -183,8 +199,9 @@ HeffAdjointWork& adjoint_work(HeffPlan& p) {
             for (uint32_t k = 0; k < u.nk; ++k)
                 if (p.slice_off[u.slice0 + k] + u.ne > p.t_len) throw std::runtime_error("heff adjoint: slice outside T");
         }
-        for (uint32_t m0 = 0; m0 < u.nl; m0 += SW::BM)
-            for (uint32_t n0 = 0; n0 < u.nk; n0 += SW::BN) w->tiles.push_back(TileD{i, m0, n0, 0});
+        const int sh = shape_for_rows(u.nl);
+        for (uint32_t m0 = 0; m0 < u.nl; m0 += shape_bm(sh))
+            for (uint32_t n0 = 0; n0 < u.nk; n0 += shape_bn(sh)) w->tiles[sh].push_back(TileD{i, m0, n0, 0});
     }
     // partials: per line (global line order), one per entry of its MPO row
     const std::size_t nlines = cg.line_major.size();
@@ -228,7 +245,7 @@ HeffAdjointWork& adjoint_work(HeffPlan& p) {
             w->sjobs.push_back(j);
         }
     cudaStream_t s = p.stream;
-    w->d_tiles.upload(w->tiles, s);
+    for (int sh = 0; sh < N_SHAPES; ++sh) w->d_tiles[sh].upload(w->tiles[sh], s);
     w->d_Wb.alloc(p.w_len ? p.w_len : 1);
     w->d_P.alloc(w->p_len ? w->p_len : 1);
     w->d_pofs.upload(pofs, s);
@@ -256,9 +273,10 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
     heff_tgemm_device(p, x, T);
     if (!w.sjobs.empty())
         batched_gemm(w.sjobs, p.L->data.get(), p.L->data.size(), ybar, p.x_len, Sb, p.s_len, w.d_jobs, w.d_jtiles, s);
-    if (!w.tiles.empty())
-        k_wbar<<<unsigned(w.tiles.size()), NTHR, 0, s>>>(p.d_units.get(), w.d_tiles.get(), p.d_line_b1.get(),
-                                                         p.d_slice_off.get(), Sb, T, w.d_Wb.get());
+    uint32_t n_tiles;
+    const TileSet<TileD> tiles = tile_set(w.d_tiles, w.tiles, n_tiles);
+    if (n_tiles)
+        k_wbar<<<n_tiles, NTHR, 0, s>>>(tiles, p.d_units.get(), p.d_line_b1.get(), p.d_slice_off.get(), Sb, T, w.d_Wb.get());
     QCM_CUDA(cudaGetLastError());
     const CoefGen& cg = p.cg;
     QCM_CUDA(cudaMemsetAsync(w.d_err.get(), 0, sizeof(uint32_t), s));
@@ -266,8 +284,8 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
         k_wadj<<<cg.task_ptr.back(), wg::THR, 0, s>>>(cg.tables(), w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
                                                              w.d_err.get());
     QCM_CUDA(cudaGetLastError());
-    const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 255) / 256, 148 * 16));
-    k_entry_sum<<<grid, 256, 0, s>>>(w.n_terms, w.d_e_row.get(), cg.d_m_ptr.get(), w.d_rl_ptr.get(), w.d_rl_line.get(),
+    const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 31) / 32, 148 * 16));
+    k_entry_sum<<<grid, 32 * ES_WARPS, 0, s>>>(w.n_terms, w.d_e_row.get(), cg.d_m_ptr.get(), w.d_rl_ptr.get(), w.d_rl_line.get(),
                                      w.d_pofs.get(), w.d_P.get(), coeff_bar);
     QCM_CUDA(cudaGetLastError());
     uint32_t h = 0;

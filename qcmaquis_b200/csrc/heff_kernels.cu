@@ -37,54 +37,6 @@ namespace {
 
 using namespace dm;
 
-// ---------------------------------------------------------------------------
-// Staging of one operand of a stage (X x BK elements, X = BM or BN) in one of three ways.  get(x, k): pointer to
-// element (x, k); nx, nk: how many x and k of the stage exist (elements past them are zero).
-//   k contiguous in memory: k fastest in shared memory (kfast), 16 bytes at a time if v16 (every k pair starts on
-//     16 bytes and nk is even), else 8;
-//   x contiguous: rows of X + PAD elements per k, 16 bytes at a time if v16 (nx even), else 8.
-// UNROLL copies in one loop body.
-template <int X, int UNROLL, class Get>
-__device__ __forceinline__ void stage_kfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
-    const int tid = threadIdx.x;
-    if (v16) {
-        constexpr int CH = X * BK / 2;
-        static_assert(CH % NTHR == 0, "whole chunks per thread");
-#pragma unroll UNROLL
-        for (int rr = 0; rr < CH / NTHR; ++rr) {
-            const int e = tid + rr * NTHR, k = 2 * (e % (BK / 2)), x = e / (BK / 2);
-            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
-            cp16(dst + kfast(x, k), ok ? get(x, k) : any, ok);
-        }
-    } else {
-#pragma unroll UNROLL
-        for (int rr = 0; rr < X * BK / NTHR; ++rr) {
-            const int e = tid + rr * NTHR, k = e % BK, x = e / BK;
-            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
-            cp8(dst + kfast(x, k), ok ? get(x, k) : any, ok);
-        }
-    }
-}
-template <int X, int UNROLL, class Get>
-__device__ __forceinline__ void stage_xfast(double* dst, const double* any, uint32_t nx, uint32_t nk, bool v16, Get get) {
-    const int tid = threadIdx.x;
-    if (v16) {
-        constexpr int CH = X * BK / 2;
-#pragma unroll UNROLL
-        for (int rr = 0; rr < CH / NTHR; ++rr) {
-            const int e = tid + rr * NTHR, x = 2 * (e % (X / 2)), k = e / (X / 2);
-            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
-            cp16(dst + k * (X + PAD) + x, ok ? get(x, k) : any, ok);
-        }
-    } else {
-#pragma unroll UNROLL
-        for (int rr = 0; rr < X * BK / NTHR; ++rr) {
-            const int e = tid + rr * NTHR, x = e % X, k = e / X;
-            const bool ok = uint32_t(x) < nx && uint32_t(k) < nk;
-            cp8(dst + k * (X + PAD) + x, ok ? get(x, k) : any, ok);
-        }
-    }
-}
 // An apply's kernels are launched as programmatic dependents of one another: each lets the next one start once
 // all its own CTAs run (grid_trigger), so that the next kernel's CTAs load their descriptors into the slots that
 // the last wave leaves empty, and waits (grid_wait) for the one before it to be complete before it touches anything

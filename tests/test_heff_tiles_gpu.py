@@ -1,13 +1,13 @@
 """H_eff . psi where sector sizes lie around the edges of the kernels' tiles and copies (fragments of 8 rows, K steps
-of 16, tiles of 16, 32 and 64 rows and 64 or 128 columns; 16-byte copies for even sizes only), and lockstep solves of
-vectors of unlike lengths."""
+of 16, tiles of 16, 32 and 64 rows and 64 or 128 columns; 16-byte copies for even sizes only), its adjoint over
+the same, and lockstep solves of vectors of unlike lengths."""
 import os
 import sys
 
 import numpy as np
 import pytest
 
-from oracle.oracle import heff_apply, site_problem
+from oracle.oracle import heff_adjoint, heff_apply, site_problem
 from qcmaquis_b200 import heff
 
 from helpers import qc_system
@@ -48,6 +48,19 @@ def test_apply_at_tile_edges(gpu_ctx, kind):
     assert np.abs(plan.apply(x) - ref).max() <= 1e-12 * scale  # the bound of every FP64 apply against the oracle
     for form in ("mixed", "mixed_tc"):
         assert np.abs(plan.apply(x, precision=form) - ref).max() <= 2e-6 * scale  # likewise (3xTF32 products, FP32 sums)
+
+
+@pytest.mark.parametrize("kind", ["fragments", "steps", "small tiles", "large tiles", "even"])
+def test_adjoint_at_tile_edges(gpu_ctx, kind):
+    ts = qc_system(L)[4]
+    snap, p = problem(SIZES[kind], 7)
+    plan = heff.plan_from_problem(gpu_ctx, p, ts, SITE)
+    x, ybar = np.random.default_rng(4).standard_normal((2, plan.n))
+    pb, g = plan.adjoint(x, ybar)
+    pb_ref, g_ref = heff_adjoint(snap, ts.blob(), SITE, x, ybar, g.size)
+    # the bounds of every adjoint against the oracle
+    assert np.abs(pb - pb_ref).max() <= 1e-12 * np.abs(pb_ref).max()
+    assert np.abs(g - g_ref).max() <= 1e-11 * np.abs(g_ref).max()
 
 
 def test_lockstep_solves_of_unlike_lengths(gpu_ctx):
