@@ -15,8 +15,9 @@
 // through shared memory (dot product, two rotations), which binds one SM at 128 B per clock, and rows are
 // what can be split without moving columns between SMs.  Each round every CTA sends its partial dot products
 // to all of them (distributed shared memory), and after one cluster barrier each CTA adds the partials in rank
-// order and derives the same rotations, one thread per pair.  A second cluster barrier per round (the partials
-// may be overwritten) is split: it is arrived at before the rotations and waited for after them.
+// order and derives the same rotations, one thread per pair.  The partials have two buffers, used in turn, so that a round
+// has one barrier; where G leaves room for one only, a second barrier (the partials may be overwritten) is split: it is
+// arrived at before the rotations and waited for after them.
 //
 // The largest blocks (more than about 420 columns on 16 CTAs) leave no shared memory for Q, and rotating it in L2
 // took three quarters of their time.  Nothing in the iteration reads Q, and its rows take the same rotations
