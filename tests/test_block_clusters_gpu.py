@@ -8,12 +8,12 @@ from qcmaquis_b200 import dmrg, heff
 pytestmark = pytest.mark.gpu
 EPS = np.finfo(float).eps
 
-# (rows, cols): around 48 columns (one CTA), 36 rows per CTA (2, 4, 8, 16 CTAs), the shared-memory limits of G and
-# Q at 16 CTAs (about 420 and 660 columns), and beyond them
-SVD_SHAPES = [(1, 1), (2, 1), (3, 3), (47, 48), (48, 49), (49, 49), (72, 73), (73, 75), (144, 145), (145, 149),
+# (rows, cols): around 48 and 88 columns (one CTA), 36 rows per CTA (2, 4, 8, 16 CTAs), the limits at 16 CTAs above which
+# Q comes from the rotation log (about 420 columns) and G leaves shared memory (about 660), and beyond them
+SVD_SHAPES = [(1, 1), (2, 1), (3, 3), (47, 48), (48, 49), (49, 49), (72, 73), (73, 75), (87, 88), (90, 89), (144, 145), (145, 149),
               (289, 291), (431, 437), (701, 699)]
-# around the elements per block at which the QR splits (64, 128, 256, 512 squared), flat and tall blocks
-QR_SHAPES = [(1, 1), (1, 7), (7, 1), (63, 65), (65, 65), (129, 127), (131, 131), (257, 256), (261, 263), (519, 517),
+# around the elements per block at which the QR splits (112, 128, 256, 512 squared), flat and tall blocks
+QR_SHAPES = [(1, 1), (1, 7), (7, 1), (63, 65), (65, 65), (112, 112), (113, 112), (129, 127), (131, 131), (257, 256), (261, 263), (519, 517),
              (30, 900), (900, 30), (700, 701)]
 
 
