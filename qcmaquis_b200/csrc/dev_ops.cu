@@ -246,9 +246,8 @@ void batched_copy(const std::vector<CopyJob>& jobs, const double* src, uint64_t 
         if (j.rows) cols = std::max(cols, j.cols);
     }
     if (!cols) return;
-    if (cols > 65535u * CP_COLS) throw std::runtime_error("copy: too many columns");
     jobbuf.upload(jobs, s);
-    k_bcopy<<<dim3(unsigned(jobs.size()), (cols + CP_COLS - 1) / CP_COLS), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
+    k_bcopy<<<dim3(unsigned(jobs.size()), std::min((cols - 1) / CP_COLS + 1, 65535u)), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
     QCM_CUDA(cudaGetLastError());
 }
 

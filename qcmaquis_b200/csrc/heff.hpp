@@ -7,11 +7,11 @@
 // L[ci_eff] * S (contract, :286-313), with the output accumulated under a
 // mutex (CPU) or with atomics (GPU).
 //
-// B200 form: the whole H.psi is three launches over flat work lists --
+// B200 form: the whole H.psi is four launches over flat work lists --
 //   (1) one grouped FP64 GEMM over every T job of every sector,
-//   (2) one gather launch building every cohort's S (HBM-bound),
-//   (3) one grouped FP64 GEMM per output tile whose K loop runs over all
-//       cohorts writing that output block (deterministic, no atomics).
+//   (2) one grouped FP64 GEMM building every cohort's S from dense coefficient blocks,
+//   (3) one grouped split-K FP64 GEMM of L and S over all cohorts of every output block,
+//   (4) the sum of its partial tiles in a fixed order (deterministic, no atomics).
 #pragma once
 
 #include <cuda_runtime.h>
