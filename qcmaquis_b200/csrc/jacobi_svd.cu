@@ -212,7 +212,6 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
             const uint32_t col = i / hq, k = i - col * hq;
             Q[col * ldq + k] = q0 + k == col ? 1.0 : 0.0;
         }
-    __syncthreads();
     const double tol2 = (JEPS * double(r)) * (JEPS * double(r));
     auto cluster_sync = [&] {
         if (nc > 1) {
@@ -222,6 +221,7 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
             __syncthreads();
         }
     };
+    cluster_sync();  // every CTA of the cluster runs: from here on the others may store into its shared memory
     // An exchange: every CTA's partial of item t goes to its row of the buffer in all CTAs (put, by the group's lanes);
     // after the barrier (arrived) gather adds them in rank order.  With one buffer it may be filled again once all CTAs
     // have gathered: they arrive at a second barrier then (gathered), waited for before the next put (free).
