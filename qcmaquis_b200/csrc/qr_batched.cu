@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
     }
     for (uint32_t c = tid; c < nn; c += nthr) perm[c] = c;
     for (uint32_t c = tid; c < ncl; c += nthr) lpos[c] = rank + c * nc;
-    __syncthreads();
+    cluster_sync();  // every CTA of the cluster runs: from here on the others may store into its shared memory
     // candidate of this CTA for step `step`, sent to every CTA: `best` of the calling warp's columns
     auto send_candidate = [&](QrCand best, uint32_t step) {
         if (lane == 0) wbest[warp] = best;

@@ -7,7 +7,7 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "qcmaquis_b200", "csrc")
 # every source whose kernels address the shared memory of other CTAs of their cluster
-SOURCES = ["jacobi_svd.cu"]
+SOURCES = ["jacobi_svd.cu", "qr_batched.cu"]
 
 
 @pytest.mark.parametrize("name", SOURCES)
