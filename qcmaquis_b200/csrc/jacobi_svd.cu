@@ -544,6 +544,9 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
         QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(JSMEM_DOUBLES * sizeof(double))));
         QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
+    // attributes belong to the functions, for all contexts and host threads: the same values on every call
+    QCM_CUDA(cudaFuncSetAttribute(k_jacobi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(JMAX_COLS * ROWS_SLICE * sizeof(double))));
     if (used > 1 && !side) side = std::make_unique<SideStreams>();
     if (used > 1) side->fork(s);
     std::size_t first = 0;
@@ -580,7 +583,6 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
             // LOG_SWEEPS sweeps, then their rotations applied to Q, up to the limit of sweeps (launches after the last
             // block is done return at once)
             const std::size_t qb = std::size_t(log_cols) * ROWS_SLICE * sizeof(double);
-            err = cudaFuncSetAttribute(k_jacobi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(qb));
             const dim3 qg((log_cols + ROWS_SLICE - 1) / ROWS_SLICE, unsigned(cls[i].size()));
             auto* kernel = i == 0 ? k_jacobi_svd<J_LOGGED_L2> : k_jacobi_svd<J_LOGGED>;
             int* meta = metas.get() + (i == 0 ? 0 : 2 * cls[0].size());
