@@ -198,6 +198,11 @@ typedef struct {
 int qcm_ctx_create(int device, qcm_ctx** out);
 void qcm_ctx_destroy(qcm_ctx* ctx);
 int qcm_ctx_synchronize(qcm_ctx* ctx);
+/* CTAs per cluster that the context's block factorisations (truncation SVD, QR, LQ)
+ * may use: 1, 2, 4, 8 or 16, the default; never more than the device can schedule
+ * (one of few SMs, or a partition of one, may not have 16 side by side).  For runs
+ * created from the context afterwards too. */
+int qcm_ctx_limit_clusters(qcm_ctx* ctx, uint32_t ctas);
 
 /* Copy a boundary into HBM (resident).  Replaces storage::gpu::broadcast::fetch
  * of Boundary cohorts (utils/storage.h:441-519, 594-615). */

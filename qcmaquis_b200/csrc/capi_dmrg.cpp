@@ -279,6 +279,7 @@ int qcm_dmrg_create(qcm_ctx* ctx, const qcm_mpo* mpo, int nup, int ndown, const 
     qcm::AllocStream scope(ctx->stream);
     qcm::DMRGParams p;
     if (const char* err = to_params(*prm, p)) return qcm::fail(QCM_ERR_ARG, err);
+    p.max_cluster = ctx->max_cluster;
     qcm::MPO ts = qcm::make_twosite_mpo(m);
     auto d = std::make_unique<qcm_dmrg>();
     d->ctx = ctx;
@@ -306,6 +307,7 @@ int qcm_dmrg_create_from_mps_at(qcm_ctx* ctx, const qcm_mpo* mpo, const qcm_dmrg
     qcm::AllocStream scope(ctx->stream);
     qcm::DMRGParams p;
     if (const char* err = to_params(*prm, p)) return qcm::fail(QCM_ERR_ARG, err);
+    p.max_cluster = ctx->max_cluster;
     qcm::Ctx tmp;
     tmp.s = ctx->stream;
     std::vector<qcm::DMPS> ms;

@@ -56,6 +56,15 @@ void qcm_ctx_destroy(qcm_ctx* c) {
     delete c;
 }
 
+int qcm_ctx_limit_clusters(qcm_ctx* c, uint32_t ctas) {
+    QCM_TRY
+    if (!c) return qcm::fail(QCM_ERR_ARG, "qcm_ctx_limit_clusters: NULL context");
+    if (ctas < 1 || ctas > 16 || (ctas & (ctas - 1))) return qcm::fail(QCM_ERR_ARG, "qcm_ctx_limit_clusters: 1, 2, 4, 8 or 16 CTAs");
+    c->max_cluster = ctas;
+    return QCM_OK;
+    QCM_CATCH
+}
+
 int qcm_ctx_synchronize(qcm_ctx* c) {
     QCM_TRY
     QCM_CUDA(cudaStreamSynchronize(c->stream));

@@ -56,6 +56,7 @@ int qcm_truncate_svd(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* rows, cons
     qcm::Ctx c;
     c.s = ctx->stream;
     c.device = ctx->device;
+    c.max_cluster = ctx->max_cluster;
     qcm::DBlocks M = upload_blocks(c, n_blocks, rows, cols, blocks, true);  // the solver is made only if needed
     qcm::BlockSVD sv = qcm::svd_truncate(c, M, max_bond_dimension, cutoff);
     // U_k (rows x keep, ld rows), S_k (keep), Vt_k (keep x cols, ld keep) packed in block order: gathered and
@@ -94,6 +95,7 @@ int qcm_truncate_heev(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* dims, con
     qcm::Ctx c;
     c.s = ctx->stream;
     c.device = ctx->device;
+    c.max_cluster = ctx->max_cluster;
     qcm::DBlocks dm = upload_blocks(c, n_blocks, dims, dims, blocks, false);
     qcm::BlockHeev hv = qcm::heev_truncate(c, dm, max_bond_dimension, cutoff);
     // U_k = the kept eigenvectors in descending eigenvalue order (dim x keep, ld dim)
@@ -124,6 +126,7 @@ extern "C" int qcm_qr_blocks(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* ro
     qcm::Ctx c;
     c.s = ctx->stream;
     c.device = ctx->device;
+    c.max_cluster = ctx->max_cluster;
     qcm::DBlocks M = upload_blocks(c, n_blocks, rows, cols, blocks, true);
     // outputs packed like the inputs: per block Q (m x k or k x n) then R / L, k = min(m, n)
     std::vector<uint64_t> qo(n_blocks), ro(n_blocks);
@@ -139,7 +142,7 @@ extern "C" int qcm_qr_blocks(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* ro
         wl += (qcm::qr_scratch(uint32_t(m), uint32_t(n), lq != 0) + 31) / 32 * 32;
     }
     qcm::DBuf<double> dq(std::max<uint64_t>(ql, 1)), dr(std::max<uint64_t>(rl, 1)), dw(std::max<uint64_t>(wl, 1));
-    qcm::batched_qr(jobs, M.d.get(), M.total, dq.get(), ql, dr.get(), rl, dw.get(), wl ? wl : 1, c.qjobs, c.side, c.s);
+    qcm::batched_qr(jobs, M.d.get(), M.total, dq.get(), ql, dr.get(), rl, dw.get(), wl ? wl : 1, c.qjobs, c.side, c.s, c.max_cluster);
     download(c, dq.get(), Q, ql);
     download(c, dr.get(), R, rl);
     QCM_CUDA(cudaStreamSynchronize(c.s));

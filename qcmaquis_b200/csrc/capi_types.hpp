@@ -13,6 +13,7 @@ struct qcm_ctx {
     // device address of the allocation-free apply's fixed scratch array on this device, looked
     // up when the context is created (qcm_heff_apply_device_noalloc)
     double* noalloc_scratch = nullptr;
+    uint32_t max_cluster = 16;  // qcm_ctx_limit_clusters
 };
 
 namespace qcm {

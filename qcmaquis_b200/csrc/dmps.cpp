@@ -214,7 +214,7 @@ DBlocks normalize_left(Ctx& c, DMPS& t) {
         wl += (qr_scratch(t.b.rows[k], t.b.cols[k], false) + 31) / 32 * 32;
     }
     Ctx::ensure(c.qrw, std::max<uint64_t>(wl, 1));
-    batched_qr(jobs, t.b.d.get(), t.b.total, Q.d.get(), Q.total, R.d.get(), R.total, c.qrw.get(), c.qrw.size(), c.qjobs, c.side, c.s);
+    batched_qr(jobs, t.b.d.get(), t.b.total, Q.d.get(), Q.total, R.d.get(), R.total, c.qrw.get(), c.qrw.size(), c.qjobs, c.side, c.s, c.max_cluster);
     t.b = std::move(Q);
     t.right = t.b.right_basis();
     return R;
@@ -239,7 +239,7 @@ DBlocks normalize_right(Ctx& c, DMPS& t) {
         wl += (qr_scratch(t.b.rows[k], t.b.cols[k], true) + 31) / 32 * 32;
     }
     Ctx::ensure(c.qrw, std::max<uint64_t>(wl, 1));
-    batched_qr(jobs, t.b.d.get(), t.b.total, Q.d.get(), Q.total, Lm.d.get(), Lm.total, c.qrw.get(), c.qrw.size(), c.qjobs, c.side, c.s);
+    batched_qr(jobs, t.b.d.get(), t.b.total, Q.d.get(), Q.total, Lm.d.get(), Lm.total, c.qrw.get(), c.qrw.size(), c.qjobs, c.side, c.s, c.max_cluster);
     t.b = std::move(Q);
     t.left = t.b.left_basis();
     return Lm;
@@ -449,10 +449,10 @@ void preconditioned_svd(Ctx& c, const DBlocks& both, BlockSVD& r, int* zero_coun
     if (sweeps)
         for (auto& e : ev) QCM_CUDA(cudaEventCreate(&e));
     if (sweeps) QCM_CUDA(cudaEventRecord(ev[0], c.s));
-    batched_qr(qj, both.d.get(), both.total, Qb.get(), ql, Xb.get(), xl, Wq.get(), wq, c.qjobs, c.side, c.s, Pb.get(), pl);
+    batched_qr(qj, both.d.get(), both.total, Qb.get(), ql, Xb.get(), xl, Wq.get(), wq, c.qjobs, c.side, c.s, c.max_cluster, Pb.get(), pl);
     if (sweeps) QCM_CUDA(cudaEventRecord(ev[1], c.s));
     batched_jacobi_svd(sj, Xb.get(), xl, Uxb.get(), xl, r.S.get(), r.s_len, Vxb.get(), xl, Wjb.get(), wj, zero_count, c.sjobs,
-                       c.side, c.s, sweeps);
+                       c.side, c.s, c.max_cluster, sweeps);
     if (sweeps) QCM_CUDA(cudaEventRecord(ev[2], c.s));
     if (!gu.empty()) batched_gemm(gu, Qb.get(), ql, Vxb.get(), xl, r.U.get(), r.u_len, c.gjobs, c.gtiles, c.s);
     if (!gv.empty()) batched_gemm(gv, Qb.get(), ql, Vxb.get(), xl, r.V.get(), r.v_len, c.gjobs, c.gtiles, c.s);

@@ -100,6 +100,7 @@ struct SBuild {
 struct Ctx {
     cudaStream_t s = nullptr;
     int device = 0;
+    uint32_t max_cluster = 16;  // CTAs per cluster of the block factorisations, at most
     std::unique_ptr<Solver> sv;
     DBuf<double> T, S, W, work, tmp, jd, scal, coef;
     DBuf<GemmJob> gjobs;
@@ -305,6 +306,7 @@ struct DMRGParams {
     // optimization = singlesite (ss_optimize.hpp:59-186): 2L steps per sweep over sites 0 .. L-1, L-1 .. 0,
     // each solved with the single-site MPO tensor and grown with the alphas above (heev does not apply)
     bool single_site = false;
+    uint32_t max_cluster = 16;  // Ctx::max_cluster
 };
 
 struct DMRGStats {

@@ -83,12 +83,12 @@ __host__ __device__ inline JacobiLayout jacobi_layout(uint32_t r, uint32_t c, ui
 // 100 columns, 2 us at 500) is near its fixed part (barriers, square root chain); splitting further only adds
 // CTAs that wait: 36 rows 13.8 ms for the blocks of M=1200, 20 or 24 rows 14.9 ms.  Up to 88 columns one CTA, which has no
 // exchange and one barrier a round (clusters from 48 columns on made batches of small blocks 0.87 times as fast).
-inline uint32_t jacobi_cluster(uint32_t r, uint32_t c) {
+inline uint32_t jacobi_cluster(uint32_t r, uint32_t c, uint32_t most) {
     if (c <= 88) return 1;
     const uint32_t rows = std::max(r, c);
     uint32_t nc = 2;
     while (nc < JMAX_CLUSTER && rows > 36 * nc) nc *= 2;
-    return nc;
+    return std::min(nc, most);
 }
 
 constexpr int LOG_SWEEPS = 4;       // sweeps per launch of a logged block
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
                 double2* gp = reinterpret_cast<double2*>(G + p * ldg);
                 double2* gq = reinterpret_cast<double2*>(G + q * ldg);
                 const double ga = group_dot(gp, gq, hr / 2, hl, gs, act);
-                if (nc == 1) {
+                if (!logged && nc == 1) {
                     // a block of one CTA needs no exchange: each group rotates its pair at once, one barrier a round
                     const double al = act ? nrm[p] : 0.0, be = act ? nrm[q] : 0.0;
                     if (act && ga * ga > tol2 * (al * be)) {
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
                 if (pass == 0) free();
                 if (act) put(t, ga, hl, gs);
             }
-            if (nc == 1) {
+            if (!logged && nc == 1) {
                 __syncthreads();
                 continue;
             }
@@ -361,13 +361,13 @@ __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ 
         if (!done) {
             if (MODE == J_LOGGED)
                 for (uint32_t i = tid; i < ldg * c; i += nthr) scratch[i] = G[i];
-            if (nc > 1) free();
+            free();
             return;  // every CTA of the cluster has passed its last exchange
         }
     }
     // sigma_j = |G_j| and its rank in descending order (ties by index)
     column_norms();
-    if (nc > 1) free();
+    free();
     for (uint32_t j = tid; j < c; j += nthr) nrm[j] = sqrt(nrm[j]);
     __syncthreads();
     double* sv = S + J.s_off;
@@ -493,9 +493,25 @@ uint64_t jacobi_svd_scratch(uint32_t m, uint32_t n) {
 
 void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64_t a_len, double* U, uint64_t u_len, double* S,
                         uint64_t s_len, double* V, uint64_t v_len, double* W, uint64_t w_len, int* zero_count,
-                        DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, int* sweeps_used) {
+                        DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, uint32_t max_cluster,
+                        int* sweeps_used) {
+    // attributes belong to the functions, for all contexts and host threads: the same values on every call
+    for (auto* k : {k_jacobi_svd<J_SMEM>, k_jacobi_svd<J_LOGGED>, k_jacobi_svd<J_LOGGED_L2>}) {
+        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(JSMEM_DOUBLES * sizeof(double))));
+        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+    QCM_CUDA(cudaFuncSetAttribute(k_jacobi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(JMAX_COLS * ROWS_SLICE * sizeof(double))));
+    // the most CTAs that a block wants, and that a cluster can have here
+    uint32_t most = 1;
+    for (const SvdJob& j : jobs) {
+        const uint32_t c = std::min(j.m, j.n), nc = jacobi_cluster(std::max(j.m, j.n), c, JMAX_CLUSTER);
+        most = std::max(most, jacobi_layout(std::max(j.m, j.n), c, nc, JSMEM_DOUBLES).q_smem ? nc : JMAX_CLUSTER);
+    }
+    most = largest_cluster(reinterpret_cast<const void*>(&k_jacobi_svd<J_LOGGED>), JTHR, JSMEM_DOUBLES * sizeof(double),
+                           std::min(most, max_cluster));
     // one launch per cluster size, the largest first (they take longest), each on a stream of its own
-    constexpr int NCLS = 7;  // 16 logged (G in L2, in shared memory), then 16, 8, 4, 2, 1 CTAs per block
+    constexpr int NCLS = 7;  // the most, logged (G in L2, in shared memory), then 16, 8, 4, 2, 1 CTAs per block
     static_assert(JMAX_CLUSTER >> (NCLS - 3) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
     std::vector<SvdJob> cls[NCLS];
     uint64_t log_len = 0;
@@ -511,11 +527,11 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
             throw std::runtime_error("batched_jacobi_svd: block outside its buffers");
         if (j.w_off % 2) throw std::runtime_error("batched_jacobi_svd: scratch offset not 16-byte aligned");
         if (uint64_t(j.m) * j.n > 0x7fffffffu) throw std::runtime_error("batched_jacobi_svd: block too large");
-        const uint32_t nc = jacobi_cluster(std::max(j.m, j.n), uint32_t(k));
+        const uint32_t nc = jacobi_cluster(std::max(j.m, j.n), uint32_t(k), most);
         int i = 2;
         for (uint32_t x = JMAX_CLUSTER; x > nc; x /= 2) ++i;
         if (!jacobi_layout(std::max(j.m, j.n), uint32_t(k), nc, JSMEM_DOUBLES).q_smem) {
-            i = jacobi_layout(std::max(j.m, j.n), uint32_t(k), JMAX_CLUSTER, JSMEM_DOUBLES).g_smem ? 1 : 0;
+            i = jacobi_layout(std::max(j.m, j.n), uint32_t(k), most, JSMEM_DOUBLES).g_smem ? 1 : 0;
             log_cols = std::max(log_cols, uint32_t(k));
         }
         cls[i].push_back(j);
@@ -540,13 +556,6 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     }
     if (all.empty()) return;
     jobbuf.upload(all, s);
-    for (auto* k : {k_jacobi_svd<J_SMEM>, k_jacobi_svd<J_LOGGED>, k_jacobi_svd<J_LOGGED_L2>}) {
-        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(JSMEM_DOUBLES * sizeof(double))));
-        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    // attributes belong to the functions, for all contexts and host threads: the same values on every call
-    QCM_CUDA(cudaFuncSetAttribute(k_jacobi_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(JMAX_COLS * ROWS_SLICE * sizeof(double))));
     if (used > 1 && !side) side = std::make_unique<SideStreams>();
     if (used > 1) side->fork(s);
     std::size_t first = 0;
@@ -554,7 +563,7 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < NCLS && err == cudaSuccess; ++i) {
         if (cls[i].empty()) continue;
-        const uint32_t nc = i < 2 ? JMAX_CLUSTER : JMAX_CLUSTER >> (i - 2);
+        const uint32_t nc = i < 2 ? most : JMAX_CLUSTER >> (i - 2);
         // shared memory of the launch's largest block (everything that fits), threads by its pairs per round
         uint64_t sm = 0;
         uint32_t lanes = 0;

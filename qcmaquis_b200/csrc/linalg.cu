@@ -107,6 +107,25 @@ void svd_thin_lane(Solver& sv, int l, const double* A, int m, int n, double* U, 
                                  info, L.svdp));
 }
 
+uint32_t largest_cluster(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t want) {
+    for (uint32_t nc = want; nc > 1; nc /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(nc);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = bytes;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = nc;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) return nc;
+        cudaGetLastError();  // a size that the device does not know is an error
+    }
+    return 1;
+}
+
 void syevd_lane(Solver& sv, int l, double* A, int n, double* W, int* info) {
     if (n == 0) return;
     Solver::Lane& L = sv.lane[l];

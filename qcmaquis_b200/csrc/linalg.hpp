@@ -68,6 +68,11 @@ struct SideStreams {
     void join(cudaStream_t to);
 };
 
+// CTAs per cluster, at most `want` (a power of two, up to 16), that the device can schedule of a kernel with the given
+// threads and dynamic shared memory per CTA.  Clusters of 16, and on a partitioned device smaller ones too, need more SMs
+// side by side than it may have; a cluster of one always runs.
+uint32_t largest_cluster(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t want);
+
 // Thin SVDs of many blocks (one-sided Jacobi, a cluster of 1 to 16 CTAs per block; jacobi_svd.cu):
 // A_j (m x n, ld m) = U_j diag(S_j) V_j^T with U_j (m x k, ld m), S_j descending (k), V_j
 // (n x k, ld n), k = min(m, n) -- the layout of gesvdj with econ = 1.  A singular value that
@@ -86,10 +91,11 @@ uint64_t jacobi_svd_scratch(uint32_t m, uint32_t n);
 // Replaces heevd('V') of alps/matrix/algorithms.hpp:374-396 (which then reverses the order).
 void syevd_lane(Solver& sv, int l, double* A, int n, double* W, int* info);
 // A, U, S, V, W: base pointers of the offsets in jobs (host list, validated against the lengths); side: made on
-// the first call that launches more than one cluster size
+// the first call that launches more than one cluster size; max_cluster: CTAs per cluster at most (1, 2, 4, 8 or 16)
 void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64_t a_len, double* U, uint64_t u_len, double* S,
                         uint64_t s_len, double* V, uint64_t v_len, double* W, uint64_t w_len, int* zero_count,
-                        DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, int* sweeps_used = nullptr);
+                        DBuf<SvdJob>& jobbuf, std::unique_ptr<SideStreams>& side, cudaStream_t s, uint32_t max_cluster,
+                        int* sweeps_used = nullptr);
 // Thin QR / LQ of many blocks (Householder, a cluster of 1 to 16 CTAs per block; qr_batched.cu):
 //   lq = 0: A_j (m x n, ld m) = Q_j R_j, Q_j (m x k, ld m), R_j (k x n, ld k);
 //   lq = 1: A_j = L_j Q_j, L_j (m x k, ld m) at r_off, Q_j (k x n, ld k) at q_off;
@@ -115,7 +121,7 @@ struct QrJob {
 uint64_t qr_scratch(uint32_t m, uint32_t n, bool lq);
 void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len, double* Q, uint64_t q_len, double* R,
                 uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, std::unique_ptr<SideStreams>& side,
-                cudaStream_t s, uint32_t* P = nullptr, uint64_t p_len = 0);
+                cudaStream_t s, uint32_t max_cluster, uint32_t* P = nullptr, uint64_t p_len = 0);
 
 // Does a cyclic Jacobi diagonalisation end before sweep `sweep`?  off, tot: sums of squares of the off-diagonal and of
 // all elements; last: off before the previous sweep.  Sweeps converge quadratically down to rounding (off about

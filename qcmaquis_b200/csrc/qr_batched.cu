@@ -52,11 +52,11 @@ constexpr uint32_t QR_MAX_CLUSTER = 16;
 // barrier costs more than a CTA's, and up to about 112 columns of 112 rows one CTA is the faster (66 to 90 columns:
 // 0.37 ms against 0.62 ms).  The pivoted QRs of a two-site truncation at L=24: M=2048 70 ms with one CTA per block, 8.6 ms
 // so; M=512 1.54 and 1.04 ms.
-inline uint32_t qr_cluster(uint32_t mm, uint32_t nn) {
+inline uint32_t qr_cluster(uint32_t mm, uint32_t nn, uint32_t most) {
     const uint64_t e = uint64_t(mm) * nn;
     if (e <= 112 * 112) return 1;
     uint32_t nc = 1;
-    while (nc < QR_MAX_CLUSTER && nc * 2 <= nn && e > uint64_t(64 * 64) * nc * nc) nc *= 2;
+    while (nc < most && nc * 2 <= nn && e > uint64_t(64 * 64) * nc * nc) nc *= 2;
     return nc;
 }
 
@@ -344,21 +344,29 @@ void batched_permute_rows(const std::vector<PermJob>& jobs, const double* src, u
 }
 
 uint64_t qr_scratch(uint32_t m, uint32_t n, bool) {
-    // reflectors, and per CTA its fixed part and columns (both rounded up), as k_qr lays them out; F is A or A^T
+    // reflectors, and per CTA its fixed part and columns (both rounded up), as k_qr lays them out; F is A or A^T, and the
+    // cluster may have to be smaller than it would best be
     const uint64_t k = std::min(m, n);
     uint64_t d = 0;
     for (auto [mm, nn] : {std::pair<uint32_t, uint32_t>{m, n}, {n, m}}) {
-        const uint32_t nc = qr_cluster(mm, nn);
-        const QrLayout l = qr_layout(mm, nn, nc, 0);
-        d = std::max<uint64_t>(d, uint64_t(mm) * k + nc * (l.fixed + uint64_t(l.ncol) * mm));
+        for (uint32_t nc = qr_cluster(mm, nn, QR_MAX_CLUSTER); nc; nc /= 2) {
+            const QrLayout l = qr_layout(mm, nn, nc, 0);
+            d = std::max<uint64_t>(d, uint64_t(mm) * k + nc * (l.fixed + uint64_t(l.ncol) * mm));
+        }
     }
     return d;
 }
 
 void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len, double* Q, uint64_t q_len, double* R,
                 uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, std::unique_ptr<SideStreams>& side,
-                cudaStream_t s, uint32_t* P, uint64_t p_len) {
+                cudaStream_t s, uint32_t max_cluster, uint32_t* P, uint64_t p_len) {
     if (jobs.empty()) return;
+    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QR_SMEM_DOUBLES * sizeof(double))));
+    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // the most CTAs that a block wants, and that a cluster can have here
+    uint32_t most = 1;
+    for (const QrJob& j : jobs) most = std::max(most, j.lq ? qr_cluster(j.n, j.m, QR_MAX_CLUSTER) : qr_cluster(j.m, j.n, QR_MAX_CLUSTER));
+    most = largest_cluster(reinterpret_cast<const void*>(&k_qr), QR_THR, QR_SMEM_DOUBLES * sizeof(double), std::min(most, max_cluster));
     constexpr int NCLS = 5;  // 16, 8, 4, 2, 1 CTAs per block, a launch each
     static_assert(QR_MAX_CLUSTER >> (NCLS - 1) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
     std::vector<QrJob> cls[NCLS];
@@ -372,7 +380,7 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
         if ((j.flags & QR_PIVOT) && (!P || nn > QR_PIV_MAX || j.p_off + nn > p_len))
             throw std::runtime_error("batched QR: pivoting needs a permutation buffer and at most 1024 columns");
         int i = 0;
-        for (uint32_t x = QR_MAX_CLUSTER; x > qr_cluster(mm, nn); x /= 2) ++i;
+        for (uint32_t x = QR_MAX_CLUSTER; x > qr_cluster(mm, nn, most); x /= 2) ++i;
         cls[i].push_back(j);
     }
     std::vector<QrJob> all;
@@ -386,8 +394,6 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
         used += !v.empty();
     }
     jobbuf.upload(all, s);
-    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QR_SMEM_DOUBLES * sizeof(double))));
-    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (used > 1 && !side) side = std::make_unique<SideStreams>();
     if (used > 1) side->fork(s);
     std::size_t first = 0;

@@ -419,6 +419,7 @@ DevDMRG::DevDMRG(const std::vector<MPOTensor>& single, const std::vector<MPOTens
                  const DMRGParams& prm, cudaStream_t s)
     : mpo(single), ts_mpo(twosite), p(prm) {
     c.s = s;
+    c.max_cluster = p.max_cluster;
     QCM_CUDA(cudaGetDevice(&c.device));
     L = int(mpo.size());
     if (L < 2 || int(ts_mpo.size()) != L - 1) throw std::runtime_error("DMRG: need L >= 2 site tensors and L - 1 two-site tensors");
@@ -447,6 +448,7 @@ DevDMRG::DevDMRG(const std::vector<MPOTensor>& single, const std::vector<MPOTens
                  const DMRGParams& prm, cudaStream_t s, int initial_site)
     : mpo(single), ts_mpo(twosite), mps(std::move(sites)), p(prm) {
     c.s = s;
+    c.max_cluster = p.max_cluster;
     QCM_CUDA(cudaGetDevice(&c.device));
     L = int(mpo.size());
     if (L < 2 || int(ts_mpo.size()) != L - 1 || int(mps.size()) != L)

@@ -60,6 +60,7 @@ class BoundaryInfo(ctypes.Structure):
 _lib._sig("qcm_ctx_create", c_int, c_int, P(c_void_p))
 _lib._sig("qcm_ctx_destroy", None, c_void_p)
 _lib._sig("qcm_ctx_synchronize", c_int, c_void_p)
+_lib._sig("qcm_ctx_limit_clusters", c_int, c_void_p, c_uint32)
 _lib._sig("qcm_boundary_upload", c_int, c_void_p, P(BoundaryDesc), P(c_void_p))
 _lib._sig("qcm_boundary_index_create", c_int, P(BoundaryDesc), P(c_void_p))
 _lib._sig("qcm_boundary_free", None, c_void_p)
@@ -227,6 +228,10 @@ class Context:
 
     def synchronize(self):
         check(lib.qcm_ctx_synchronize(self.h), "qcm_ctx_synchronize")
+
+    def limit_clusters(self, ctas: int):
+        """CTAs per cluster that the block factorisations may use (1, 2, 4, 8 or 16)."""
+        check(lib.qcm_ctx_limit_clusters(self.h, ctas), "qcm_ctx_limit_clusters")
 
     def __del__(self):
         if getattr(self, "h", None) is not None and self.h.value:
