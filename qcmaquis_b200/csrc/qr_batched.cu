@@ -18,9 +18,10 @@
 // differently).
 // LQ is the QR of the transpose (the same reflectors as gelqf): L = R'^T, Q = Q'^T.
 //
-// A block is factorised by a cluster of 1 to 16 CTAs, its columns dealt out to them in turn.  A step reads and
-// writes the whole trailing matrix, so one SM's shared memory (or L2, for a block beyond it) binds a large block,
-// and the columns are what a step treats independently.  Per step one cluster barrier: each CTA has sent the best
+// An unpivoted block of one CTA's size is factorised by k_qr_one.  The others (k_qr) by a cluster of 1 to
+// 16 CTAs each, the columns dealt out to them in turn.  A step reads and writes the whole trailing matrix, so one SM's
+// shared memory (or L2, for a block beyond it) binds a large block, and the columns are what a step treats
+// independently.  Per step one cluster barrier: each CTA has sent the best
 // of its remaining columns as the next pivot (norm, position, leading element; computed while updating them), all
 // of them pick the same winner and read its column from the owner's shared memory.  A pivot column is never
 // written again in its owner's store (its diagonal and reflector are kept apart), so nobody waits for its readers.
@@ -117,7 +118,6 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
     __shared__ double red[QR_WARPS];
     __shared__ double fro[QR_MAX_CLUSTER];
     __shared__ double sh_tau, sh_scale;
-    __shared__ int sh_zero;
     cg::cluster_group cl = cg::this_cluster();
     const uint32_t nc = cl.num_blocks(), rank = cl.block_rank();
     const QrJob J = jobs[blockIdx.x / nc];
@@ -218,7 +218,6 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
                 }
                 sh_tau = tau;
                 sh_scale = scale;
-                sh_zero = zero;
                 taus[j] = tau;
                 diag[j] = zero ? 0.0 : beta;  // a negligible column: exactly zero in R, no reflector
                 const uint32_t other = perm[j];
@@ -318,6 +317,127 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
     }
 }
 
+// An unpivoted factorisation by one CTA: no pivot is looked for and nothing is exchanged, so a step is the norm of its
+// column, the reflector in place of it, and the trailing columns, one warp each.  Against k_qr with one CTA, which finds
+// the norms of all columns and keeps its reflectors in L2: 100 x 100 0.57 against 0.73 ms, 48 x 48 0.21 against 0.26 ms,
+// 20 x 400 0.25 against 0.39 ms (whole calls).  Pivoted blocks are the faster in k_qr.
+__global__ void __launch_bounds__(QR_THR) k_qr_one(const QrJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ Q,
+                                                   double* __restrict__ R, double* __restrict__ W, uint32_t smem_doubles) {
+    extern __shared__ double qsm[];
+    __shared__ double red[QR_WARPS];
+    __shared__ double sh_tau, sh_scale, sh_thr;
+    __shared__ int sh_zero;
+    const QrJob J = jobs[blockIdx.x];
+    const uint32_t nthr = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr / 32;
+    // the matrix factorised: F (mm x nn) = A_j, or A_j^T for an LQ
+    const uint32_t mm = J.lq ? J.n : J.m, nn = J.lq ? J.m : J.n, k = mm < nn ? mm : nn;
+    // F, then R above and the reflectors below the diagonal, with the k reflector scales after it: in shared memory
+    // if they fit the launch's, else in the block's scratch (L2-resident)
+    const uint64_t fsz = uint64_t(mm) * nn + k;
+    double* w = fsz <= smem_doubles ? qsm : W + J.w_off;
+    double* taus = w + uint64_t(mm) * nn;
+    const double* a = A + J.a_off;
+    double f = 0.0;
+    for (uint64_t e = tid; e < uint64_t(mm) * nn; e += nthr) {
+        const uint32_t i = uint32_t(e % mm), c = uint32_t(e / mm);
+        const double x = J.lq ? a[c + uint64_t(i) * J.m] : a[i + uint64_t(c) * J.m];
+        w[e] = x;
+        f = fma(x, x, f);
+    }
+    // sum over the CTA in thread 0; red is free again after the barrier that follows
+    auto cta_sum = [&](double v) {
+        v = warp_sum(v);
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        double t = 0.0;
+        if (tid == 0)
+            for (uint32_t q = 0; q < nwarp; ++q) t += red[q];
+        return t;
+    };
+    f = cta_sum(f);
+    if (tid == 0) sh_thr = 64.0 * 2.220446049250313e-16 * sqrt(f);  // negligible columns: 64 eps |A|_F
+    __syncthreads();
+    for (uint32_t j = 0; j < k; ++j) {
+        double* vj = w + uint64_t(j) * mm;
+        double s = 0.0;
+        for (uint32_t i = j + 1 + tid; i < mm; i += nthr) s = fma(vj[i], vj[i], s);
+        s = cta_sum(s);
+        if (tid == 0) {
+            const double alpha = vj[j], xnorm = sqrt(s), nrm = hypot(alpha, xnorm);
+            double tau = 0.0, scale = 1.0;
+            const int zero = nrm <= sh_thr;
+            if (!zero && xnorm != 0.0) {
+                const double beta = -copysign(nrm, alpha);
+                tau = (beta - alpha) / beta;
+                scale = 1.0 / (alpha - beta);
+                vj[j] = beta;
+            }
+            sh_tau = tau;
+            sh_scale = scale;
+            sh_zero = zero;
+            taus[j] = tau;
+        }
+        __syncthreads();
+        const double tau = sh_tau, scale = sh_scale;
+        if (sh_zero)  // a negligible column: exactly zero in R, no reflector
+            for (uint32_t i = j + tid; i < mm; i += nthr) vj[i] = 0.0;
+        if (tau != 0.0) {
+            for (uint32_t i = j + 1 + tid; i < mm; i += nthr) vj[i] *= scale;
+            __syncthreads();
+            // trailing columns, one warp each: F(j:mm, c) -= tau v (v^T F(j:mm, c)), v_j = 1
+            for (uint32_t c = j + 1 + warp; c < nn; c += nwarp) {
+                double* fc = w + uint64_t(c) * mm;
+                const double fj = fc[j];  // read by every lane before lane 0 writes it
+                double d = 0.0;
+                for (uint32_t i = j + 1 + lane; i < mm; i += 32) d = fma(vj[i], fc[i], d);
+                d = (warp_sum(d) + fj) * tau;
+                if (lane == 0) fc[j] = fj - d;
+                for (uint32_t i = j + 1 + lane; i < mm; i += 32) fc[i] = fma(-d, vj[i], fc[i]);
+            }
+        }
+        __syncthreads();
+    }
+    // R (k x nn, ld k) from the upper triangle; for an LQ, L = R'^T (m x k, ld m)
+    double* r = R + J.r_off;
+    for (uint64_t e = tid; e < uint64_t(k) * nn; e += nthr) {
+        const uint32_t i = uint32_t(e % k), c = uint32_t(e / k);
+        const double v = i <= c ? w[i + uint64_t(c) * mm] : 0.0;
+        if (J.lq) r[c + uint64_t(i) * J.m] = v;
+        else if (J.flags & QR_RT) r[c + uint64_t(i) * nn] = v;
+        else r[e] = v;
+    }
+    // Q' = H_0 ... H_{k-1} I(:, 0:k), the reflectors applied from the last to the first; an LQ's in the scratch first
+    double* qf = W + J.w_off + fsz;
+    double* qo = J.lq ? qf : Q + J.q_off;
+    for (uint64_t e = tid; e < uint64_t(mm) * k; e += nthr) {
+        const uint32_t i = uint32_t(e % mm), c = uint32_t(e / mm);
+        qo[e] = i == c ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    for (int jj = int(k) - 1; jj >= 0; --jj) {
+        const uint32_t j = uint32_t(jj);
+        const double tau = taus[j];
+        if (tau != 0.0) {
+            const double* vj = w + uint64_t(j) * mm;
+            for (uint32_t c = j + warp; c < k; c += nwarp) {
+                double* qc = qo + uint64_t(c) * mm;
+                const double qj = qc[j];
+                double d = 0.0;
+                for (uint32_t i = j + 1 + lane; i < mm; i += 32) d = fma(vj[i], qc[i], d);
+                d = (warp_sum(d) + qj) * tau;
+                if (lane == 0) qc[j] = qj - d;
+                for (uint32_t i = j + 1 + lane; i < mm; i += 32) qc[i] = fma(-d, vj[i], qc[i]);
+            }
+        }
+        __syncthreads();
+    }
+    if (J.lq)  // Q = Q'^T (k x n, ld k)
+        for (uint64_t e = tid; e < uint64_t(mm) * k; e += nthr) {
+            const uint32_t i = uint32_t(e % mm), c = uint32_t(e / mm);
+            Q[J.q_off + c + uint64_t(i) * k] = qf[e];
+        }
+}
+
 __global__ void k_permute_rows(const PermJob* __restrict__ jobs, const double* __restrict__ src, double* __restrict__ dst,
                                const uint32_t* __restrict__ perm) {
     const PermJob J = jobs[blockIdx.x];
@@ -345,7 +465,7 @@ void batched_permute_rows(const std::vector<PermJob>& jobs, const double* src, u
 
 uint64_t qr_scratch(uint32_t m, uint32_t n, bool) {
     // reflectors, and per CTA its fixed part and columns (both rounded up), as k_qr lays them out; F is A or A^T, and the
-    // cluster may have to be smaller than it would best be
+    // cluster may have to be smaller than it would best be.  k_qr_one's F, scales and Q' (mm nn + k + mm k) are less.
     const uint64_t k = std::min(m, n);
     uint64_t d = 0;
     for (auto [mm, nn] : {std::pair<uint32_t, uint32_t>{m, n}, {n, m}}) {
@@ -361,14 +481,18 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
                 uint64_t r_len, double* W, uint64_t w_len, DBuf<QrJob>& jobbuf, std::unique_ptr<SideStreams>& side,
                 cudaStream_t s, uint32_t max_cluster, uint32_t* P, uint64_t p_len) {
     if (jobs.empty()) return;
-    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QR_SMEM_DOUBLES * sizeof(double))));
-    QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // attributes belong to the functions, for all contexts and host threads: the same values on every call
+    for (const void* k : {reinterpret_cast<const void*>(&k_qr), reinterpret_cast<const void*>(&k_qr_one)})
+        QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QR_SMEM_DOUBLES * sizeof(double))));
     // the most CTAs that a block wants, and that a cluster can have here
     uint32_t most = 1;
     for (const QrJob& j : jobs) most = std::max(most, j.lq ? qr_cluster(j.n, j.m, QR_MAX_CLUSTER) : qr_cluster(j.m, j.n, QR_MAX_CLUSTER));
-    most = largest_cluster(reinterpret_cast<const void*>(&k_qr), QR_THR, QR_SMEM_DOUBLES * sizeof(double), std::min(most, max_cluster));
-    constexpr int NCLS = 5;  // 16, 8, 4, 2, 1 CTAs per block, a launch each
-    static_assert(QR_MAX_CLUSTER >> (NCLS - 1) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
+    if (most > 1) {
+        QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        most = largest_cluster(reinterpret_cast<const void*>(&k_qr), QR_THR, QR_SMEM_DOUBLES * sizeof(double), std::min(most, max_cluster));
+    }
+    constexpr int NCLS = 6;  // 16, 8, 4, 2, 1 CTAs per block, and one CTA unpivoted: a launch each
+    static_assert(QR_MAX_CLUSTER >> (NCLS - 2) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
     std::vector<QrJob> cls[NCLS];
     for (const QrJob& j : jobs) {
         const uint64_t k = std::min(j.m, j.n);
@@ -381,6 +505,7 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
             throw std::runtime_error("batched QR: pivoting needs a permutation buffer and at most 1024 columns");
         int i = 0;
         for (uint32_t x = QR_MAX_CLUSTER; x > qr_cluster(mm, nn, most); x /= 2) ++i;
+        if (i == NCLS - 2 && !(j.flags & QR_PIVOT)) ++i;
         cls[i].push_back(j);
     }
     std::vector<QrJob> all;
@@ -401,6 +526,20 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < NCLS && err == cudaSuccess; ++i) {
         if (cls[i].empty()) continue;
+        if (i == NCLS - 1) {
+            // shared memory of the largest work matrix that fits, a warp per column and a thread per row
+            uint64_t sm = 0, thr = 0;
+            for (const QrJob& j : cls[i]) {
+                const uint64_t e = uint64_t(j.m) * j.n + std::min(j.m, j.n);
+                if (e <= QR_SMEM_DOUBLES) sm = std::max(sm, e);
+                thr = std::max<uint64_t>(thr, std::max(32 * uint64_t(j.lq ? j.m : j.n), uint64_t(j.lq ? j.n : j.m)));
+            }
+            thr = std::min<uint64_t>(QR_THR, std::max<uint64_t>(128, (thr + 127) / 128 * 128));
+            k_qr_one<<<unsigned(cls[i].size()), unsigned(thr), std::size_t(sm) * sizeof(double), lane < 0 ? s : side->s[lane]>>>(
+                jobbuf.get() + first, A, Q, R, W, uint32_t(sm));
+            err = cudaGetLastError();
+            break;  // the last class
+        }
         const uint32_t nc = QR_MAX_CLUSTER >> i;
         uint64_t sm = 0;
         uint32_t cols = 0;
