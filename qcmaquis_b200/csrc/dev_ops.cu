@@ -86,11 +86,13 @@ __global__ void __launch_bounds__(NTHR) k_bgemm(const GemmJob* __restrict__ jobs
     }
 }
 
-// One CTA per (job, strip of 32 source columns): a warp per column, its rows over the lanes (no division per element);
+// One CTA per (job, 32 source columns, 128 rows): a warp per column, its rows over the lanes (no division per element);
 // a transposing copy passes 32 x 32 tiles through shared memory, so that both sides move whole lines.  Small copies in
 // one launch: launches, and waits after them, were the cost.  A truncation of the 75 two-site blocks at L=24, M=512 with
 // its results read back: 6.4 ms with a copy and a wait per block and result, 5.4 ms gathered and read in one copy each.
-constexpr int CP_COLS = 32;
+// The rows of a tall block are split because its tiles are a chain of reads and barriers: with whole columns per CTA the
+// results of a 5 x 2000 block took 0.05 ms longer.
+constexpr uint32_t CP_COLS = 32, CP_ROWS = 128;
 __global__ void __launch_bounds__(256) k_bcopy(const CopyJob* __restrict__ jobs, const double* __restrict__ src,
                                                double* __restrict__ dst, const double* __restrict__ scale) {
     __shared__ double tile[CP_COLS][33];
@@ -98,28 +100,31 @@ __global__ void __launch_bounds__(256) k_bcopy(const CopyJob* __restrict__ jobs,
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto column = [&](uint32_t j) { return src + J.src_off + uint64_t(J.rev ? J.cols - 1 - j : j) * J.src_ld; };
     auto factor = [&](uint32_t j) { return J.scaled ? scale[J.s_off + j] : 1.0; };
-    for (uint64_t strip = uint64_t(blockIdx.y) * CP_COLS; strip < J.cols; strip += uint64_t(gridDim.y) * CP_COLS) {
-        const uint32_t j0 = uint32_t(strip), j1 = uint32_t(min(uint64_t(J.cols), strip + CP_COLS));
+    const uint32_t nr = (J.rows + CP_ROWS - 1) / CP_ROWS;
+    const uint64_t n = uint64_t(nr) * ((J.cols + CP_COLS - 1) / CP_COLS);
+    for (uint64_t t = blockIdx.y; t < n; t += gridDim.y) {
+        const uint32_t j0 = uint32_t(t / nr) * CP_COLS, j1 = min(J.cols, j0 + CP_COLS);
+        const uint32_t r0 = uint32_t(t % nr) * CP_ROWS, r1 = min(J.rows, r0 + CP_ROWS);
         if (!J.trans) {
             for (uint32_t j = j0 + warp; j < j1; j += 8) {
                 const double* c = column(j);
                 double* d = dst + J.dst_off + uint64_t(j) * J.dst_ld;
                 if (J.scaled) {
                     const double f = factor(j);
-                    for (uint32_t i = lane; i < J.rows; i += 32) d[i] = c[i] * f;
+                    for (uint32_t i = r0 + lane; i < r1; i += 32) d[i] = c[i] * f;
                 } else {
-                    for (uint32_t i = lane; i < J.rows; i += 32) d[i] = c[i];
+                    for (uint32_t i = r0 + lane; i < r1; i += 32) d[i] = c[i];
                 }
             }
             continue;
         }
-        for (uint32_t i0 = 0; i0 < J.rows; i0 += 32) {
+        for (uint32_t i0 = r0; i0 < r1; i0 += 32) {
             for (uint32_t j = j0 + warp; j < j1; j += 8)
-                if (i0 + lane < J.rows) tile[j - j0][lane] = column(j)[i0 + lane];
+                if (i0 + lane < r1) tile[j - j0][lane] = column(j)[i0 + lane];
             __syncthreads();
             const uint32_t j = j0 + lane;
             if (j < j1)
-                for (uint32_t i = i0 + warp; i < min(J.rows, i0 + 32); i += 8) {
+                for (uint32_t i = i0 + warp; i < min(r1, i0 + 32); i += 8) {
                     const double v = tile[lane][i - i0];
                     dst[J.dst_off + j + uint64_t(i) * J.dst_ld] = J.scaled ? v * factor(j) : v;
                 }
@@ -238,16 +243,22 @@ void batched_copy(const std::vector<CopyJob>& jobs, const double* src, uint64_t 
                   DBuf<CopyJob>& jobbuf, cudaStream_t s, const double* scale, uint64_t scale_len) {
     if (jobs.empty()) return;
     uint32_t cols = 0;
+    uint64_t parts = 0;
     for (const CopyJob& j : jobs) {
         check_extent(j.src_off, j.rows, j.cols, j.src_ld, src_len, "copy source");
         if (j.trans) check_extent(j.dst_off, j.cols, j.rows, j.dst_ld, dst_len, "copy destination");
         else check_extent(j.dst_off, j.rows, j.cols, j.dst_ld, dst_len, "copy destination");
         if (j.scaled && (!scale || j.s_off + j.cols > scale_len)) throw std::runtime_error("device work list out of bounds: copy factors");
-        if (j.rows) cols = std::max(cols, j.cols);
+        if (!j.rows || !j.cols) continue;
+        cols = std::max(cols, j.cols);
+        parts = std::max(parts, uint64_t((j.rows - 1) / CP_ROWS + 1) * ((j.cols - 1) / CP_COLS + 1));
     }
     if (!cols) return;
+    // CTAs per job by the largest job's parts, but (the smaller jobs' have nothing to do) not beyond 64 per SM in all where
+    // a CTA per column strip is less
+    const uint64_t y = std::min(parts, std::max<uint64_t>((cols - 1) / CP_COLS + 1, 148 * 64 / jobs.size()));
     jobbuf.upload(jobs, s);
-    k_bcopy<<<dim3(unsigned(jobs.size()), std::min((cols - 1) / CP_COLS + 1, 65535u)), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
+    k_bcopy<<<dim3(unsigned(jobs.size()), unsigned(std::min<uint64_t>(y, 65535))), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
     QCM_CUDA(cudaGetLastError());
 }
 
