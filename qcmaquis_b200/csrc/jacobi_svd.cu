@@ -79,16 +79,35 @@ __host__ __device__ inline JacobiLayout jacobi_layout(uint32_t r, uint32_t c, ui
     }
 }
 
-// CTAs per block: about 36 rows of each column per CTA.  There a round's shared-memory time (under 1 us up to
+// CTAs per block, alone: about 36 rows of each column per CTA.  There a round's shared-memory time (under 1 us up to
 // 100 columns, 2 us at 500) is near its fixed part (barriers, square root chain); splitting further only adds
 // CTAs that wait: 36 rows 13.8 ms for the blocks of M=1200, 20 or 24 rows 14.9 ms.  Up to 88 columns one CTA, which has no
 // exchange and one barrier a round (clusters from 48 columns on made batches of small blocks 0.87 times as fast).
-inline uint32_t jacobi_cluster(uint32_t r, uint32_t c, uint32_t most) {
+inline uint32_t jacobi_cluster(uint32_t r, uint32_t c) {
     if (c <= 88) return 1;
     const uint32_t rows = std::max(r, c);
     uint32_t nc = 2;
     while (nc < JMAX_CLUSTER && rows > 36 * nc) nc *= 2;
-    return std::min(nc, most);
+    return nc;
+}
+// where a launch's blocks keep their work arrays (known at compile time: shared-memory addresses are a third of the
+// kernel's instructions): G and Q in one CTA's shared memory; in a cluster's; G there and Q logged; G in the scratch.
+// One CTA has an instance without the exchange: 88 x 88 block 2.51 -> 2.21 ms, 64 x 64 1.21 -> 1.07 ms.
+enum JacobiMode { J_ONE, J_SMEM, J_LOGGED, J_LOGGED_L2 };
+// the instance that a block needs in a cluster of nc CTAs
+inline JacobiMode jacobi_mode(uint32_t r, uint32_t c, uint32_t nc) {
+    const JacobiLayout l = jacobi_layout(r, c, nc, JSMEM_DOUBLES);
+    return l.q_smem ? (nc == 1 ? J_ONE : J_SMEM) : (l.g_smem ? J_LOGGED : J_LOGGED_L2);
+}
+// time of a sweep of a block in us: c' - 1 rounds of a fixed part (barriers, exchange, square root chain) and of the
+// columns' way through shared memory at 128 bytes a clock, dealt out to the CTAs; 2.4 times that for a G in L2; 1.5 us a
+// round for k_jacobi_rows (from single blocks of 64 to 512 columns, within a fifth)
+inline double jacobi_cost(uint32_t r, uint32_t c, int log2nc) {
+    constexpr double fixed[N_CLUSTER_SIZES] = {0.35, 1.2, 1.2, 1.3, 2.3};
+    const JacobiMode m = jacobi_mode(r, c, 1u << log2nc);
+    const double np = (c + 1) / 2, way = np / 30400.0 / (1 << log2nc);
+    const double logged = m == J_LOGGED || m == J_LOGGED_L2 ? 1.5 : 0.0;
+    return (2.0 * np - 1.0) * (fixed[log2nc] + logged + way * (logged > 0.0 ? 6.0 * r * (m == J_LOGGED_L2 ? 2.4 : 1.0) : 6.0 * r + 4.0 * c));
 }
 
 constexpr int LOG_SWEEPS = 4;       // sweeps per launch of a logged block
@@ -165,11 +184,6 @@ __device__ __forceinline__ double group_dot(const double2* x, const double2* y, 
         }
     return group_sum(a + b, gs);
 }
-
-// where a launch's blocks keep their work arrays (known at compile time: shared-memory addresses are a third of the
-// kernel's instructions): G and Q in one CTA's shared memory; in a cluster's; G there and Q logged; G in the scratch.
-// One CTA has an instance without the exchange: 88 x 88 block 2.51 -> 2.21 ms, 64 x 64 1.21 -> 1.07 ms.
-enum JacobiMode { J_ONE, J_SMEM, J_LOGGED, J_LOGGED_L2 };
 
 template <int MODE>
 __global__ void __launch_bounds__(JTHR) k_jacobi_svd(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
@@ -502,53 +516,57 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     };
     const std::size_t full = JSMEM_DOUBLES * sizeof(double);
     allow(reinterpret_cast<const void*>(&k_jacobi_svd<J_ONE>), full);
-    // the most CTAs that a block wants, and that a cluster can have here
-    uint32_t most = 1;
-    for (const SvdJob& j : jobs) {
-        const uint32_t c = std::min(j.m, j.n), nc = jacobi_cluster(std::max(j.m, j.n), c, JMAX_CLUSTER);
-        most = std::max(most, jacobi_layout(std::max(j.m, j.n), c, nc, JSMEM_DOUBLES).q_smem ? nc : JMAX_CLUSTER);
+    // cluster sizes: alone, or by the batch; blocks whose Q does not fit one want the most
+    std::vector<std::array<double, N_CLUSTER_SIZES>> cost(jobs.size());
+    std::vector<uint8_t> size(jobs.size(), 0);
+    bool split = false;
+    for (std::size_t b = 0; b < jobs.size(); ++b) {
+        const uint32_t r = std::max(jobs[b].m, jobs[b].n), c = std::min(jobs[b].m, jobs[b].n);
+        if (!c) continue;
+        if (c > JMAX_COLS) throw std::runtime_error("batched_jacobi_svd: block larger than 1024 in both dimensions");
+        if (uint64_t(r) * c > 0x7fffffffu) throw std::runtime_error("batched_jacobi_svd: block too large");
+        const uint32_t nc = jacobi_cluster(r, c), want = jacobi_mode(r, c, nc) >= J_LOGGED ? JMAX_CLUSTER : nc;
+        while ((2u << size[b]) <= want) ++size[b];
+        split = split || size[b];
+        for (int i = 0; i < N_CLUSTER_SIZES; ++i) cost[b][i] = jacobi_cost(r, c, i);
     }
-    if (most > 1) {
+    if (split) {
         for (const void* k : {reinterpret_cast<const void*>(&k_jacobi_svd<J_SMEM>), reinterpret_cast<const void*>(&k_jacobi_svd<J_LOGGED>),
                               reinterpret_cast<const void*>(&k_jacobi_svd<J_LOGGED_L2>)}) {
             allow(k, full);
             QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         }
         allow(reinterpret_cast<const void*>(&k_jacobi_rows), JMAX_COLS * ROWS_SLICE * sizeof(double));
-        most = largest_cluster(reinterpret_cast<const void*>(&k_jacobi_svd<J_LOGGED>), JTHR, full, std::min(most, max_cluster));
+        size = plan_clusters(cost, size, cluster_slots(reinterpret_cast<const void*>(&k_jacobi_svd<J_LOGGED>), JTHR, full, max_cluster));
     }
-    // one launch per cluster size, the largest first (they take longest), each on a stream of its own
-    constexpr int NCLS = 7;  // the most, logged (G in L2, in shared memory), then 16, 8, 4, 2, 1 CTAs per block
-    static_assert(JMAX_CLUSTER >> (NCLS - 3) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
+    // one launch per instance and cluster size, the largest clusters first, each on a stream of its own while they last
+    constexpr int NCLS = 4 * N_CLUSTER_SIZES;
+    auto cls_of = [](int log2nc, JacobiMode m) { return (N_CLUSTER_SIZES - 1 - log2nc) * 4 + (J_LOGGED_L2 - m); };
     std::vector<SvdJob> cls[NCLS];
     uint64_t log_len = 0;
-    uint32_t log_cols = 0;
+    uint32_t log_cols = 0, n_logged = 0;
     uint32_t nid = 0;
-    for (const SvdJob& j : jobs) {
+    for (std::size_t b = 0; b < jobs.size(); ++b) {
+        const SvdJob& j = jobs[b];
         nid = std::max(nid, j.id + 1);
         const uint64_t k = std::min(j.m, j.n);
         if (!j.m || !j.n) continue;
-        if (k > JMAX_COLS) throw std::runtime_error("batched_jacobi_svd: block larger than 1024 in both dimensions");
         if (j.a_off + uint64_t(j.m) * j.n > a_len || j.u_off + uint64_t(j.m) * k > u_len || j.s_off + k > s_len ||
             j.v_off + uint64_t(j.n) * k > v_len || j.w_off + jacobi_svd_scratch(j.m, j.n) > w_len)
             throw std::runtime_error("batched_jacobi_svd: block outside its buffers");
         if (j.w_off % 2) throw std::runtime_error("batched_jacobi_svd: scratch offset not 16-byte aligned");
-        if (uint64_t(j.m) * j.n > 0x7fffffffu) throw std::runtime_error("batched_jacobi_svd: block too large");
-        const uint32_t nc = jacobi_cluster(std::max(j.m, j.n), uint32_t(k), most);
-        int i = 2;
-        for (uint32_t x = JMAX_CLUSTER; x > nc; x /= 2) ++i;
-        if (!jacobi_layout(std::max(j.m, j.n), uint32_t(k), nc, JSMEM_DOUBLES).q_smem) {
-            i = jacobi_layout(std::max(j.m, j.n), uint32_t(k), most, JSMEM_DOUBLES).g_smem ? 1 : 0;
-            log_cols = std::max(log_cols, uint32_t(k));
-        }
-        cls[i].push_back(j);
-        if (i < 2) {
-            cls[i].back().l_off = log_len;
+        const JacobiMode m = jacobi_mode(std::max(j.m, j.n), uint32_t(k), 1u << size[b]);
+        std::vector<SvdJob>& v = cls[cls_of(size[b], m)];
+        v.push_back(j);
+        if (m >= J_LOGGED) {
+            v.back().l_off = log_len;
             log_len += log_entries(uint32_t(k));
+            log_cols = std::max(log_cols, uint32_t(k));
+            ++n_logged;
         }
     }
     DBuf<double2> log(log_len);
-    DBuf<int> metas(2 * (cls[0].size() + cls[1].size()));
+    DBuf<int> metas(2 * n_logged);
     if (metas.size()) QCM_CUDA(cudaMemsetAsync(metas.get(), 0, metas.size() * sizeof(int), s));
     if (nid) QCM_CUDA(cudaMemsetAsync(zero_count, 0, nid * sizeof(int), s));
     std::vector<SvdJob> all;
@@ -565,26 +583,27 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
     jobbuf.upload(all, s);
     if (used > 1 && !side) side = std::make_unique<SideStreams>();
     if (used > 1) side->fork(s);
-    std::size_t first = 0;
+    std::size_t first = 0, first_logged = 0;
     int lane = -1;  // the first launch stays on s
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < NCLS && err == cudaSuccess; ++i) {
         if (cls[i].empty()) continue;
-        const uint32_t nc = i < 2 ? most : JMAX_CLUSTER >> (i - 2);
+        const uint32_t nc = 1u << (N_CLUSTER_SIZES - 1 - i / 4);
+        const JacobiMode mode = JacobiMode(J_LOGGED_L2 - i % 4);
         // shared memory of the launch's largest block (everything that fits), threads by its pairs per round
         uint64_t sm = 0;
         uint32_t lanes = 0;
         for (const SvdJob& j : cls[i]) {
             const uint32_t r = std::max(j.m, j.n), c = std::min(j.m, j.n);
             const JacobiLayout l = jacobi_layout(r, c, nc, JSMEM_DOUBLES);
-            sm = std::max(sm, l.fixed + (i > 0 ? uint64_t(l.ldg) * c : 0) + (i > 1 ? uint64_t(l.ldq) * c : 0));
+            sm = std::max(sm, l.fixed + (mode != J_LOGGED_L2 ? uint64_t(l.ldg) * c : 0) + (mode < J_LOGGED ? uint64_t(l.ldq) * c : 0));
             lanes = std::max(lanes, (c + 1) / 2 * (nc == 1 ? 16 : 8));
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(unsigned(cls[i].size()) * nc);
         cfg.blockDim = dim3(std::min<uint32_t>(JTHR, std::max<uint32_t>(128, (lanes + 127) / 128 * 128)));
         cfg.dynamicSmemBytes = std::size_t(sm) * sizeof(double);
-        cfg.stream = lane < 0 ? s : side->s[lane];
+        cfg.stream = lane < 0 ? s : side->s[lane % SideStreams::N];
         cudaLaunchAttribute at{};
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = nc;
@@ -592,16 +611,17 @@ void batched_jacobi_svd(const std::vector<SvdJob>& jobs, const double* A, uint64
         cfg.attrs = &at;
         cfg.numAttrs = 1;
         const SvdJob* dj = jobbuf.get() + first;
-        if (i > 1) {
-            err = cudaLaunchKernelEx(&cfg, nc == 1 ? k_jacobi_svd<J_ONE> : k_jacobi_svd<J_SMEM>, dj, A, U, S, V, W, zero_count,
+        if (mode < J_LOGGED) {
+            err = cudaLaunchKernelEx(&cfg, mode == J_ONE ? k_jacobi_svd<J_ONE> : k_jacobi_svd<J_SMEM>, dj, A, U, S, V, W, zero_count,
                                      sweeps_used, JacobiLog{nullptr, nullptr, 0});
         } else {
             // LOG_SWEEPS sweeps, then their rotations applied to Q, up to the limit of sweeps (launches after the last
             // block is done return at once)
             const std::size_t qb = std::size_t(log_cols) * ROWS_SLICE * sizeof(double);
             const dim3 qg((log_cols + ROWS_SLICE - 1) / ROWS_SLICE, unsigned(cls[i].size()));
-            auto* kernel = i == 0 ? k_jacobi_svd<J_LOGGED_L2> : k_jacobi_svd<J_LOGGED>;
-            int* meta = metas.get() + (i == 0 ? 0 : 2 * cls[0].size());
+            auto* kernel = mode == J_LOGGED_L2 ? k_jacobi_svd<J_LOGGED_L2> : k_jacobi_svd<J_LOGGED>;
+            int* meta = metas.get() + 2 * first_logged;
+            first_logged += cls[i].size();
             for (int x = 0; x < JMAX_SWEEPS / LOG_SWEEPS && err == cudaSuccess; ++x) {
                 const JacobiLog lg{log.get(), meta, x};
                 err = cudaLaunchKernelEx(&cfg, kernel, dj, A, U, S, V, W, zero_count, sweeps_used, lg);

@@ -4,6 +4,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
+#include <queue>
 #include <stdexcept>
 #include <string>
 
@@ -107,23 +109,84 @@ void svd_thin_lane(Solver& sv, int l, const double* A, int m, int n, double* U, 
                                  info, L.svdp));
 }
 
-uint32_t largest_cluster(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t want) {
-    for (uint32_t nc = want; nc > 1; nc /= 2) {
+ClusterSlots cluster_slots(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t max_cluster) {
+    ClusterSlots r{};
+    for (int i = 0; i < N_CLUSTER_SIZES && (1u << i) <= max_cluster; ++i) {
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(nc);
+        cfg.gridDim = dim3(1u << i);
         cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = bytes;
         cudaLaunchAttribute at{};
         at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = nc;
+        at.val.clusterDim.x = 1u << i;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) return nc;
-        cudaGetLastError();  // a size that the device does not know is an error
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) r[i] = uint32_t(std::max(n, 0));
+        else cudaGetLastError();  // a size that the device does not know is an error
     }
-    return 1;
+    r[0] = std::max(r[0], 1u);
+    return r;
+}
+
+std::vector<uint8_t> plan_clusters(const std::vector<std::array<double, N_CLUSTER_SIZES>>& cost, const std::vector<uint8_t>& want,
+                                   const ClusterSlots& slots) {
+    const std::size_t n = want.size();
+    std::vector<uint8_t> most(want), best;
+    double full = 0.0, t0 = 0.0;
+    for (std::size_t i = 0; i < n; ++i) {
+        while (!slots[most[i]]) --most[i];
+        full += 1.0 / slots[most[i]];
+        t0 = std::max(t0, *std::min_element(cost[i].begin(), cost[i].begin() + most[i] + 1));
+    }
+    if (full <= 1.0) return most;
+    std::vector<uint8_t> size(n), before;
+    std::vector<std::size_t> order(n);
+    double end = 0.0, limit = t0;
+    for (int step = 0; step < 24; ++step, limit *= 1.25) {
+        bool least = true;  // every block at its size of least area
+        for (std::size_t i = 0; i < n; ++i) {
+            int within = -1, area = 0, fast = 0;
+            for (int k = 0; k <= most[i]; ++k) {
+                if (!slots[k]) continue;
+                const double a = cost[i][k] / slots[k];
+                if (a < cost[i][area] / slots[area]) area = k;
+                if (cost[i][k] < cost[i][fast]) fast = k;
+                if (cost[i][k] <= limit && (within < 0 || a < cost[i][within] / slots[within])) within = k;
+            }
+            size[i] = uint8_t(within < 0 ? fast : within);
+            least = least && size[i] == area;
+        }
+        if (size != before) {
+            before = size;
+            for (std::size_t i = 0; i < n; ++i) order[i] = i;
+            std::sort(order.begin(), order.end(), [&](std::size_t a, std::size_t b) {
+                if (size[a] != size[b]) return size[a] > size[b];
+                return cost[a][size[a]] != cost[b][size[b]] ? cost[a][size[a]] > cost[b][size[b]] : a < b;
+            });
+            // blocks start in this order, each as soon as its share of the device is free
+            std::priority_queue<std::pair<double, double>, std::vector<std::pair<double, double>>, std::greater<>> running;
+            double now = 0.0, free = 1.0, last = 0.0;
+            for (std::size_t i : order) {
+                const double share = 1.0 / slots[size[i]];
+                while (free < share - 1e-9) {
+                    now = running.top().first;
+                    free += running.top().second;
+                    running.pop();
+                }
+                free -= share;
+                running.push({now + cost[i][size[i]], share});
+                last = std::max(last, now + cost[i][size[i]]);
+            }
+            if (best.empty() || last < end) {
+                best = size;
+                end = last;
+            }
+        }
+        if (least) break;
+    }
+    return best;
 }
 
 void syevd_lane(Solver& sv, int l, double* A, int n, double* W, int* info) {

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
+#include <array>
 #include <cstdint>
 #include <memory>
 #include <vector>
@@ -68,10 +69,21 @@ struct SideStreams {
     void join(cudaStream_t to);
 };
 
-// CTAs per cluster, at most `want` (a power of two, up to 16), that the device can schedule of a kernel with the given
-// threads and dynamic shared memory per CTA.  Clusters of 16, and on a partitioned device smaller ones too, need more SMs
-// side by side than it may have; a cluster of one always runs.
-uint32_t largest_cluster(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t want);
+// Clusters of 1, 2, 4, 8 and 16 CTAs of a kernel, with the given threads and dynamic shared memory per CTA, that the
+// device runs at once; 0 for sizes above max_cluster or that it cannot schedule (clusters of 16, and on a partitioned
+// device smaller ones too, need more SMs side by side than it may have; a cluster of one always runs)
+constexpr int N_CLUSTER_SIZES = 5;
+using ClusterSlots = std::array<uint32_t, N_CLUSTER_SIZES>;
+ClusterSlots cluster_slots(const void* kernel, uint32_t threads, std::size_t bytes, uint32_t max_cluster);
+
+// Cluster size (log2) of every block of a batch.  want: the size at which a block alone is fastest; cost: its time by
+// size, in one unit for all blocks.  A batch that fits the device at once takes the wanted sizes (or the largest that can
+// run).  A larger one does not: what a cluster gains is less than the CTAs that it takes (500 blocks of 160 x 160, 8 CTAs
+// each: 171 ms a truncation, with one each 121 ms).  There a time is tried, from the longest block's shortest up: each
+// block takes the size of least area (time over the clusters of that size that run at once) within it, and the time for
+// which the whole batch, launched in order of size, ends first is kept.
+std::vector<uint8_t> plan_clusters(const std::vector<std::array<double, N_CLUSTER_SIZES>>& cost, const std::vector<uint8_t>& want,
+                                   const ClusterSlots& slots);
 
 // Thin SVDs of many blocks (one-sided Jacobi, a cluster of 1 to 16 CTAs per block; jacobi_svd.cu):
 // A_j (m x n, ld m) = U_j diag(S_j) V_j^T with U_j (m x k, ld m), S_j descending (k), V_j

@@ -49,15 +49,15 @@ constexpr uint32_t QR_PIV_MAX = 1024;           // columns of a pivoted factoris
 constexpr uint32_t QR_SMEM_DOUBLES = 28400;     // dynamic shared memory per CTA (222 KiB; 2.4 KiB static)
 constexpr uint32_t QR_MAX_CLUSTER = 16;
 
-// CTAs per block: 64 columns of 64 rows are two passes of the 32 warps, about what a step's barriers cost; a cluster's
+// CTAs per block, alone: 64 columns of 64 rows are two passes of the 32 warps, about what a step's barriers cost; a cluster's
 // barrier costs more than a CTA's, and up to about 112 columns of 112 rows one CTA is the faster (66 to 90 columns:
 // 0.37 ms against 0.62 ms).  The pivoted QRs of a two-site truncation at L=24: M=2048 70 ms with one CTA per block, 8.6 ms
 // so; M=512 1.54 and 1.04 ms.
-inline uint32_t qr_cluster(uint32_t mm, uint32_t nn, uint32_t most) {
+inline uint32_t qr_cluster(uint32_t mm, uint32_t nn) {
     const uint64_t e = uint64_t(mm) * nn;
     if (e <= 112 * 112) return 1;
     uint32_t nc = 1;
-    while (nc < most && nc * 2 <= nn && e > uint64_t(64 * 64) * nc * nc) nc *= 2;
+    while (nc < QR_MAX_CLUSTER && nc * 2 <= nn && e > uint64_t(64 * 64) * nc * nc) nc *= 2;
     return nc;
 }
 
@@ -317,24 +317,28 @@ __global__ void __launch_bounds__(QR_THR) k_qr(const QrJob* __restrict__ jobs, c
     }
 }
 
+__host__ __device__ inline uint64_t qr_one_size(uint32_t m, uint32_t n) { return uint64_t(m) * n + (m < n ? m : n); }
+
 // An unpivoted factorisation by one CTA: no pivot is looked for and nothing is exchanged, so a step is the norm of its
 // column, the reflector in place of it, and the trailing columns, one warp each.  Against k_qr with one CTA, which finds
 // the norms of all columns and keeps its reflectors in L2: 100 x 100 0.57 against 0.73 ms, 48 x 48 0.21 against 0.26 ms,
-// 20 x 400 0.25 against 0.39 ms (whole calls).  Pivoted blocks are the faster in k_qr.
+// 20 x 400 0.25 against 0.39 ms (whole calls).  Pivoted blocks are the faster in k_qr.  SMEM: the work matrix is in shared
+// memory; else in the block's scratch, by all the CTA's 1024 threads, a number known to the compiler (75 blocks of
+// 256 x 256: 4.7 ms, 5.3 ms without).
+template <bool SMEM>
 __global__ void __launch_bounds__(QR_THR) k_qr_one(const QrJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ Q,
-                                                   double* __restrict__ R, double* __restrict__ W, uint32_t smem_doubles) {
+                                                   double* __restrict__ R, double* __restrict__ W) {
     extern __shared__ double qsm[];
     __shared__ double red[QR_WARPS];
     __shared__ double sh_tau, sh_scale, sh_thr;
     __shared__ int sh_zero;
     const QrJob J = jobs[blockIdx.x];
-    const uint32_t nthr = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr / 32;
+    const uint32_t nthr = SMEM ? blockDim.x : QR_THR, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr / 32;
     // the matrix factorised: F (mm x nn) = A_j, or A_j^T for an LQ
     const uint32_t mm = J.lq ? J.n : J.m, nn = J.lq ? J.m : J.n, k = mm < nn ? mm : nn;
-    // F, then R above and the reflectors below the diagonal, with the k reflector scales after it: in shared memory
-    // if they fit the launch's, else in the block's scratch (L2-resident)
-    const uint64_t fsz = uint64_t(mm) * nn + k;
-    double* w = fsz <= smem_doubles ? qsm : W + J.w_off;
+    // F, then R above and the reflectors below the diagonal, with the k reflector scales after it
+    const uint64_t fsz = qr_one_size(mm, nn);
+    double* w = SMEM ? qsm : W + J.w_off;
     double* taus = w + uint64_t(mm) * nn;
     const double* a = A + J.a_off;
     double f = 0.0;
@@ -469,7 +473,7 @@ uint64_t qr_scratch(uint32_t m, uint32_t n, bool) {
     const uint64_t k = std::min(m, n);
     uint64_t d = 0;
     for (auto [mm, nn] : {std::pair<uint32_t, uint32_t>{m, n}, {n, m}}) {
-        for (uint32_t nc = qr_cluster(mm, nn, QR_MAX_CLUSTER); nc; nc /= 2) {
+        for (uint32_t nc = qr_cluster(mm, nn); nc; nc /= 2) {
             const QrLayout l = qr_layout(mm, nn, nc, 0);
             d = std::max<uint64_t>(d, uint64_t(mm) * k + nc * (l.fixed + uint64_t(l.ncol) * mm));
         }
@@ -482,30 +486,41 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
                 cudaStream_t s, uint32_t max_cluster, uint32_t* P, uint64_t p_len) {
     if (jobs.empty()) return;
     // attributes belong to the functions, for all contexts and host threads: the same values on every call
-    for (const void* k : {reinterpret_cast<const void*>(&k_qr), reinterpret_cast<const void*>(&k_qr_one)})
+    for (const void* k : {reinterpret_cast<const void*>(&k_qr), reinterpret_cast<const void*>(&k_qr_one<true>)})
         QCM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(QR_SMEM_DOUBLES * sizeof(double))));
-    // the most CTAs that a block wants, and that a cluster can have here
-    uint32_t most = 1;
-    for (const QrJob& j : jobs) most = std::max(most, j.lq ? qr_cluster(j.n, j.m, QR_MAX_CLUSTER) : qr_cluster(j.m, j.n, QR_MAX_CLUSTER));
-    if (most > 1) {
-        QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        most = largest_cluster(reinterpret_cast<const void*>(&k_qr), QR_THR, QR_SMEM_DOUBLES * sizeof(double), std::min(most, max_cluster));
+    // time of a block in us by the cluster's size: k steps of a fixed part and of the trailing matrix and Q, dealt out (from
+    // single pivoted blocks of 115 to 512 columns, within a fifth)
+    std::vector<std::array<double, N_CLUSTER_SIZES>> cost(jobs.size());
+    std::vector<uint8_t> size(jobs.size(), 0);
+    bool split = false;
+    for (std::size_t b = 0; b < jobs.size(); ++b) {
+        const QrJob& j = jobs[b];
+        const uint32_t mm = j.lq ? j.n : j.m, nn = j.lq ? j.m : j.n;
+        while ((2u << size[b]) <= qr_cluster(mm, nn)) ++size[b];
+        split = split || size[b];
+        for (int i = 0; i < N_CLUSTER_SIZES; ++i)
+            cost[b][i] = std::min(mm, nn) * ((i || (j.flags & QR_PIVOT) ? 3.5 : 2.0) + 0.31e-3 * mm * nn / (1 << i));
     }
-    constexpr int NCLS = 6;  // 16, 8, 4, 2, 1 CTAs per block, and one CTA unpivoted: a launch each
-    static_assert(QR_MAX_CLUSTER >> (NCLS - 2) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
+    if (split) {
+        QCM_CUDA(cudaFuncSetAttribute(k_qr, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        size = plan_clusters(cost, size, cluster_slots(reinterpret_cast<const void*>(&k_qr), QR_THR, QR_SMEM_DOUBLES * sizeof(double), max_cluster));
+    }
+    // 16, 8, 4, 2, 1 CTAs per block, and one CTA unpivoted beyond and in shared memory: a launch each
+    constexpr int ONE_L2 = N_CLUSTER_SIZES, ONE = ONE_L2 + 1, NCLS = ONE + 1;
+    static_assert(QR_MAX_CLUSTER >> (N_CLUSTER_SIZES - 1) == 1 && SideStreams::N >= NCLS - 1, "a stream per class");
     std::vector<QrJob> cls[NCLS];
-    for (const QrJob& j : jobs) {
+    for (std::size_t b = 0; b < jobs.size(); ++b) {
+        const QrJob& j = jobs[b];
         const uint64_t k = std::min(j.m, j.n);
         if (!j.m || !j.n || j.a_off + uint64_t(j.m) * j.n > a_len || j.w_off + qr_scratch(j.m, j.n, j.lq != 0) > w_len ||
             j.q_off + k * (j.lq ? j.n : j.m) > q_len || j.r_off + k * (j.lq ? j.m : j.n) > r_len)
             throw std::runtime_error("batched QR: a block outside its buffers");
-        const uint32_t mm = j.lq ? j.n : j.m, nn = j.lq ? j.m : j.n;
+        const uint32_t nn = j.lq ? j.m : j.n;
         if ((j.flags & QR_RT) && j.lq) throw std::runtime_error("batched QR: a transposed R is for a QR, not an LQ");
         if ((j.flags & QR_PIVOT) && (!P || nn > QR_PIV_MAX || j.p_off + nn > p_len))
             throw std::runtime_error("batched QR: pivoting needs a permutation buffer and at most 1024 columns");
-        int i = 0;
-        for (uint32_t x = QR_MAX_CLUSTER; x > qr_cluster(mm, nn, most); x /= 2) ++i;
-        if (i == NCLS - 2 && !(j.flags & QR_PIVOT)) ++i;
+        int i = N_CLUSTER_SIZES - 1 - size[b];
+        if (!size[b] && !(j.flags & QR_PIVOT)) i = qr_one_size(j.m, j.n) > QR_SMEM_DOUBLES ? ONE_L2 : ONE;
         cls[i].push_back(j);
     }
     std::vector<QrJob> all;
@@ -526,19 +541,21 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < NCLS && err == cudaSuccess; ++i) {
         if (cls[i].empty()) continue;
-        if (i == NCLS - 1) {
-            // shared memory of the largest work matrix that fits, a warp per column and a thread per row
+        const cudaStream_t st = lane < 0 ? s : side->s[lane];
+        if (i >= ONE_L2) {
+            // shared memory of the largest work matrix, a warp per column and a thread per row
             uint64_t sm = 0, thr = 0;
             for (const QrJob& j : cls[i]) {
-                const uint64_t e = uint64_t(j.m) * j.n + std::min(j.m, j.n);
-                if (e <= QR_SMEM_DOUBLES) sm = std::max(sm, e);
+                if (i == ONE) sm = std::max(sm, qr_one_size(j.m, j.n));
                 thr = std::max<uint64_t>(thr, std::max(32 * uint64_t(j.lq ? j.m : j.n), uint64_t(j.lq ? j.n : j.m)));
             }
-            thr = std::min<uint64_t>(QR_THR, std::max<uint64_t>(128, (thr + 127) / 128 * 128));
-            k_qr_one<<<unsigned(cls[i].size()), unsigned(thr), std::size_t(sm) * sizeof(double), lane < 0 ? s : side->s[lane]>>>(
-                jobbuf.get() + first, A, Q, R, W, uint32_t(sm));
+            thr = i == ONE_L2 ? QR_THR : std::min<uint64_t>(QR_THR, std::max<uint64_t>(128, (thr + 127) / 128 * 128));
+            auto* kernel = i == ONE ? k_qr_one<true> : k_qr_one<false>;
+            kernel<<<unsigned(cls[i].size()), unsigned(thr), std::size_t(sm) * sizeof(double), st>>>(jobbuf.get() + first, A, Q, R, W);
             err = cudaGetLastError();
-            break;  // the last class
+            first += cls[i].size();
+            ++lane;
+            continue;
         }
         const uint32_t nc = QR_MAX_CLUSTER >> i;
         uint64_t sm = 0;
@@ -553,7 +570,7 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
         cfg.gridDim = dim3(unsigned(cls[i].size()) * nc);
         cfg.blockDim = dim3(std::min<uint32_t>(QR_THR, std::max<uint32_t>(128, (cols * 32 + 127) / 128 * 128)));
         cfg.dynamicSmemBytes = std::size_t(sm) * sizeof(double);
-        cfg.stream = lane < 0 ? s : side->s[lane];
+        cfg.stream = st;
         cudaLaunchAttribute at{};
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = nc;
