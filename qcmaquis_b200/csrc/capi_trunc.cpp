@@ -74,9 +74,13 @@ int qcm_truncate_svd(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* rows, cons
         pu += uint64_t(m) * kp; ps += kp; pv += uint64_t(kp) * n;
     }
     qcm::DBuf<double> out(std::max<uint64_t>(pu + pv, 1));
-    qcm::batched_copy(ju, sv.U.get(), sv.u_len, out.get(), pu, c.cjobs, c.s);
     qcm::batched_copy(jv, sv.V.get(), sv.v_len, out.get() + pu, pv, c.cjobs, c.s);
-    download(c, out.get(), U, pu);
+    if (ju.size() == 1) {
+        download(c, sv.U.get() + ju[0].src_off, U, pu);  // one block's kept columns lie together
+    } else {
+        qcm::batched_copy(ju, sv.U.get(), sv.u_len, out.get(), pu, c.cjobs, c.s);
+        download(c, out.get(), U, pu);
+    }
     download(c, out.get() + pu, Vt, pv);
     QCM_CUDA(cudaStreamSynchronize(c.s));
     to_result(sv.tr, result);

@@ -51,8 +51,8 @@ constexpr uint32_t QR_MAX_CLUSTER = 16;
 
 // CTAs per block, alone: 64 columns of 64 rows are two passes of the 32 warps, about what a step's barriers cost; a cluster's
 // barrier costs more than a CTA's, and up to about 112 columns of 112 rows one CTA is the faster (66 to 90 columns:
-// 0.37 ms against 0.62 ms).  The pivoted QRs of a two-site truncation at L=24: M=2048 70 ms with one CTA per block, 8.6 ms
-// so; M=512 1.54 and 1.04 ms.
+// 0.37 ms against 0.62 ms).  The pivoted QRs of a two-site truncation at L=24: M=2048 70 ms with one CTA per block, 8.8 ms
+// so; M=512 1.54 and 1.1 ms.
 inline uint32_t qr_cluster(uint32_t mm, uint32_t nn) {
     const uint64_t e = uint64_t(mm) * nn;
     if (e <= 112 * 112) return 1;
@@ -559,16 +559,16 @@ void batched_qr(const std::vector<QrJob>& jobs, const double* A, uint64_t a_len,
         }
         const uint32_t nc = QR_MAX_CLUSTER >> i;
         uint64_t sm = 0;
-        uint32_t cols = 0;
+        uint32_t lanes = 0;  // a warp per column, a thread per row
         for (const QrJob& j : cls[i]) {
             const uint32_t mm = j.lq ? j.n : j.m, nn = j.lq ? j.m : j.n;
             const QrLayout l = qr_layout(mm, nn, nc, QR_SMEM_DOUBLES);
             if (l.fixed_smem) sm = std::max(sm, l.fixed + (l.cols_smem ? uint64_t(l.ncol) * mm : 0));
-            cols = std::max(cols, l.ncol);
+            lanes = std::max(lanes, std::max(l.ncol * 32, mm));
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(unsigned(cls[i].size()) * nc);
-        cfg.blockDim = dim3(std::min<uint32_t>(QR_THR, std::max<uint32_t>(128, (cols * 32 + 127) / 128 * 128)));
+        cfg.blockDim = dim3(std::min<uint32_t>(QR_THR, std::max<uint32_t>(128, (std::min<uint32_t>(lanes, QR_THR) + 127) / 128 * 128)));
         cfg.dynamicSmemBytes = std::size_t(sm) * sizeof(double);
         cfg.stream = st;
         cudaLaunchAttribute at{};

@@ -18,3 +18,17 @@ def test_flat_and_tall_blocks(n):
         # backward error of the QR and the rotations: far below 100 sqrt(k) eps of the largest singular value
         assert u.shape == (a.shape[0], k) and vt.shape == (k, a.shape[1]) and k == min(a.shape)
         assert np.abs((u * s) @ vt - a).max() <= 100 * np.sqrt(k) * EPS * s[0]
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (40, 7), (7, 40), (50, 50)])
+@pytest.mark.parametrize("keep", [1, 5, 50])
+def test_one_block_cut(shape, keep):
+    """A single block's kept columns, which are read back without a gather."""
+    a = np.random.default_rng(8).standard_normal(shape)
+    (u, s, vt), = dmrg.truncate_svd(heff.Context(0), [a], keep, 1e-30)[0]
+    ru, rs, rvt = np.linalg.svd(a, full_matrices=False)
+    k = min(keep, rs.size)
+    assert u.shape == (shape[0], k) and vt.shape == (k, shape[1])
+    assert np.abs(s - rs[:k]).max() <= 100 * np.sqrt(rs.size) * EPS * rs[0]  # as above
+    # the leading subspace: errors are amplified by the gap to the values cut off, none of which is within 1e-3 here
+    assert np.abs((u * s) @ vt - (ru[:, :k] * rs[:k]) @ rvt[:k]).max() <= 1e3 * 100 * np.sqrt(rs.size) * EPS * rs[0]
