@@ -320,8 +320,8 @@ void qcm_heff_group_free(qcm_heff_group* g);
  * allocator reserves HBM and before any stream capture.  The address belongs to
  * the context: after cudaDeviceReset the context and its plans are invalid.
  * All calls on a device share the array and it keeps the last call's contents
- * (S is cleared inside each call): calls that overlap on the GPU -- other
- * streams, other threads -- race.  Makes the context's device current for the
+ * (a call writes all that it reads, or clears it first): calls that overlap on
+ * the GPU -- other streams, other threads -- race.  Makes the context's device current for the
  * call and restores the caller's.  Enqueued on the context stream
  * (asynchronous). */
 #define QCM_NOALLOC_SCRATCH_DOUBLES (8u * 1024u * 1024u)
@@ -585,12 +585,13 @@ void qcm_dmrg_free(qcm_dmrg* d);
  * below cutoff * s_max).  Outputs per block k, packed in block order with keep[k]
  * columns: U_k (rows x keep, ld rows), S_k (keep, descending), Vt_k (keep x cols, ld keep).
  * Size U, S, Vt for keep = min(rows, cols).  A block larger than 1024 in both
- * dimensions is refused. */
+ * dimensions is refused.  The CTAs that share a block, and with them the rounding of
+ * its results, depend on the other blocks of the call. */
 int qcm_truncate_svd(qcm_ctx* ctx, uint32_t n_blocks, const uint32_t* rows, const uint32_t* cols, const double* blocks,
                      uint64_t max_bond_dimension, double cutoff, uint32_t* keep, double* U, double* S, double* Vt,
                      qcm_trunc_result* result);
-/* Thin QR (lq = 0) or LQ (lq = 1) of every block, all blocks in one launch (one CTA each, Householder
- * reflectors as geqrf / orgqr and gelqf / orglq define them): replaces qr / lq of
+/* Thin QR (lq = 0) or LQ (lq = 1) of every block, all blocks at once (one CTA or a cluster of up to 16 each, a launch
+ * per cluster size; Householder reflectors as geqrf / orgqr and gelqf / orglq define them): replaces qr / lq of
  * framework/alps/matrix/algorithms.hpp:260-325, which MPSTensor::normalize_left / normalize_right
  * (mp_tensors/mpstensor.hpp:242-300) call per block.  With k = min(rows, cols), outputs packed in block
  * order: QR -- Q_k (rows x k) in Q, R_k (k x cols, upper triangular) in R; LQ -- Q_k (k x cols) in Q,

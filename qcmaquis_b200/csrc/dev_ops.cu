@@ -199,7 +199,7 @@ __global__ void k_fill(double* p, uint64_t n, double v) {
 
 unsigned grid_for(uint64_t n, unsigned bs = 256) {
     uint64_t g = (n + bs - 1) / bs;
-    return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, 148 * 16)));
+    return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, N_SM * 16)));
 }
 
 }  // namespace
@@ -256,7 +256,7 @@ void batched_copy(const std::vector<CopyJob>& jobs, const double* src, uint64_t 
     if (!cols) return;
     // CTAs per job by the largest job's parts, but (the smaller jobs' have nothing to do) not beyond 64 per SM in all where
     // a CTA per column strip is less
-    const uint64_t y = std::min(parts, std::max<uint64_t>((cols - 1) / CP_COLS + 1, 148 * 64 / jobs.size()));
+    const uint64_t y = std::min(parts, std::max<uint64_t>((cols - 1) / CP_COLS + 1, N_SM * 64 / jobs.size()));
     jobbuf.upload(jobs, s);
     k_bcopy<<<dim3(unsigned(jobs.size()), unsigned(std::min<uint64_t>(y, 65535))), 256, 0, s>>>(jobbuf.get(), src, dst, scale);
     QCM_CUDA(cudaGetLastError());

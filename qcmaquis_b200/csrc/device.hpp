@@ -21,6 +21,8 @@
 
 namespace qcm {
 
+constexpr unsigned N_SM = 148;  // SMs of a B200
+
 // Stream-ordered device memory.  While an AllocStream scope is active on this
 // thread, DBuf allocations come from the library's own memory pool on that stream
 // (cudaMallocFromPoolAsync) and are released on it (cudaFreeAsync), so freeing and

@@ -284,7 +284,7 @@ void heff_adjoint_device(HeffPlan& p, const double* x, const double* ybar, doubl
         k_wadj<<<cg.task_ptr.back(), wg::THR, 0, s>>>(cg.tables(), w.d_Wb.get(), w.d_pofs.get(), w.d_P.get(),
                                                              w.d_err.get());
     QCM_CUDA(cudaGetLastError());
-    const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 31) / 32, 148 * 16));
+    const unsigned grid = unsigned(std::min<uint64_t>((w.n_terms + 31) / 32, N_SM * 16));
     k_entry_sum<<<grid, 32 * ES_WARPS, 0, s>>>(w.n_terms, w.d_e_row.get(), cg.d_m_ptr.get(), w.d_rl_ptr.get(), w.d_rl_line.get(),
                                      w.d_pofs.get(), w.d_P.get(), coeff_bar);
     QCM_CUDA(cudaGetLastError());

@@ -41,7 +41,8 @@ using namespace dm;
 // all its own CTAs run (grid_trigger), so that the next kernel's CTAs load their descriptors into the slots that
 // the last wave leaves empty, and waits (grid_wait) for the one before it to be complete before it touches anything
 // that a kernel writes.  What is read before grid_wait (tiles, jobs, units, k-step lists) is written by copies when a
-// plan is staged, never by a kernel.  A call with host vectors at L=8, M=64: 121 -> 113 us, L=12, M=101 95 -> 90 us.
+// plan is staged, never by a kernel.  A call with host vectors at L=8, M=64 91 -> 83 us, with device vectors at L=12, M=101
+// 79 -> 75 us (medians of calls waited for one by one).
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 template <class... P, class... X>
@@ -865,12 +866,12 @@ void rebind_plan(HeffPlan& p, const DevBoundary& L, const DevBoundary& R) {
 
 namespace {
 // Launch order of a launch's tiles of one shape: those of most k-steps first (as many: in the given order), so that no
-// long tile starts when the chip is about to run empty.  Only up to 24 sets of the 148 x 5 CTAs that run at once: the
+// long tile starts when the chip is about to run empty.  Only up to 24 sets of the N_SM x 5 CTAs that run at once: the
 // end of a longer launch is a small part of it, and the given order keeps a unit's operands in L2.
 //   S-GEMM at L=12, M=101 33 -> 29 us, L=16, M=256 (17 sets in all) 302 -> 291 us, streamed chunks at L=20, M=384 3.33
 //   -> 3.13 ms; ordered whole at L=24, M=1024 (over 100 sets) 7.88 -> 7.98 ms.
 //   L.S at L=16, M=256 83 -> 75 us, L=24, M=512 0.441 -> 0.425 ms.  The T-GEMM's tiles differ too little: no effect.
-constexpr std::size_t ORDERED_TILES = 24 * 148 * 5;
+constexpr std::size_t ORDERED_TILES = 24 * N_SM * 5;
 template <class D, class Steps>
 void longest_first(std::vector<D>& t, std::size_t first, std::size_t last, Steps steps) {
     if (last - first > ORDERED_TILES) return;

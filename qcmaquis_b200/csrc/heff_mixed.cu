@@ -503,14 +503,14 @@ void launch_tc(const HeffPlan& p, int sh, const float* Wh, const float* Wl, cons
 
 void to_f32(const double* x, float* y, uint64_t n, cudaStream_t s) {
     if (!n) return;
-    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148 * 16);
+    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, N_SM * 16);
     k_to_f32<<<unsigned(blocks), 256, 0, s>>>(x, y, n);
     QCM_CUDA(cudaGetLastError());
 }
 
 void split_tf32(const double* x, float* hi, float* lo, uint64_t n, cudaStream_t s) {
     if (!n) return;
-    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148 * 16);
+    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, N_SM * 16);
     k_split<<<unsigned(blocks), 256, 0, s>>>(x, hi, lo, n);
     QCM_CUDA(cudaGetLastError());
 }

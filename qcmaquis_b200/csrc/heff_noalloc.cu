@@ -78,8 +78,8 @@ extern "C" int qcm_heff_apply_device_noalloc(qcm_heff* h, const double* x_dev, d
     double* Tb = base;
     double* Sb = Tb + round32(p.t_len);
     double* Pb = Sb + round32(p.s_len);
-    // T and the partial tiles are fully written by their kernels; the S buffer is cleared
-    // inside the apply (rows without coefficients must read as zero).
+    // What the apply reads of T, S and the partial tiles its kernels write first; an S that its tiles do not cover
+    // is cleared inside the apply (rows without coefficients must read as zero).
     qcm::heff_apply_device_scratch(p, x_dev, y_dev, Tb, Sb, Pb);
     return QCM_OK;
     QCM_CATCH

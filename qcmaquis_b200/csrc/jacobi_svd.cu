@@ -25,8 +25,8 @@
 // of rows that fit shared memory, LOG_SWEEPS sweeps at a time.
 //
 // Measured, the blocks of a two-site truncation at L=24: M=2048 (93 blocks, up to 558 columns) 1265 ms with one CTA per
-// block, 76 ms with clusters, 58 ms with the log, two buffers and one CTA up to 88 columns; M=512 (75 blocks, up to 142)
-// 8.5, 3.2 and 2.9 ms.  What is left is a round's chain, 9.8 us at 546 columns.
+// block, 76 ms with clusters, 58 ms with the log, two buffers and one CTA up to 88 columns, 55 ms with sizes by the batch;
+// M=512 (75 blocks, up to 142) 8.5, 3.2, 2.9 and 2.9 ms.  What is left is a round's chain, 9.3 us at 546 columns.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

@@ -13,8 +13,8 @@ namespace qcm {
 
 // The tiles of a phase in all its shapes, one launch: the CTA's tile is looked up by running ends in the order
 // 128-, 64-, 32-, 16-row tiles.  A launch per shape left the chip idle at the end of each one: a few long 128-row
-// tiles alone took as long as a tenth of the phase (S-GEMM at L=16, M=256 425 -> 333 us, at L=24, M=512 2.72 -> 2.50 ms).  Shared memory is the largest shape's; registers are set by
-// the launch bounds in any case.
+// tiles alone took as long as a tenth of the phase (S-GEMM at L=16, M=256 425 -> 333 us, at L=24, M=512 2.72 ->
+// 2.50 ms).  Shared memory is the largest shape's; registers are set by the launch bounds in any case.
 template <class D>
 struct TileSet {
     const D* t[N_SHAPES];

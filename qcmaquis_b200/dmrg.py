@@ -131,7 +131,7 @@ _lib._sig("qcm_qr_blocks", c_int, c_void_p, ctypes.c_uint32, _U32, _U32, P(c_dou
 
 
 def qr_blocks(ctx, blocks, lq: bool = False):
-    """Thin QR (or LQ) of every block on the device, one launch: [(Q, R) per block] (LQ: [(L, Q)])."""
+    """Thin QR (or LQ) of every block on the device, all at once: [(Q, R) per block] (LQ: [(L, Q)])."""
     bl = [np.asarray(b, dtype=np.float64) for b in blocks]
     rows = np.array([b.shape[0] for b in bl], dtype=np.uint32)
     cols = np.array([b.shape[1] for b in bl], dtype=np.uint32)
